@@ -63,6 +63,7 @@ struct Group {
   int ntiles = 0;
   int grid = 0;
   BatchInst* d_inst = nullptr;
+  BatchInst one{};  // host copy of the descriptor of a group of one problem
 };
 
 }  // namespace
@@ -90,6 +91,7 @@ struct fv_batch {
   cudaGraphExec_t graph = nullptr;
   cudaGraphExec_t graph_loop = nullptr;  // steps in each control block's own mode
   BatchInst* d_inst_multi = nullptr;     // descriptors of the multi-step launch
+  BatchInst one_multi{};
   int ntiles_multi = 0, grid_multi = 0, rows_multi = 0;
   long launches = 0;
   std::string err;
@@ -224,7 +226,8 @@ std::string GroupKey(const fv_batch* b, const Group& g) {
     cells += (long long)s.first * s.second;
   }
   std::ostringstream k;
-  k << "p" << b->precision << "_d" << g.ndim << "_co" << (g.rs >= 2) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
+  // the FP32-mixed 2-D groups' kernels (marched by warps) have a key of their own
+  k << "p" << b->precision << (b->precision != FV_PREC_FP64 && g.ndim == 2 ? "m" : "") << "_d" << g.ndim << "_co" << (g.rs >= 2) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
     << rs_mask << "_ts" << b->ts << "_n" << g.members.size() << "_c" << cells << "_h" << std::hex << h;
   return k.str();
 }
@@ -262,16 +265,29 @@ Schedule Schedule3d(const fv_batch* b, int layers) {
   return sc;
 }
 
+// Work items a CTA of the group's stage kernel runs at once (one per warp in
+// the warp-marched FP32-mixed form).
+int ItemsPerCta(const fv_batch* b, const Group& g, int shape) {
+  return g.ndim == 2 && b->precision != FV_PREC_FP64 ? fv::batch_items_per_cta32(shape) : 1;
+}
+
+// CTAs of a persistent launch over ntiles work items.
+int GridFor(const fv_batch* b, const Group& g, int shape, int occupancy, int ntiles);
+
 int Occupancy(const fv_batch* b, const Group& g, int shape) {
   if (g.ndim == 3)
     return b->precision == FV_PREC_FP64 ? fv::batch_stage3d_occupancy64(g.rs, g.tc)
                                         : fv::batch_stage3d_occupancy32(g.rs, g.tc);
   return b->precision == FV_PREC_FP64 ? fv::batch_stage_occupancy64(g.plane, g.wact, shape, g.tc)
-                                      : fv::batch_stage_occupancy32(g.plane, g.wact, shape, g.tc);
+                                      : fv::batch_stage_occupancy32(
+                                            g.plane, g.wact, shape, g.tc,
+                                            b->ts == FV_TS_RK2 ? fv::STAGE_RK_2 : fv::STAGE_EULER,
+                                            g.members.size() == 1);
 }
 
-cudaError_t LaunchStage(const fv_batch* b, const Group& g, const BatchInst* insts, int ntiles, int grid,
-                        unsigned* queue, int kind, int flip) {
+// one: the host copy of insts[0] (used when the group has one problem).
+cudaError_t LaunchStage(const fv_batch* b, const Group& g, const BatchInst* insts, const BatchInst* one, int ntiles,
+                        int grid, unsigned* queue, int kind, int flip) {
   if (g.ndim == 3)
     return b->precision == FV_PREC_FP64
                ? fv::launch_batch_stage3d64(insts, (int)g.members.size(), ntiles, queue, kind, flip, g.rs, grid, g.tc,
@@ -282,7 +298,7 @@ cudaError_t LaunchStage(const fv_batch* b, const Group& g, const BatchInst* inst
              ? fv::launch_batch_stage64(g.plane, g.wact, g.shape, insts, (int)g.members.size(), ntiles, queue, kind,
                                         flip, grid, g.tc, b->stream)
              : fv::launch_batch_stage32(g.plane, g.wact, g.shape, insts, (int)g.members.size(), ntiles, queue, kind,
-                                        flip, grid, g.tc, b->stream);
+                                        flip, grid, g.tc, b->stream, g.members.size() == 1 ? one : nullptr);
 }
 
 // Descriptors of group g for work-item shape `shape` with `rows` rows per
@@ -308,6 +324,8 @@ std::vector<BatchInst> Describe(const fv_batch* b, const Group& g, int shape, St
     I.tiles_x = (I.G.na + tx - 1) / tx;
     I.tiles_y = (I.G.nb + ty - 1) / ty;
     I.tz = g.ndim == 3 ? std::min(I.G.nc, rows > 0 ? rows : 16) : ty;  // 3-D: z layers per item
+    // marched strips carry no block structure: the rows split into even runs
+    if (g.ndim == 2 && ItemsPerCta(b, g, shape) > 1) I.tz = (I.G.nb + I.tiles_y - 1) / I.tiles_y;
     const int chunks = g.ndim == 3 ? (I.G.nc + I.tz - 1) / I.tz : 1;
     I.tile0 = t0;
     I.rs = b->p[i].riemann_solver == FV_HLL ? 0 : 1;
@@ -325,6 +343,30 @@ int SmCount() {
   return sms > 0 ? sms : 1;
 }
 
+int GridFor(const fv_batch* b, const Group& g, int shape, int occupancy, int ntiles) {
+  const int per = ItemsPerCta(b, g, shape);
+  return std::max(1, std::min(occupancy * SmCount(), (ntiles + per - 1) / per));
+}
+
+// The fewest rows per work item with which the group's strips of tx columns
+// make at most `slots` items.
+int RowsForSlots(const fv_batch* b, const Group& g, int tx, long long slots) {
+  int max_nb = 1;
+  for (int i : g.members) max_nb = std::max(max_nb, b->G[i].nb);
+  auto items = [&](int rows) {
+    long long n = 0;
+    for (int i : g.members) n += (long long)((b->G[i].na + tx - 1) / tx) * ((b->G[i].nb + rows - 1) / rows);
+    return n;
+  };
+  int lo = 1, hi = max_nb;
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (items(mid) <= slots) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
+}
+
 // Times the candidate shapes of a group on its own data, one whole step per
 // run (RK2: both stages; Euler: its one stage, which writes the idle
 // buffer), against scratch control blocks.  RK2 stage 2 overwrites U^n, so
@@ -336,8 +378,6 @@ int Autotune(fv_batch* b, Group& g) {
   if (d3 && Occupancy(b, g, 0) <= 0) return Fail(b, FV_ERR_CUDA, "the 3-D batch kernel cannot be launched");
   const fv::TileShape* shapes;
   const int ns = d3 ? 1 : NumShapes(b->precision, &shapes);
-  bool visc = false;  // the viscous form matters only with viscosity
-  for (int i : g.members) visc = visc || b->G[i].visc;
   // the first shape of a kernel (it serves every row count): strip width,
   // block rows and viscous form
   auto shape_of = [&](const Schedule& sc) {
@@ -409,19 +449,24 @@ int Autotune(fv_batch* b, Group& g) {
       if (!dup && items(z) <= r * slots) cand.push_back({0, z});
     }
   }
+  const bool marched = !d3 && b->precision != FV_PREC_FP64;  // mixed 2-D: the warp-marched shapes
   for (int s = 0; s < ns && !d3; ++s)
-    if (visc || !ShapeSchedule(b, s).vface || b->precision == FV_PREC_FP64) cand.push_back({s, shapes[s].ty});
+    if (marched == fv::batch_shape_marched32(s) || b->precision == FV_PREC_FP64) cand.push_back({s, shapes[s].ty});
   for (int s = 0; s < ns && !d3; ++s) {
     const Schedule ks = ShapeSchedule(b, s);
-    if ((ks.vface && !visc && b->precision != FV_PREC_FP64) || shape_of(ks) != s) continue;
+    if ((marched && !fv::batch_shape_marched32(s)) || shape_of(ks) != s) continue;
+    const long long slots = (long long)Occupancy(b, g, s) * SmCount() * ItemsPerCta(b, g, s);
+    if (slots <= 0) continue;
     long long units = 0;
     for (int i : g.members) units += (long long)((b->G[i].na + shapes[s].tx - 1) / shapes[s].tx) * b->G[i].nb;
-    const long long slots = (long long)Occupancy(b, g, s) * SmCount();
-    if (slots <= 0) continue;
-    const int rows = (int)std::max(4LL, (units + slots - 1) / slots);
-    bool dup = false;
-    for (auto& c : cand) dup = dup || (shape_of(ShapeSchedule(b, c.first)) == s && c.second == rows);
-    if (!dup) cand.push_back({s, rows});
+    // the rows that fill the resident slots once (marched: at most once to four times)
+    for (int k = 1; k <= (marched ? 4 : 1); ++k) {
+      const int rows = marched ? RowsForSlots(b, g, shapes[s].tx, k * slots)
+                               : (int)std::max(4LL, (units + slots - 1) / slots);
+      bool dup = false;
+      for (auto& c : cand) dup = dup || (shape_of(ShapeSchedule(b, c.first)) == s && c.second == rows);
+      if (!dup) cand.push_back({s, rows});
+    }
   }
   StepCtrl* tune_ctrl = nullptr;
   BatchInst* tune_inst = nullptr;
@@ -455,7 +500,7 @@ int Autotune(fv_batch* b, Group& g) {
     for (auto& I : descs[c]) I.Q = Fields{};
     cudaMemcpyAsync(tune_inst + c * nm, descs[c].data(), sizeof(BatchInst) * descs[c].size(),
                     cudaMemcpyHostToDevice, b->stream);
-    grid[c] = std::min(occ * SmCount(), ntiles[c]);
+    grid[c] = GridFor(b, g, s, occ, ntiles[c]);
   }
   // U^n of the group aside (RK2), when a quarter of the free memory holds it
   double* backup = nullptr;
@@ -491,9 +536,10 @@ int Autotune(fv_batch* b, Group& g) {
       g.shape = cand[c].first;
       cudaMemsetAsync(tune_queue, 0, 2 * sizeof(unsigned), b->stream);
       cudaEventRecord(e0, b->stream);
-      cudaError_t e = LaunchStage(b, g, tune_inst + c * nm, ntiles[c], grid[c], tune_queue, kind, b->flip);
+      cudaError_t e = LaunchStage(b, g, tune_inst + c * nm, descs[c].data(), ntiles[c], grid[c], tune_queue, kind, b->flip);
       if (e == cudaSuccess && both_stages)
-        e = LaunchStage(b, g, tune_inst + c * nm, ntiles[c], grid[c], tune_queue + 1, fv::STAGE_RK_2, 0);
+        e = LaunchStage(b, g, tune_inst + c * nm, descs[c].data(), ntiles[c], grid[c], tune_queue + 1, fv::STAGE_RK_2,
+                        0);
       cudaEventRecord(e1, b->stream);
       if (e != cudaSuccess) {
         grid[c] = 0;  // not launchable: drop it
@@ -582,9 +628,10 @@ int Prepare(fv_batch* b) {
     int rc = Autotune(b, g);
     if (rc) return rc;
     std::vector<BatchInst> d = Describe(b, g, g.shape, b->d_ctrl, &g.ntiles, g.rows);
+    g.one = d[0];
     BCUDA(b, cudaMalloc(&g.d_inst, sizeof(BatchInst) * d.size()));
     BCUDA(b, cudaMemcpyAsync(g.d_inst, d.data(), sizeof(BatchInst) * d.size(), cudaMemcpyHostToDevice, b->stream));
-    g.grid = std::max(1, std::min(Occupancy(b, g, g.shape) * SmCount(), g.ntiles));
+    g.grid = GridFor(b, g, g.shape, Occupancy(b, g, g.shape), g.ntiles);
   }
   BCUDA(b, cudaStreamSynchronize(b->stream));
   b->prepared = true;
@@ -603,7 +650,7 @@ bool MultiEligible(const fv_batch* b) {
   if (b->precision != FV_PREC_FP32_MIXED || b->ts != FV_TS_RK2 || b->groups.size() != 1) return false;
   const Group& g = b->groups[0];
   if (g.ndim != 2 || (int)g.members.size() > fv::batch_multi_problems32()) return false;
-  if (ShapeSchedule(b, g.shape).vface) return false;  // multi-step kernels: the fused viscous form
+  if (!fv::batch_shape_marched32(g.shape)) return false;  // the multi-step kernels march by warps
   const char* env = std::getenv("FV3D_MULTISTEP");
   if (env && env[0] == '0') return false;
   long long cells = 0;
@@ -611,30 +658,28 @@ bool MultiEligible(const fv_batch* b) {
   return cells <= kMultiMaxCells || (env && env[0] == '1');
 }
 
-// Descriptors of the multi-step launch: the group's strip width, rows per
-// work item that give each resident CTA about one item (4 to 64; measured on
-// Sedov 128^2 / 256^2 / 512^2 and 16 Sod tubes of 96^2, this count was the
-// fastest of 4 / 8 / 16 / 32 rows each time; FV3D_MULTI_ROWS forces it).
+// Descriptors of the multi-step launch: the fewest rows per work item that
+// give each resident warp at most one item (the items are assigned
+// statically, so a second round of them would wait for the first;
+// FV3D_MULTI_ROWS forces the rows).
 int PrepareMulti(fv_batch* b) {
   if (b->d_inst_multi) return FV_OK;
   Group& g = b->groups[0];
-  const int occ = fv::batch_multi_occupancy32(g.plane, g.wact, g.shape, g.tc);
+  const int occ = fv::batch_multi_occupancy32(g.plane, g.wact, g.shape, g.members.size() == 1);
   if (occ <= 0) return Fail(b, FV_ERR_CUDA, "the multi-step kernel cannot be launched");
   const fv::TileShape* shapes;
   NumShapes(b->precision, &shapes);
   const int tx = shapes[g.shape].tx;
-  long long units = 0;
-  for (int i : g.members) units += (long long)((b->G[i].na + tx - 1) / tx) * b->G[i].nb;
-  const long long slots = (long long)occ * SmCount();
-  int rows = (int)std::min(64LL, std::max(4LL, (units + slots - 1) / slots));
+  int rows = RowsForSlots(b, g, tx, (long long)occ * SmCount() * ItemsPerCta(b, g, g.shape));
   if (const char* f = std::getenv("FV3D_MULTI_ROWS")) rows = std::max(1, std::atoi(f));
   std::vector<BatchInst> d = Describe(b, g, g.shape, b->d_ctrl, &b->ntiles_multi, rows);
+  b->one_multi = d[0];
   BCUDA(b, cudaMalloc(&b->d_inst_multi, sizeof(BatchInst) * d.size()));
   BCUDA(b, cudaMemcpyAsync(b->d_inst_multi, d.data(), sizeof(BatchInst) * d.size(), cudaMemcpyHostToDevice,
                            b->stream));
   BCUDA(b, cudaStreamSynchronize(b->stream));
   b->rows_multi = rows;
-  b->grid_multi = (int)std::max(1LL, std::min((long long)b->ntiles_multi, slots));
+  b->grid_multi = GridFor(b, g, g.shape, occ, b->ntiles_multi);
   return FV_OK;
 }
 
@@ -645,8 +690,8 @@ int RunMulti(fv_batch* b, int nsteps, int mode_override) {
   BCUDA(b, cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), b->stream));
   const fv::GridBarrier gb{bar, reinterpret_cast<int*>(bar + 1)};
   const cudaError_t e = fv::launch_batch_multi32(g.plane, g.wact, g.shape, b->d_inst_multi, (int)g.members.size(),
-                                                 b->ntiles_multi, nsteps, mode_override, gb, b->grid_multi, g.tc,
-                                                 b->stream);
+                                                 b->ntiles_multi, nsteps, mode_override, gb, b->grid_multi, b->stream,
+                                                 g.members.size() == 1 ? &b->one_multi : nullptr);
   if (e != cudaSuccess) return Fail(b, FV_ERR_CUDA, "multi-step launch: %s", cudaGetErrorString(e));
   b->launches += 1;
   return FV_OK;
@@ -695,10 +740,10 @@ int EnqueueStep(fv_batch* b, int mode_override = 2, double dt = 0.0) {
     const Group& g = b->groups[gi];
     unsigned* q = b->d_queue + 2 * gi;
     if (b->ts == FV_TS_RK2) {
-      e = LaunchStage(b, g, g.d_inst, g.ntiles, g.grid, q, fv::STAGE_RK_1, 0);
-      if (e == cudaSuccess) e = LaunchStage(b, g, g.d_inst, g.ntiles, g.grid, q + 1, fv::STAGE_RK_2, 0);
+      e = LaunchStage(b, g, g.d_inst, &g.one, g.ntiles, g.grid, q, fv::STAGE_RK_1, 0);
+      if (e == cudaSuccess) e = LaunchStage(b, g, g.d_inst, &g.one, g.ntiles, g.grid, q + 1, fv::STAGE_RK_2, 0);
     } else {
-      e = LaunchStage(b, g, g.d_inst, g.ntiles, g.grid, q, fv::STAGE_EULER, b->flip);
+      e = LaunchStage(b, g, g.d_inst, &g.one, g.ntiles, g.grid, q, fv::STAGE_EULER, b->flip);
     }
   }
   if (e != cudaSuccess) return Fail(b, FV_ERR_CUDA, "batch step launch: %s", cudaGetErrorString(e));

@@ -1,11 +1,12 @@
-// fv_batch32.cu -- FP32-mixed persistent stage kernel for batches, plus the
-// mixed form's CFL reduction and its (hi, lo) pair conversions.  Built with
+// fv_batch32.cu -- dispatch of the FP32-mixed 2-D kernels: the warp-marched
+// form (fv_march32.cuh), which every mixed 2-D group takes, and the
+// shared-memory block form below, which a forced schedule (FV3D_TILE with 32-
+// or 64-wide blocks) selects; plus the mixed form's CFL reduction and its
+// (hi, lo) pair conversions.  Built with
 // fast-math (FP32 division / sqrt approximations, FMA contraction); the
 // error-free pair arithmetic of fv_tile32.cuh is written with adds and _rn
 // intrinsics, which contraction leaves alone.
-#include "fv_control.cuh"
-#include "fv_grid.cuh"
-#include "fv_tile32.cuh"
+#include "fv_march32.cuh"
 
 namespace fv {
 
@@ -18,8 +19,9 @@ namespace {
 // or split into a per-face pass (VF).  The rows of an item are a run-time
 // value (BatchInst::tz), so shapes of one kernel differ only in their
 // starting rows.
+// march: the warp-marched form (0: the block form).
 struct MixedKernel {
-  int tx, block_rows, vface;
+  int tx, block_rows, vface, march;
 };
 // Block rows of the two block heights (cells per thread in the update: 2 and
 // 1 for 32-wide blocks).
@@ -30,11 +32,11 @@ struct MixedKernel {
 #define FV_MIXED_BR_B 8
 #endif
 constexpr int kBrA = FV_MIXED_BR_A, kBrB = FV_MIXED_BR_B;
-constexpr MixedKernel kKernels32[] = {{32, kBrA, 0}, {64, kBrA, 0}, {32, kBrB, 0},
-                                      {64, kBrB, 0}, {32, kBrA, 1}, {64, kBrA, 1}};
-constexpr TileShape kShapes32[] = {{32, 2 * kBrA}, {64, kBrA},     {32, kBrA}, {64, 2 * kBrA},
-                                   {32, 2 * kBrB}, {64, kBrB},     {32, 2 * kBrA}, {64, kBrA}};
-constexpr int kKernelOf32[] = {0, 1, 0, 1, 2, 3, 4, 5};
+constexpr MixedKernel kKernels32[] = {{32, kBrA, 0, 0}, {64, kBrA, 0, 0}, {32, kBrB, 0, 0}, {64, kBrB, 0, 0},
+                                      {32, kBrA, 1, 0}, {64, kBrA, 1, 0}, {kMarchWidth, 0, 0, 1}};
+constexpr TileShape kShapes32[] = {{32, 2 * kBrA}, {64, kBrA}, {32, kBrA},     {64, 2 * kBrA},        {32, 2 * kBrB},
+                                   {64, kBrB},     {32, 2 * kBrA}, {64, kBrA}, {kMarchWidth, 32}};
+constexpr int kKernelOf32[] = {0, 1, 0, 1, 2, 3, 4, 5, 6};
 constexpr int kNumShapes32 = sizeof(kShapes32) / sizeof(kShapes32[0]);
 
 // Copies the descriptor of the problem holding work item t to s_inst and
@@ -122,109 +124,6 @@ batch_stage32(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsign
   }
 }
 
-// Problems a multi-step launch can carry (per-problem step state sits in
-// shared memory).
-constexpr int kMultiMaxProblems = 256;
-
-// Several RK2 steps of a group in one cooperative launch (every CTA
-// resident): per step, each CTA decides every problem's dt and active flag
-// itself (step_decide on the reduced CFL maximum, the same arithmetic as the
-// control kernel, so every CTA reaches the same values), then stage 1 over
-// the work items t = blockIdx.x, blockIdx.x + gridDim.x, ..., a grid
-// barrier, stage 2 (CFL maxima by atomics), a grid barrier.  Each work item
-// runs the per-stage kernel's body, so the result is bit-identical to the
-// per-stage launches.  The time and step counter of each problem are kept in
-// shared memory during the launch and written back to the control blocks at
-// its end by CTA 0; the CFL slot of the next step is zeroed by CTA 0.  A
-// barrier wait that runs out sets bit 1 of every problem's error flag and
-// the kernel returns.
-template <int PLANE, bool WACT, class TL>
-__global__ void FV_MIXED_BOUNDS batch_multi32(const BatchInst* __restrict__ insts, int ninst, int ntiles, int nsteps,
-                                              int mode_override, GridBarrier gb) {
-  extern __shared__ float smem_f[];
-  __shared__ unsigned long long s_red[kTileThreads / 32];
-  __shared__ BatchInst s_inst;
-  __shared__ double s_t[kMultiMaxProblems], s_dt[kMultiMaxProblems];
-  __shared__ long long s_step[kMultiMaxProblems];
-  __shared__ int s_act[kMultiMaxProblems], s_par[kMultiMaxProblems], s_err[kMultiMaxProblems];
-  __shared__ int s_any;
-  auto timed_out = [&]() {
-    if (threadIdx.x == 0)
-      for (int m = 0; m < ninst; ++m) atomicOr(&insts[m].ctrl->err, 2);
-  };
-  for (int m = threadIdx.x; m < ninst; m += blockDim.x) {
-    const StepCtrl* c = insts[m].ctrl;
-    s_t[m] = c->t;
-    s_step[m] = c->step;
-    s_err[m] = 0;
-  }
-  __syncthreads();
-  unsigned bar = 0;
-  // every CTA has read the initial times before CTA 0 may write any control block
-  if (!grid_sync(gb, bar++)) {
-    timed_out();
-    return;
-  }
-  int k = 0;
-  bool decided = false;
-  for (; k < nsteps; ++k) {
-    if (threadIdx.x == 0) s_any = 0;
-    __syncthreads();
-    for (int m = threadIdx.x; m < ninst; m += blockDim.x) {
-      StepCtrl* c = insts[m].ctrl;
-      double dt;
-      int active;
-      bool bad;
-      step_decide(*c, s_t[m], s_step[m], c->err | s_err[m], mode_override, 0.0, dt, active, bad);
-      const int p = (int)(s_step[m] & 1);
-      if (bad) s_err[m] = 1;
-      s_dt[m] = active ? dt : 0.0;
-      s_act[m] = active;
-      s_par[m] = p;
-      if (blockIdx.x == 0) c->slot[p ^ 1] = 0ull;  // read by no CTA in this step
-      if (active) {
-        s_t[m] = __dadd_rn(s_t[m], dt);
-        s_step[m] += 1;
-        s_any = 1;
-      }
-    }
-    __syncthreads();
-    decided = true;
-    if (!s_any) break;  // every CTA decides alike: no problem steps any more
-    // kind stays a run-time value, as in the per-stage kernel: a copy of the
-    // stage body specialised per kind may contract its multiply-adds
-    // differently and break the bit-for-bit equality with the per-stage form
-#pragma unroll 1
-    for (int kind = STAGE_RK_1; kind <= STAGE_RK_2; ++kind) {
-      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        __syncthreads();  // the previous item is finished with s_inst and smem
-        const int m = fetch_inst32(insts, ninst, t, &s_inst);
-        __syncthreads();
-        StepCtrl* ctrl = s_inst.ctrl;
-        stage_item32<PLANE, WACT, TL, false>(s_inst, t, kind, 0, s_act[m] != 0, s_dt[m], &ctrl->slot[s_par[m] ^ 1],
-                                      &ctrl->err, smem_f, s_red);
-      }
-      if (!grid_sync(gb, bar++)) {
-        timed_out();
-        return;
-      }
-    }
-  }
-  if (blockIdx.x == 0) {  // the control blocks as the per-stage launches leave them
-    for (int m = threadIdx.x; m < ninst; m += blockDim.x) {
-      StepCtrl* c = insts[m].ctrl;
-      if (decided) {
-        c->parity = s_par[m];
-        c->active = s_act[m];
-        c->dt_cur = s_dt[m];
-      }
-      c->t = s_t[m];
-      c->step = s_step[m];
-      if (s_err[m]) atomicOr(&c->err, 1);
-    }
-  }
-}
-
 template <int K>
 using BlockOf32 = Tile<kKernels32[K].tx, kKernels32[K].block_rows>;
 
@@ -241,21 +140,18 @@ size_t smem_for(bool wact, bool tc) {
 
 typedef void (*BatchKernel)(const BatchInst*, int, int, unsigned*, int, int);
 
-typedef void (*MultiKernel)(const BatchInst*, int, int, int, int, GridBarrier);
-
-template <int PLANE, bool WACT>
-MultiKernel pick_multi(int shape) {  // fused viscous form only (shapes of kernels 0-3)
-  switch (kKernelOf32[shape]) {
-    case 0: return batch_multi32<PLANE, WACT, BlockOf32<0>>;
-    case 1: return batch_multi32<PLANE, WACT, BlockOf32<1>>;
-    case 2: return batch_multi32<PLANE, WACT, BlockOf32<2>>;
-    default: return batch_multi32<PLANE, WACT, BlockOf32<3>>;
-  }
+MarchKernel march_kernel(int plane, bool wact, int kind, bool one) {
+  return plane == PLANE_XY ? march_kernel_xy(wact, kind, one) : march_kernel_xz(wact, kind, one);
 }
 
-MultiKernel pick_multi_any(int plane, bool wact, int shape) {
-  if (plane == PLANE_XY) return wact ? pick_multi<PLANE_XY, true>(shape) : pick_multi<PLANE_XY, false>(shape);
-  return wact ? pick_multi<PLANE_XZ, true>(shape) : pick_multi<PLANE_XZ, false>(shape);
+MarchMultiKernel march_multi_kernel(int plane, bool wact, bool one) {
+  return plane == PLANE_XY ? march_multi_kernel_xy(wact, one) : march_multi_kernel_xz(wact, one);
+}
+
+// A parameter every launch passes: the descriptor of a one-problem group.
+const BatchInst& one_or_empty(const BatchInst* one) {
+  static const BatchInst empty{};
+  return one ? *one : empty;
 }
 
 template <int PLANE, bool WACT>
@@ -292,16 +188,6 @@ cudaError_t prepare(int plane, bool wact, int shape) {
   if (flag) return cudaSuccess;
   cudaError_t e = cudaFuncSetAttribute(pick_any(plane, wact, shape), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem_any(shape, wact, true));
-  if (e == cudaSuccess) flag = true;
-  return e;
-}
-
-cudaError_t prepare_multi(int plane, bool wact, int shape) {
-  static bool done[2][2][kNumShapes32] = {};
-  bool& flag = done[plane == PLANE_XY ? 0 : 1][wact ? 1 : 0][shape];
-  if (flag) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(pick_multi_any(plane, wact, shape),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_any(shape, wact, true));
   if (e == cudaSuccess) flag = true;
   return e;
 }
@@ -379,7 +265,19 @@ int batch_shape_kernel32(int shape, int* block_rows, int* vface) {
   return kKernelOf32[shape];
 }
 
-int batch_stage_occupancy32(int plane, bool wact, int shape, bool tc) {
+bool batch_shape_marched32(int shape) {
+  return shape >= 0 && shape < kNumShapes32 && kKernels32[kKernelOf32[shape]].march;
+}
+
+int batch_items_per_cta32(int shape) { return batch_shape_marched32(shape) ? kMarchWarps : 1; }
+
+int batch_stage_occupancy32(int plane, bool wact, int shape, bool tc, int kind,
+                            bool one) {
+  if (batch_shape_marched32(shape)) {
+    int nb = 0;
+    const MarchKernel k = march_kernel(plane, wact, kind, one);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kMarchThreads, 0) == cudaSuccess ? nb : 0;
+  }
   if (shape < 0 || shape >= kNumShapes32 || prepare(plane, wact, shape) != cudaSuccess) return 0;
   int nb = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_any(plane, wact, shape), kTileThreads,
@@ -389,8 +287,14 @@ int batch_stage_occupancy32(int plane, bool wact, int shape, bool tc) {
 }
 
 cudaError_t launch_batch_stage32(int plane, bool wact, int shape, const BatchInst* insts, int ninst, int ntiles,
-                                 unsigned* queue, int kind, int flip, int grid, bool tc, cudaStream_t st) {
+                                 unsigned* queue, int kind, int flip, int grid, bool tc, cudaStream_t st,
+                                 const BatchInst* one) {
   if (shape < 0 || shape >= kNumShapes32) return cudaErrorInvalidValue;
+  if (batch_shape_marched32(shape)) {
+    const cudaError_t e = launch_pdl(march_kernel(plane, wact, kind, one != nullptr), dim3(grid), dim3(kMarchThreads),
+                                     0, st, insts, ninst, ntiles, queue, flip, one_or_empty(one));
+    return e != cudaSuccess ? e : cudaGetLastError();
+  }
   cudaError_t e = prepare(plane, wact, shape);
   if (e != cudaSuccess) return e;
   e = launch_pdl(pick_any(plane, wact, shape), dim3(grid), dim3(kTileThreads), smem_any(shape, wact, tc), st, insts,
@@ -400,32 +304,28 @@ cudaError_t launch_batch_stage32(int plane, bool wact, int shape, const BatchIns
 
 int batch_multi_problems32() { return kMultiMaxProblems; }
 
-int batch_multi_occupancy32(int plane, bool wact, int shape, bool tc) {
-  if (shape < 0 || shape >= kNumShapes32 || prepare_multi(plane, wact, shape) != cudaSuccess) return 0;
+int batch_multi_occupancy32(int plane, bool wact, int shape, bool one) {
+  if (!batch_shape_marched32(shape)) return 0;
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_multi_any(plane, wact, shape), kTileThreads,
-                                                    smem_any(shape, wact, tc)) != cudaSuccess)
-    return 0;
-  return nb;
+  const MarchMultiKernel k = march_multi_kernel(plane, wact, one);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kMarchThreads, 0) == cudaSuccess ? nb : 0;
 }
 
 cudaError_t launch_batch_multi32(int plane, bool wact, int shape, const BatchInst* insts, int ninst, int ntiles,
-                                 int nsteps, int mode_override, GridBarrier gb, int grid, bool tc,
-                                 cudaStream_t st) {
-  if (shape < 0 || shape >= kNumShapes32 || ninst > kMultiMaxProblems) return cudaErrorInvalidValue;
-  cudaError_t e = prepare_multi(plane, wact, shape);
-  if (e != cudaSuccess) return e;
+                                 int nsteps, int mode_override, GridBarrier gb, int grid, cudaStream_t st,
+                                 const BatchInst* one) {
+  if (!batch_shape_marched32(shape) || ninst > kMultiMaxProblems) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kTileThreads);
-  cfg.dynamicSmemBytes = smem_any(shape, wact, tc);
+  cfg.blockDim = dim3(kMarchThreads);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;  // every CTA resident: the grid barriers need it
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, pick_multi_any(plane, wact, shape), insts, ninst, ntiles, nsteps, mode_override, gb);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, march_multi_kernel(plane, wact, one != nullptr), insts, ninst, ntiles,
+                                           nsteps, mode_override, gb, one_or_empty(one));
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -15,6 +15,9 @@
 namespace fv {
 
 constexpr int kGridBarrierPolls = 1 << 24;
+// Polls before the wait sleeps between them: a small grid's stages end within
+// microseconds of one another, and a sleep there lengthens every step.
+constexpr int kGridBarrierSpins = 256;
 
 struct GridBarrier {
   unsigned* count;  // arrivals so far
@@ -43,7 +46,7 @@ __device__ __forceinline__ bool grid_sync(const GridBarrier& gb, unsigned k, int
         atomicExch(gb.abort, 1);
         break;
       }
-      __nanosleep(64);
+      if (polls > kGridBarrierSpins) __nanosleep(64);
     }
     __threadfence();
     s_ok = ok;

@@ -168,6 +168,10 @@ int batch_tile_shapes32(const TileShape** shapes);
 // differ only in their starting rows), its block rows (8 or 16) and whether
 // it computes the viscous fluxes in a per-face pass (1) or per cell (0).
 int batch_shape_kernel32(int shape, int* block_rows, int* vface);
+// Whether FP32-mixed shape `shape` is marched by warps (fv_march32.cuh), one
+// work item per warp, and how many items a CTA of it has in flight.
+bool batch_shape_marched32(int shape);
+int batch_items_per_cta32(int shape);
 
 // Persistent stage kernel over a group of problems sharing plane and third
 // momentum: `grid` CTAs pull tiles from the work-queue counter *queue (reset
@@ -176,11 +180,14 @@ int batch_shape_kernel32(int shape, int* block_rows, int* vface);
 // temperature tile.  Shape indexes batch_tile_shapes64/32.
 cudaError_t launch_batch_stage64(int plane, bool wact, int shape, const BatchInst* insts, int ninst, int ntiles,
                                  unsigned* queue, int kind, int flip, int grid, bool tc, cudaStream_t stream);
+// one (FP32-mixed, a group of one problem): the host copy of its descriptor,
+// which the warp-marched kernels then read from the launch parameters.
 cudaError_t launch_batch_stage32(int plane, bool wact, int shape, const BatchInst* insts, int ninst, int ntiles,
-                                 unsigned* queue, int kind, int flip, int grid, bool tc, cudaStream_t stream);
+                                 unsigned* queue, int kind, int flip, int grid, bool tc, cudaStream_t stream,
+                                 const BatchInst* one);
 // Resident CTAs per SM of one batch stage kernel (0 on error).
 int batch_stage_occupancy64(int plane, bool wact, int shape, bool tc);
-int batch_stage_occupancy32(int plane, bool wact, int shape, bool tc);
+int batch_stage_occupancy32(int plane, bool wact, int shape, bool tc, int kind, bool one);
 
 // Persistent stage kernels for groups of 3-D problems sharing a Riemann
 // solver (rs): a work item is a 16 x 16 column block and a chunk of tz z
@@ -197,17 +204,17 @@ int batch_stage3d_occupancy64(int rs, bool tc);
 int batch_stage3d_occupancy32(int rs, bool tc);
 
 // Several RK2 steps of a group of FP32-mixed 2-D problems in one cooperative
-// launch (fv_batch32.cu, batch_multi32): for small grids, whose steps are
-// bound by launch latency.  At most batch_multi_problems32() problems; grid
-// at most batch_multi_occupancy32() x SMs CTAs (all resident); the barrier
-// counter and abort flag of gb zeroed before the launch; a grid-barrier wait
-// that runs out sets bit 1 of every problem's error flag.  mode_override as
-// launch_control.
+// launch (fv_march32.cuh, march_multi32; marched shapes only): for small
+// grids, whose steps are bound by launch latency.  At most
+// batch_multi_problems32() problems; grid at most batch_multi_occupancy32() x
+// SMs CTAs (all resident); the barrier counter and abort flag of gb zeroed
+// before the launch; a grid-barrier wait that runs out sets bit 1 of every
+// problem's error flag.  mode_override as launch_control.
 int batch_multi_problems32();
-int batch_multi_occupancy32(int plane, bool wact, int shape, bool tc);
+int batch_multi_occupancy32(int plane, bool wact, int shape, bool one);
 cudaError_t launch_batch_multi32(int plane, bool wact, int shape, const BatchInst* insts, int ninst, int ntiles,
-                                 int nsteps, int mode_override, GridBarrier gb, int grid, bool tc,
-                                 cudaStream_t stream);
+                                 int nsteps, int mode_override, GridBarrier gb, int grid, cudaStream_t stream,
+                                 const BatchInst* one);
 
 // launch_control for n problems plus a reset of nq work-queue counters.
 cudaError_t launch_batch_control(StepCtrl* ctrl, int n, unsigned* queue, int nq, int mode_override, double dt_given,
