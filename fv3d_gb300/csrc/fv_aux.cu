@@ -20,15 +20,17 @@ int grid_for(long long n, int block) {
 template <int PLANE, bool WACT>
 __global__ void __launch_bounds__(256) reduce2d_fp64(const Grid G, const Fields u, StepCtrl* ctrl, int slot) {
   __shared__ unsigned long long s_red[8];
+  opaque64_init();
+  __syncthreads();
   unsigned long long red = 0ull;
   const long long n = (long long)G.na * G.rows;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
     const int y = (int)(c / G.na), x = (int)(c - (long long)y * G.na);
     const long long o = (long long)y * G.pitch + x;
-    double w[5];
+    X64 w[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) w[v] = (WACT || v != 3) ? u.f[v][o] : 0.0;
-    const double inv = inv_dt_hyp64<PLANE, WACT>(w, G);
+    const double inv = inv_dt_hyp64<PLANE, WACT>(w, G).v;
     const unsigned long long b = (unsigned long long)__double_as_longlong(inv);
     red = b > red ? b : red;
     if (!(inv <= 1.0e300)) atomicOr(&ctrl->err, 1);
@@ -81,6 +83,8 @@ template <int PLANE, bool WACT, bool REDUCE>
 __global__ void __launch_bounds__(256) prim_to_cons_from(const Grid G, const Fields src, const Fields dst,
                                                          StepCtrl* ctrl, int slot, const Fields qout, int* q_valid) {
   __shared__ unsigned long long s_red[8];
+  opaque64_init();
+  __syncthreads();
   unsigned long long red = 0ull;
   const long long n = (long long)G.na * G.rows;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
@@ -100,21 +104,21 @@ __global__ void __launch_bounds__(256) prim_to_cons_from(const Grid G, const Fie
     if (WACT) dst.f[3][o] = mc;
     dst.f[4][o] = E;
     if (REDUCE || qout.f[0]) {
-      const double u[5] = {r, ma, mb, mc, E};
-      double q[5];
+      const X64 u[5] = {r, ma, mb, mc, E};
+      X64 q[5];
       if (REDUCE) {
-        const double inv = inv_dt_hyp64<PLANE, WACT>(u, G, q);
+        const double inv = inv_dt_hyp64<PLANE, WACT>(u, G, q).v;
         const unsigned long long b = (unsigned long long)__double_as_longlong(inv);
         red = b > red ? b : red;
         if (!(inv <= 1.0e300)) atomicOr(&ctrl->err, 1);
       } else {
-        double y;
+        X64 y;
         cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
       }
       if (qout.f[0]) {
 #pragma unroll
         for (int v = 0; v < 5; ++v)
-          if (WACT || v != 3) qout.f[v][o] = q[v];
+          if (WACT || v != 3) qout.f[v][o] = q[v].v;
       }
     }
   }

@@ -48,6 +48,7 @@ batch_stage64(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsign
   __shared__ unsigned long long s_red[kTileThreads / 32];
   __shared__ BatchInst s_inst;
   __shared__ int s_tile;
+  opaque64_init();  // the first use follows the __syncthreads below
   pdl_wait();
   for (;;) {
     __syncthreads();  // the previous item is finished with s_tile, s_inst and smem

@@ -26,44 +26,44 @@ __device__ __forceinline__ constexpr int phys_slot(int var) {
 // dropped.  The three divisions by rho share one correctly rounded
 // reciprocal (Markstein correction, fv_exact64.cuh).
 template <int PLANE, bool WACT>
-__device__ __forceinline__ void cons_to_prim64(const double u[5], double gm1, double q[5], double& y) {
-  const double r = u[0];
-  y = 1.0 / r;
-  const double va = div_by_rcp(u[1], r, y);
-  const double vb = div_by_rcp(u[2], r, y);
-  const double vc = WACT ? div_by_rcp(u[3], r, y) : 0.0;
-  double ke;
+__device__ __forceinline__ void cons_to_prim64(const X64 u[5], X64 gm1, X64 q[5], X64& y) {
+  const X64 r = u[0];
+  y = rcp64(r);
+  const X64 va = div_by_rcp(u[1], r, y);
+  const X64 vb = div_by_rcp(u[2], r, y);
+  const X64 vc = WACT ? div_by_rcp(u[3], r, y) : X64(0.0);
+  X64 ke;
   if (WACT) {
-    const double vx = va, vy = PLANE == PLANE_XY ? vb : vc, vz = PLANE == PLANE_XY ? vc : vb;
-    ke = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
+    const X64 vx = va, vy = PLANE == PLANE_XY ? vb : vc, vz = PLANE == PLANE_XY ? vc : vb;
+    ke = vx * vx + vy * vy + vz * vz;
   } else {
-    ke = __dadd_rn(__dmul_rn(va, va), __dmul_rn(vb, vb));
+    ke = va * va + vb * vb;
   }
-  const double Ek = __dmul_rn(half64(r), ke);
+  const X64 Ek = half_of(r) * ke;
   q[0] = r;
   q[1] = va;
   q[2] = vb;
   q[3] = vc;
-  q[4] = __dmul_rn(__dsub_rn(u[4], Ek), gm1);
+  q[4] = (u[4] - Ek) * gm1;
 }
 
 // Hyperbolic inverse time step of one cell, ComputeDt.h:49-52:
 // (cs + |u|)/dx + (cs + |v|)/dy + (cs + |w|)/dz with cs = sqrt(p*gamma/rho).
 // qout, when given, receives the primitives consToPrim computes on the way.
 template <int PLANE, bool WACT, bool P2 = false>
-__device__ __forceinline__ double inv_dt_hyp64(const double u[5], const Grid& G, double* qout = nullptr) {
-  double q[5], y;
+__device__ __forceinline__ X64 inv_dt_hyp64(const X64 u[5], const Grid& G, X64* qout = nullptr) {
+  X64 q[5], y;
   cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
   if (qout) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) qout[v] = q[v];
   }
-  const double cs = sqrt(div_by_rcp(__dmul_rn(q[4], G.gamma), q[0], y));
-  const double vx = q[1], vy = PLANE == PLANE_XY ? q[2] : q[3], vz = PLANE == PLANE_XY ? q[3] : q[2];
-  const double tx = div_cell<P2>(__dadd_rn(cs, fabs(vx)), G.dx, G.inv_dx);
-  const double ty = div_cell<P2>(__dadd_rn(cs, fabs(vy)), G.dy, G.inv_dy);
-  const double tz = div_cell<P2>(__dadd_rn(cs, fabs(vz)), G.dz, G.inv_dz);
-  return __dadd_rn(__dadd_rn(tx, ty), tz);
+  const X64 cs = sqrt64(div_by_rcp(q[4] * G.gamma, q[0], y));
+  const X64 vx = q[1], vy = PLANE == PLANE_XY ? q[2] : q[3], vz = PLANE == PLANE_XY ? q[3] : q[2];
+  const X64 tx = div_cell<P2>(cs + fabs(vx.v), G.dx, G.inv_dx);
+  const X64 ty = div_cell<P2>(cs + fabs(vy.v), G.dy, G.inv_dy);
+  const X64 tz = div_cell<P2>(cs + fabs(vz.v), G.dz, G.inv_dz);
+  return tx + ty + tz;
 }
 
 // Block-wide max of non-negative doubles held as bit patterns (IEEE order of

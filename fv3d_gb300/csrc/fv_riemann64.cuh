@@ -12,10 +12,9 @@
 //   - HLLC's max(cL, cR) as sqrt(max(cL^2, cR^2)) (sqrt is monotone and
 //     correctly rounded), and u*, p* / the star state share reciprocals;
 //   - products with 0.5 by exponent arithmetic (half64, exact);
-//   - HLLC's wave-speed min / max and region tests on bit patterns
-//     (fmin_bits, gt0_bits, ...: integer pipe, same results; measured
-//     +1-2 %).  HLL keeps the FP64 forms: there the bit-pattern min / max
-//     measured 1 % slower.
+//   - wave-speed min / max and region tests on bit patterns (fmin_bits,
+//     gt0_bits, ...: integer pipe, same results; an FP64 comparison takes 19
+//     cycles of the FP64 pipe).
 #pragma once
 
 #include "fv_device.cuh"
@@ -25,7 +24,7 @@ namespace fv {
 
 // (u^2 + t1^2) + t2^2 with the exact zero slot dropped.
 template <int ZS>
-__device__ __forceinline__ double ke_sum3(double un, double t1, double t2) {
+__device__ __forceinline__ X64 ke_sum3(X64 un, X64 t1, X64 t2) {
   if (ZS == 1) return un * un + t2 * t2;
   if (ZS == 2) return un * un + t1 * t1;
   return (un * un + t1 * t1) + t2 * t2;
@@ -33,9 +32,9 @@ __device__ __forceinline__ double ke_sum3(double un, double t1, double t2) {
 
 // computeFlux (States.h:114-127) given e = p/(gamma-1).
 template <int ZS>
-__device__ __forceinline__ void euler_flux64(const Slots<double>& q, double e, double F[5]) {
-  const double Ek = half64(q.r) * ke_sum3<ZS>(q.un, q.t1, q.t2);
-  const double E = e + Ek;
+__device__ __forceinline__ void euler_flux64(const Slots<X64>& q, X64 e, X64 F[5]) {
+  const X64 Ek = half_of(q.r) * ke_sum3<ZS>(q.un, q.t1, q.t2);
+  const X64 E = e + Ek;
   F[0] = q.r * q.un;
   F[1] = F[0] * q.un + q.p;
   F[2] = ZS == 1 ? 0.0 : F[0] * q.t1;
@@ -45,12 +44,12 @@ __device__ __forceinline__ void euler_flux64(const Slots<double>& q, double e, d
 
 // primToCons (States.h:20-31) given e = p/(gamma-1) and y = RN(1/rho).
 template <int ZS>
-__device__ __forceinline__ void prim_to_cons64(const Slots<double>& q, double e, double y, double u[5]) {
+__device__ __forceinline__ void prim_to_cons64(const Slots<X64>& q, X64 e, X64 y, X64 u[5]) {
   u[0] = q.r;
   u[1] = q.r * q.un;
   u[2] = ZS == 1 ? 0.0 : q.r * q.t1;
   u[3] = ZS == 2 ? 0.0 : q.r * q.t2;
-  const double Ek = div_by_rcp(half64(ke_sum3<ZS>(u[1], u[2], u[3])), q.r, y);
+  const X64 Ek = div_by_rcp(half_of(ke_sum3<ZS>(u[1], u[2], u[3])), q.r, y);
   u[4] = Ek + e;
 }
 
@@ -58,36 +57,36 @@ __device__ __forceinline__ void prim_to_cons64(const Slots<double>& q, double e,
 // pout, when given, receives the interface pressure of RiemannSolvers.h:24-33
 // (used only by the z-boundary flux overrides of Update.h:131-143).
 template <int ZS>
-__device__ __forceinline__ void hll64(const Slots<double>& L, const Slots<double>& R, const Consts64& K,
-                                      double flux[5], double* pout = nullptr) {
+__device__ __forceinline__ void hll64(const Slots<X64>& L, const Slots<X64>& R, const Consts64& K,
+                                      X64 flux[5], X64* pout = nullptr) {
   // one correctly rounded reciprocal of each density serves both quotients by
   // it (the sound speed's p*gamma/rho and, in the star region, Ek/rho)
-  const double yL = 1.0 / L.r, yR = 1.0 / R.r;
-  const double aL = sqrt(div_by_rcp(L.p * K.gamma, L.r, yL));
-  const double aR = sqrt(div_by_rcp(R.p * K.gamma, R.r, yR));
-  const double SL = fmin(L.un - aL, R.un - aR);
-  const double SR = fmax(L.un + aL, R.un + aR);
-  const double eL = div_by_rcp(L.p, K.gm1, K.inv_gm1);
-  const double eR = div_by_rcp(R.p, K.gm1, K.inv_gm1);
-  double FL[5], FR[5];
+  const X64 yL = rcp64(L.r), yR = rcp64(R.r);
+  const X64 aL = sqrt64(div_by_rcp(L.p * K.gamma, L.r, yL));
+  const X64 aR = sqrt64(div_by_rcp(R.p * K.gamma, R.r, yR));
+  const X64 SL = fmin_bits(L.un - aL, R.un - aR);
+  const X64 SR = fmax_bits(L.un + aL, R.un + aR);
+  const X64 eL = div_by_rcp(L.p, K.gm1, K.inv_gm1);
+  const X64 eR = div_by_rcp(R.p, K.gm1, K.inv_gm1);
+  X64 FL[5], FR[5];
   euler_flux64<ZS>(L, eL, FL);
   euler_flux64<ZS>(R, eR, FR);
-  if (SL >= 0.0) {
+  if (ge0_bits(SL)) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) flux[v] = FL[v];
     if (pout) *pout = L.p;
-  } else if (SR <= 0.0) {
+  } else if (le0_bits(SR)) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) flux[v] = FR[v];
     if (pout) *pout = R.p;
   } else {
-    if (pout) *pout = half64(L.p + R.p);
-    double uL[5], uR[5];
+    if (pout) *pout = half_of(L.p + R.p);
+    X64 uL[5], uR[5];
     prim_to_cons64<ZS>(L, eL, yL, uL);
     prim_to_cons64<ZS>(R, eR, yR, uR);
-    const double slsr = SL * SR;
-    const double den = SR - SL;
-    const double y = 1.0 / den;
+    const X64 slsr = SL * SR;
+    const X64 den = SR - SL;
+    const X64 y = rcp64(den);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       if ((ZS == 1 && v == 2) || (ZS == 2 && v == 3)) {
@@ -104,36 +103,36 @@ __device__ __forceinline__ void hll64(const Slots<double>& L, const Slots<double
 // pout as for hll64 (RiemannSolvers.h:81-104: pL, p*, p*, pR by region).
 // KE3 (corrected physics): the kinetic energy of all three velocities.
 template <int ZS, bool KE3 = false>
-__device__ __forceinline__ void hllc64(const Slots<double>& L, const Slots<double>& R, const Consts64& K,
-                                       double flux[5], double* pout = nullptr) {
-  const double rL = L.r, uL = L.un, pL = L.p;
-  const double rR = R.r, uR = R.un, pR = R.p;
-  const double kL = KE3 ? ke_sum3<ZS>(uL, L.t1, L.t2) : (ZS == 1 ? uL * uL : uL * uL + L.t1 * L.t1);
-  const double kR = KE3 ? ke_sum3<ZS>(uR, R.t1, R.t2) : (ZS == 1 ? uR * uR : uR * uR + R.t1 * R.t1);
-  const double EL = half64(rL) * kL + pL * K.inv_gm1;
-  const double ER = half64(rR) * kR + pR * K.inv_gm1;
-  const double c2L = pL * K.gamma / rL;
-  const double c2R = pR * K.gamma / rR;
-  const double cmax = sqrt(fmax_bits(c2L, c2R));
-  const double SL = fmin_bits(uL, uR) - cmax;
-  const double SR = fmax_bits(uL, uR) + cmax;
-  const double rcL = rL * (uL - SL);
-  const double rcR = rR * (SR - uR);
-  const double D = rcR + rcL;
-  const double yD = 1.0 / D;
-  const double uS = div_by_rcp(rcR * uR + rcL * uL + (pL - pR), D, yD);
-  const double pS = div_by_rcp(rcR * pL + rcL * pR + rcL * rcR * (uL - uR), D, yD);
-  double sr, su, st1, st2, sp, E;
+__device__ __forceinline__ void hllc64(const Slots<X64>& L, const Slots<X64>& R, const Consts64& K,
+                                       X64 flux[5], X64* pout = nullptr) {
+  const X64 rL = L.r, uL = L.un, pL = L.p;
+  const X64 rR = R.r, uR = R.un, pR = R.p;
+  const X64 kL = KE3 ? ke_sum3<ZS>(uL, L.t1, L.t2) : (ZS == 1 ? uL * uL : uL * uL + L.t1 * L.t1);
+  const X64 kR = KE3 ? ke_sum3<ZS>(uR, R.t1, R.t2) : (ZS == 1 ? uR * uR : uR * uR + R.t1 * R.t1);
+  const X64 EL = half_of(rL) * kL + pL * K.inv_gm1;
+  const X64 ER = half_of(rR) * kR + pR * K.inv_gm1;
+  const X64 c2L = div64(pL * K.gamma, rL);
+  const X64 c2R = div64(pR * K.gamma, rR);
+  const X64 cmax = sqrt64(fmax_bits(c2L, c2R));
+  const X64 SL = fmin_bits(uL, uR) - cmax;
+  const X64 SR = fmax_bits(uL, uR) + cmax;
+  const X64 rcL = rL * (uL - SL);
+  const X64 rcR = rR * (SR - uR);
+  const X64 D = rcR + rcL;
+  const X64 yD = rcp64(D);
+  const X64 uS = div_by_rcp(rcR * uR + rcL * uL + (pL - pR), D, yD);
+  const X64 pS = div_by_rcp(rcR * pL + rcL * pR + rcL * rcR * (uL - uR), D, yD);
+  X64 sr, su, st1, st2, sp, E;
   if (gt0_bits(SL)) {
     sr = rL; su = uL; st1 = L.t1; st2 = L.t2; sp = pL; E = EL;
   } else if (gt0_bits(uS) || gt0_bits(SR)) {
     // star regions, tested in the reference's order: uS > 0 -> left star,
     // otherwise SR > 0 -> right star
     const bool left = gt0_bits(uS);
-    const double rK = left ? rL : rR, uK = left ? uL : uR, pK = left ? pL : pR, EK = left ? EL : ER;
-    const double SK = left ? SL : SR;
-    const double den = SK - uS;
-    const double y = 1.0 / den;
+    const X64 rK = left ? rL : rR, uK = left ? uL : uR, pK = left ? pL : pR, EK = left ? EL : ER;
+    const X64 SK = left ? SL : SR;
+    const X64 den = SK - uS;
+    const X64 y = rcp64(den);
     sr = div_by_rcp(rK * (SK - uK), den, y);
     E = div_by_rcp((SK - uK) * EK - pK * uK + pS * uS, den, y);
     su = uS;

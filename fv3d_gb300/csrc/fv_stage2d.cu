@@ -22,12 +22,16 @@ constexpr size_t kSmemAlign = 128;
 
 template <int PLANE, int RS, int KIND, bool WACT>
 __global__ void __launch_bounds__(kTileThreads, WACT ? FV_FP64_MIN_CTAS_W : FV_FP64_MIN_CTAS)
-stage2d_fp64(const Grid G, const Fields uin, const Fields u0, const Fields uout, StepCtrl* __restrict__ ctrl,
+stage2d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u0, const Fields uout, StepCtrl* __restrict__ ctrl,
              const Fields hout, long long units, const __grid_constant__ TmaState tin, int use_tma, const Fields qin,
              const Fields qout, const __grid_constant__ TmaState tq, int use_tq) {
   extern __shared__ __align__(128) unsigned char smem_bytes[];
   __shared__ unsigned long long s_red[kTileThreads / 32];
   __shared__ __align__(8) unsigned long long s_mbar;
+  __shared__ Grid s_grid;
+  const Grid& G = s_grid;
+  param_to_shared(grid, s_grid);
+  opaque64_init();
   const unsigned sa = smem_u32(smem_bytes);
   double* smem = reinterpret_cast<double*>(smem_bytes + (((sa + kSmemAlign - 1) & ~(unsigned)(kSmemAlign - 1)) - sa));
   pdl_wait();
@@ -36,8 +40,8 @@ stage2d_fp64(const Grid G, const Fields uin, const Fields u0, const Fields uout,
       mbar_init(&s_mbar, 1);
       fence_mbar_init();
     }
-    __syncthreads();
   }
+  __syncthreads();
   // the primitive copy of uin, when the last stage that wrote uin left one
   const bool prims = qin.f[0] != nullptr && ctrl->q_valid != 0;
   const Fields* qi = prims ? &qin : nullptr;

@@ -68,15 +68,15 @@ __device__ __forceinline__ int slot_of(int kg) { return (kg + 4) & 3; }
 // consToPrim of one stored cell (x, y, z storage order), RN(1/rho) in y.
 // With qsrc (the primitive copy of u, the same bits) the primitives are read
 // and y is computed only when need_y.
-__device__ __forceinline__ void load_prim(const Fields& u, const Fields* qsrc, long long o, double gm1, double q[5],
-                                          double& y, bool need_y = false) {
+__device__ __forceinline__ void load_prim(const Fields& u, const Fields* qsrc, long long o, X64 gm1, X64 q[5],
+                                          X64& y, bool need_y = false) {
   if (qsrc) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) q[v] = qsrc->f[v][o];
-    y = need_y ? 1.0 / q[0] : 0.0;
+    y = need_y ? rcp64(q[0]) : X64(0.0);
     return;
   }
-  double w[5];
+  X64 w[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) w[v] = u.f[v][o];
   cons_to_prim64<PLANE_XY, true>(w, gm1, q, y);
@@ -87,10 +87,10 @@ __device__ __forceinline__ void load_prim(const Fields& u, const Fields* qsrc, l
 // Note the reference scales the hydrostatic term by params.gravity, the
 // boolean, not by g.
 __device__ __forceinline__ void c91_ghost(const Grid& G, const Fields& u, const Fields* qsrc, long long col, bool fa,
-                                          bool fb, int kg, double res[5]) {
+                                          bool fb, int kg, X64 res[5]) {
   const int kref = kg < 0 ? 0 : G.nc - 1;
   const int ksym = kg < 0 ? -kg - 1 : 2 * G.nc - kg - 1;
-  double qref[5], qsym[5], y;
+  X64 qref[5], qsym[5], y;
   load_prim(u, qsrc, (long long)kref * G.nb * G.pitch + col, G.gm1, qref, y);
   load_prim(u, qsrc, (long long)ksym * G.nb * G.pitch + col, G.gm1, qsym, y);
   if (fa) {
@@ -101,30 +101,30 @@ __device__ __forceinline__ void c91_ghost(const Grid& G, const Fields& u, const 
     qref[2] = -qref[2];
     qsym[2] = -qsym[2];
   }
-  const double grav = G.gravity_flag ? 1.0 : 0.0;
-  const double posz = G.zmin + ((double)kg + 0.5) * G.dz;
+  const X64 grav = G.gravity_flag ? 1.0 : 0.0;
+  const X64 posz = X64(G.zmin) + (X64((double)kg) + 0.5) * G.dz;
   if (kg < 0) {
-    const double dz = posz - 0.5 * G.dz;
-    const double T = 1.0 + posz * G.theta1;
-    double p = qref[4] + dz * qref[0] * grav;
-    double r = p / T;
-    p = fmax(p, 1.0e-6);
-    r = fmax(r, 1.0e-6);
-    const double dratio = qsym[0] / r;
+    const X64 dz = posz - X64(0.5) * G.dz;
+    const X64 T = X64(1.0) + posz * G.theta1;
+    X64 p = qref[4] + dz * qref[0] * grav;
+    X64 r = div64(p, T);
+    p = fmax(p.v, 1.0e-6);
+    r = fmax(r.v, 1.0e-6);
+    const X64 dratio = div64(qsym[0], r);
     res[0] = r;
     res[1] = qsym[1];
     res[2] = qsym[2];
     res[3] = -qsym[3] * dratio;
     res[4] = p;
   } else {
-    const double Tref = qref[4] / qref[0];
-    const double dz = posz - (1.0 - 0.5 * G.dz);
-    const double T = Tref + dz * G.theta1;
-    const double P = qref[4] + dz * qref[0] * grav;
-    const double rho = P / T;
-    res[4] = fmax(P, 1.0e-6);
-    res[0] = fmax(rho, 1.0e-6);
-    const double dratio = qsym[0] / rho;
+    const X64 Tref = div64(qref[4], qref[0]);
+    const X64 dz = posz - (X64(1.0) - X64(0.5) * G.dz);
+    const X64 T = Tref + dz * G.theta1;
+    const X64 P = qref[4] + dz * qref[0] * grav;
+    const X64 rho = div64(P, T);
+    res[4] = fmax(P.v, 1.0e-6);
+    res[0] = fmax(rho.v, 1.0e-6);
+    const X64 dratio = div64(qsym[0], rho);
     res[1] = qsym[1] * dratio;
     res[2] = qsym[2] * dratio;
     res[3] = -qsym[3] * dratio;
@@ -146,10 +146,10 @@ __device__ __forceinline__ void load_layer(const Grid& G, const Fields& u, const
     const int sa = bc_source(x0 + hx - 2, G.na, G.bc_a, fa);
     const int sb = bc_source(y0 + hy - 2, G.nb, G.bc_b, fb);
     const long long col = (long long)sb * G.pitch + sa;
-    double q[5];
-    double T = 0.0;
+    X64 q[5];
+    X64 T = 0.0;
     if (!c91) {
-      double y;
+      X64 y;
       load_prim(u, qsrc, zoff + col, G.gm1, q, y, G.tc != 0);
       if (fa) q[1] = -q[1];
       if (fb) q[2] = -q[2];
@@ -157,19 +157,19 @@ __device__ __forceinline__ void load_layer(const Grid& G, const Fields& u, const
       if (G.tc) T = div_by_rcp(q[4], q[0], y);
     } else {
       c91_ghost(G, u, qsrc, col, fa, fb, kg, q);
-      if (G.tc) T = q[4] / q[0];
+      if (G.tc) T = div64(q[4], q[0]);
     }
 #pragma unroll
-    for (int v = 0; v < 5; ++v) S.q(s, v, hy, hx) = q[v];
-    if (G.tc) S.temp(s, hy, hx) = T;
+    for (int v = 0; v < 5; ++v) S.q(s, v, hy, hx) = q[v].v;
+    if (G.tc) S.temp(s, hy, hx) = T.v;
   }
 }
 
 // Slots of a sweep from (r, u, v, w, p): IX (u, v, w), IY (v, u, w),
 // IZ (w, v, u) -- swap_component, States.h:104-111.
 template <int DIR>
-__device__ __forceinline__ Slots<double> slots3(const double q[5]) {
-  Slots<double> s;
+__device__ __forceinline__ Slots<X64> slots3(const X64 q[5]) {
+  Slots<X64> s;
   s.r = q[0];
   s.p = q[4];
   s.un = DIR == 0 ? q[1] : (DIR == 1 ? q[2] : q[3]);
@@ -179,7 +179,7 @@ __device__ __forceinline__ Slots<double> slots3(const double q[5]) {
 }
 
 template <int DIR>
-__device__ __forceinline__ void unslot3(const double f[5], double out[5]) {
+__device__ __forceinline__ void unslot3(const X64 f[5], X64 out[5]) {
   out[0] = f[0];
   out[4] = f[4];
   if (DIR == 0) {
@@ -199,15 +199,15 @@ __device__ __forceinline__ void unslot3(const double f[5], double out[5]) {
 // CORR: corrected physics (HLLC with the kinetic energy of all three
 // velocities).
 template <int DIR, bool CORR>
-__device__ __forceinline__ void face3(const double c[4][5], int rs, int recon, const Grid& G, const Consts64& K,
-                                      double out[5], double* pout) {
-  double qL[5], qR[5];
+__device__ __forceinline__ void face3(const X64 c[4][5], int rs, int recon, const Grid& G, const Consts64& K,
+                                      X64 out[5], X64* pout) {
+  X64 qL[5], qR[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     if (recon == R_PLM) {
-      const double d01 = c[1][v] - c[0][v], d12 = c[2][v] - c[1][v], d23 = c[3][v] - c[2][v];
-      const double sL = DIR == 2 ? minmod_exact(d12, d01) : minmod_exact(d01, d12);
-      const double sR = DIR == 2 ? minmod_exact(d23, d12) : minmod_exact(d12, d23);
+      const X64 d01 = c[1][v] - c[0][v], d12 = c[2][v] - c[1][v], d23 = c[3][v] - c[2][v];
+      const X64 sL = DIR == 2 ? minmod_exact(d12, d01) : minmod_exact(d01, d12);
+      const X64 sR = DIR == 2 ? minmod_exact(d23, d12) : minmod_exact(d12, d23);
       qL[v] = recon_plus(c[1][v], sL);
       qR[v] = recon_minus(c[2][v], sR);
     } else {
@@ -216,11 +216,11 @@ __device__ __forceinline__ void face3(const double c[4][5], int rs, int recon, c
     }
   }
   if (DIR == 2 && recon == R_PCM_WB) {  // Update.h:27
-    qL[4] = qL[4] + half64(1.0 * qL[0] * G.g * G.dz);
-    qR[4] = qR[4] + half64(-1.0 * qR[0] * G.g * G.dz);
+    qL[4] = qL[4] + half_of(qL[0] * G.g * G.dz);
+    qR[4] = qR[4] + half_of(-qR[0] * G.g * G.dz);
   }
-  const Slots<double> L = slots3<DIR>(qL), R = slots3<DIR>(qR);
-  double f[5];
+  const Slots<X64> L = slots3<DIR>(qL), R = slots3<DIR>(qR);
+  X64 f[5];
   if (rs == 0)
     hll64<0>(L, R, K, f, pout);
   else
@@ -232,7 +232,7 @@ __device__ __forceinline__ void face3(const double c[4][5], int rs, int recon, c
 struct RingVel {
   Smem3 S;
   int k, hy, hx;
-  __device__ __forceinline__ double operator()(int dk, int dj, int di, int var) const {
+  __device__ __forceinline__ X64 operator()(int dk, int dj, int di, int var) const {
     return S.q(slot_of(k + dk - 1), var, hy + dj - 1, hx + di - 1);
   }
 };
@@ -244,44 +244,44 @@ struct RingVel {
 // serves both.  P is centred on the cell above the face (the s = 1 side of
 // the reference's loop).
 template <int DIR, class PA>
-__device__ __forceinline__ void viscous_face3d(const PA& P, double odx, double ody, double odz, double mu,
-                                               double g[4]) {
-  const double four_thirds = 4.0 / 3.0;
-  const double two_thirds = 2.0 / 3.0;
-  const double c4x = half64(half64(odx)), c4y = half64(half64(ody)), c4z = half64(half64(odz));
+__device__ __forceinline__ void viscous_face3d(const PA& P, X64 odx, X64 ody, X64 odz, X64 mu,
+                                               X64 g[4]) {
+  const X64 four_thirds = four_thirds_of<X64>();
+  const X64 two_thirds = two_thirds_of<X64>();
+  const X64 c4x = half_of(half_of(odx)), c4y = half_of(half_of(ody)), c4z = half_of(half_of(odz));
   const int U = 1, V = 2, W = 3;
   if (DIR == 0) {
-    const double qiu = half64(P(1, 1, 1, U) + P(1, 1, 0, U));
-    const double qiv = half64(P(1, 1, 1, V) + P(1, 1, 0, V));
-    const double qiw = half64(P(1, 1, 1, W) + P(1, 1, 0, W));
-    const double dudx = odx * (P(1, 1, 1, U) - P(1, 1, 0, U));
-    const double dvdx = odx * (P(1, 1, 1, V) - P(1, 1, 0, V));
-    const double dwdx = odx * (P(1, 1, 1, W) - P(1, 1, 0, W));
-    const double dudy = c4y * (P(1, 2, 1, U) - P(1, 0, 1, U) + P(1, 2, 0, U) - P(1, 0, 0, U));
-    const double dvdy = c4y * (P(1, 2, 1, V) - P(1, 0, 1, V) + P(1, 2, 0, V) - P(1, 0, 0, V));
-    const double dudz = c4z * (P(2, 1, 1, U) - P(0, 1, 1, U) + P(2, 1, 0, U) - P(0, 1, 0, U));
-    const double dwdz = c4z * (P(2, 1, 1, W) - P(0, 1, 1, W) + P(2, 1, 0, W) - P(0, 1, 0, W));
-    const double tau_xx = four_thirds * dudx - two_thirds * (dvdy + dwdz);
-    const double tau_xy = dvdx + dudy;
-    const double tau_xz = dwdx + dudz;
+    const X64 qiu = half_of(P(1, 1, 1, U) + P(1, 1, 0, U));
+    const X64 qiv = half_of(P(1, 1, 1, V) + P(1, 1, 0, V));
+    const X64 qiw = half_of(P(1, 1, 1, W) + P(1, 1, 0, W));
+    const X64 dudx = odx * (P(1, 1, 1, U) - P(1, 1, 0, U));
+    const X64 dvdx = odx * (P(1, 1, 1, V) - P(1, 1, 0, V));
+    const X64 dwdx = odx * (P(1, 1, 1, W) - P(1, 1, 0, W));
+    const X64 dudy = c4y * (P(1, 2, 1, U) - P(1, 0, 1, U) + P(1, 2, 0, U) - P(1, 0, 0, U));
+    const X64 dvdy = c4y * (P(1, 2, 1, V) - P(1, 0, 1, V) + P(1, 2, 0, V) - P(1, 0, 0, V));
+    const X64 dudz = c4z * (P(2, 1, 1, U) - P(0, 1, 1, U) + P(2, 1, 0, U) - P(0, 1, 0, U));
+    const X64 dwdz = c4z * (P(2, 1, 1, W) - P(0, 1, 1, W) + P(2, 1, 0, W) - P(0, 1, 0, W));
+    const X64 tau_xx = four_thirds * dudx - two_thirds * (dvdy + dwdz);
+    const X64 tau_xy = dvdx + dudy;
+    const X64 tau_xz = dwdx + dudz;
     g[0] = mu * tau_xx;
     g[1] = mu * tau_xy;
     g[2] = mu * tau_xz;
     g[3] = mu * (tau_xx * qiu + tau_xy * qiv + tau_xz * qiw);
   } else {
-    const double qiu = half64(P(1, 1, 1, U) + P(1, 0, 1, U));
-    const double qiv = half64(P(1, 1, 1, V) + P(1, 0, 1, V));
-    const double qiw = half64(P(1, 1, 1, W) + P(1, 0, 1, W));
-    const double dudy = ody * (P(1, 1, 1, U) - P(1, 0, 1, U));
-    const double dvdy = ody * (P(1, 1, 1, V) - P(1, 0, 1, V));
-    const double dwdy = ody * (P(1, 1, 1, W) - P(1, 0, 1, W));
-    const double dudx = c4x * (P(1, 1, 2, U) - P(1, 1, 0, U) + P(1, 0, 2, U) - P(1, 0, 0, U));
-    const double dvdx = c4x * (P(1, 1, 2, V) - P(1, 1, 0, V) + P(1, 0, 2, V) - P(1, 0, 0, V));
-    const double dwdz = c4z * (P(2, 1, 1, W) - P(0, 1, 1, W) + P(2, 0, 1, W) - P(0, 0, 1, W));
-    const double dvdz = c4z * (P(2, 1, 1, V) - P(0, 1, 1, V) + P(2, 0, 1, V) - P(0, 0, 1, V));
-    const double tau_yy = four_thirds * dvdy - two_thirds * (dudx + dwdz);
-    const double tau_xy = dvdx + dudy;
-    const double tau_yz = dvdz + dwdy;
+    const X64 qiu = half_of(P(1, 1, 1, U) + P(1, 0, 1, U));
+    const X64 qiv = half_of(P(1, 1, 1, V) + P(1, 0, 1, V));
+    const X64 qiw = half_of(P(1, 1, 1, W) + P(1, 0, 1, W));
+    const X64 dudy = ody * (P(1, 1, 1, U) - P(1, 0, 1, U));
+    const X64 dvdy = ody * (P(1, 1, 1, V) - P(1, 0, 1, V));
+    const X64 dwdy = ody * (P(1, 1, 1, W) - P(1, 0, 1, W));
+    const X64 dudx = c4x * (P(1, 1, 2, U) - P(1, 1, 0, U) + P(1, 0, 2, U) - P(1, 0, 0, U));
+    const X64 dvdx = c4x * (P(1, 1, 2, V) - P(1, 1, 0, V) + P(1, 0, 2, V) - P(1, 0, 0, V));
+    const X64 dwdz = c4z * (P(2, 1, 1, W) - P(0, 1, 1, W) + P(2, 0, 1, W) - P(0, 0, 1, W));
+    const X64 dvdz = c4z * (P(2, 1, 1, V) - P(0, 1, 1, V) + P(2, 0, 1, V) - P(0, 0, 1, V));
+    const X64 tau_yy = four_thirds * dvdy - two_thirds * (dudx + dwdz);
+    const X64 tau_xy = dvdx + dudy;
+    const X64 tau_yz = dvdz + dwdy;
     g[0] = mu * tau_xy;
     g[1] = mu * tau_yy;
     g[2] = mu * tau_yz;
@@ -293,27 +293,27 @@ __device__ __forceinline__ void viscous_face3d(const PA& P, double odx, double o
 // field mix-ups (some terms read the cell's own row, so this flux belongs to
 // the cell): accumulates into vz[1..4] like viscous3d<false>.
 template <class PA>
-__device__ __forceinline__ void viscous_iz3d(const PA& P, double odx, double odz, double mu, double vz[5]) {
-  const double four_thirds = 4.0 / 3.0;
-  const double two_thirds = 2.0 / 3.0;
-  const double c4x = half64(half64(odx)), c4z = half64(half64(odz));
+__device__ __forceinline__ void viscous_iz3d(const PA& P, X64 odx, X64 odz, X64 mu, X64 vz[5]) {
+  const X64 four_thirds = four_thirds_of<X64>();
+  const X64 two_thirds = two_thirds_of<X64>();
+  const X64 c4x = half_of(half_of(odx)), c4z = half_of(half_of(odz));
   const int U = 1, V = 2, W = 3;
 #pragma unroll
   for (int s = 1; s < 3; ++s) {
-    const double sm = (s == 1 ? -1.0 : 1.0) * mu;
-    const double qiu = half64(P(s, 1, 1, U) + P(s - 1, 1, 1, U));
-    const double qiv = half64(P(s, 1, 1, V) + P(s - 1, 1, 1, V));
-    const double qiw = half64(P(s, 1, 1, W) + P(s - 1, 1, 1, W));
-    const double dudz = odz * (P(s, 1, 1, U) - P(s - 1, 1, 1, U));
-    const double dvdz = odz * (P(s, 1, 1, V) - P(s - 1, 1, 1, V));
-    const double dwdz = odz * (P(s, 1, 1, W) - P(s - 1, 1, 1, W));
-    const double dudx = c4x * (P(s, 1, 2, U) - P(1, s, 0, U) + P(s - 1, 1, 2, U) - P(1, s - 1, 0, U));
-    const double dwdx = c4x * (P(s, 1, 2, V) - P(1, s, 0, W) + P(s - 1, 1, 2, V) - P(1, s - 1, 0, W));
-    const double dvdy = c4z * (P(s, 2, 1, W) - P(s, 0, 1, V) + P(s - 1, 2, 1, W) - P(s - 1, 0, 1, V));
-    const double dwdy = c4z * (P(s, 2, 1, V) - P(s, 0, 1, W) + P(s - 1, 2, 1, V) - P(s - 1, 0, 1, W));
-    const double tau_zz = four_thirds * dwdz - two_thirds * (dudx + dvdy);
-    const double tau_xz = dudz + dwdx;
-    const double tau_yz = dvdz + dwdy;
+    const X64 sm = s == 1 ? -mu : mu;
+    const X64 qiu = half_of(P(s, 1, 1, U) + P(s - 1, 1, 1, U));
+    const X64 qiv = half_of(P(s, 1, 1, V) + P(s - 1, 1, 1, V));
+    const X64 qiw = half_of(P(s, 1, 1, W) + P(s - 1, 1, 1, W));
+    const X64 dudz = odz * (P(s, 1, 1, U) - P(s - 1, 1, 1, U));
+    const X64 dvdz = odz * (P(s, 1, 1, V) - P(s - 1, 1, 1, V));
+    const X64 dwdz = odz * (P(s, 1, 1, W) - P(s - 1, 1, 1, W));
+    const X64 dudx = c4x * (P(s, 1, 2, U) - P(1, s, 0, U) + P(s - 1, 1, 2, U) - P(1, s - 1, 0, U));
+    const X64 dwdx = c4x * (P(s, 1, 2, V) - P(1, s, 0, W) + P(s - 1, 1, 2, V) - P(1, s - 1, 0, W));
+    const X64 dvdy = c4z * (P(s, 2, 1, W) - P(s, 0, 1, V) + P(s - 1, 2, 1, W) - P(s - 1, 0, 1, V));
+    const X64 dwdy = c4z * (P(s, 2, 1, V) - P(s, 0, 1, W) + P(s - 1, 2, 1, V) - P(s - 1, 0, 1, W));
+    const X64 tau_zz = four_thirds * dwdz - two_thirds * (dudx + dvdy);
+    const X64 tau_xz = dudz + dwdx;
+    const X64 tau_yz = dvdz + dwdy;
     vz[1] += sm * tau_xz;
     vz[2] += sm * tau_yz;
     vz[3] += sm * tau_zz;
@@ -352,7 +352,7 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
     }
     return;
   }
-  const double dt = ctrl->dt_cur;
+  const X64 dt = ctrl->dt_cur;
   const Consts64 K{G.gamma, G.gm1, G.inv_gm1};
   const int recon = G.recon;
   const bool need_pout = G.wb_flux_z || G.bc_c == DBC_C91;
@@ -361,9 +361,9 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
   // prologue: layers k0-2 .. k0+1, then the z face k0-1/2 of the own column
   for (int kg = k0 - 2; kg <= k0 + 1; ++kg) load_layer(G, uin, qin, x0, y0, kg, S, tid);
   __syncthreads();
-  double fzL[5], poutL = 0.0;
+  X64 fzL[5], poutL = 0.0;
   if (own) {
-    double c[4][5];
+    X64 c[4][5];
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
@@ -378,7 +378,7 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
     load_layer(G, uin, qin, x0, y0, k + 2, S, tid);
     const int sk = slot_of(k);
     for (int it = tid; it < kNFA_PAD + kNFB; it += kThreads) {
-      double c[4][5], f[5];
+      X64 c[4][5], f[5];
       if (it < kNFA_PAD) {
         if (it >= kNFA) continue;
         const int fy = it / (kTX + 1), fx = it - fy * (kTX + 1);
@@ -388,7 +388,7 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
           for (int v = 0; v < 5; ++v) c[m][v] = S.q(sk, v, fy + 2, fx + m);
         face3<0, CORR>(c, rs, recon, G, K, f, nullptr);
 #pragma unroll
-        for (int v = 0; v < 5; ++v) S.fa(v, fy, fx) = f[v];
+        for (int v = 0; v < 5; ++v) S.fa(v, fy, fx) = f[v].v;
       } else {
         const int j = it - kNFA_PAD;
         const int fy = j / kTX, fx = j - fy * kTX;
@@ -398,17 +398,17 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
           for (int v = 0; v < 5; ++v) c[m][v] = S.q(sk, v, fy + m, fx + 2);
         face3<1, CORR>(c, rs, recon, G, K, f, nullptr);
 #pragma unroll
-        for (int v = 0; v < 5; ++v) S.fb(v, fy, fx) = f[v];
+        for (int v = 0; v < 5; ++v) S.fb(v, fy, fx) = f[v].v;
       }
     }
     __syncthreads();
 
     // ---- 2. z face k+1/2 and the update of the own cell ----
-    double un[5], fzR[5], poutR = 0.0;
+    X64 un[5], fzR[5], poutR = 0.0;
     const long long o = k * zstride + col;
     if (own) {
       {
-        double c[4][5];
+        X64 c[4][5];
 #pragma unroll
         for (int m = 0; m < 4; ++m)
 #pragma unroll
@@ -420,18 +420,18 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
       // IX, IY: un += (F(-1/2) - F(+1/2)) * dt / d
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        un[v] = un[v] + div_cell<P2>((S.fa(v, cy, cx) - S.fa(v, cy, cx + 1)) * dt, G.dx, G.inv_dx);
+        un[v] = un[v] + div_cell<P2>((X64(S.fa(v, cy, cx)) - S.fa(v, cy, cx + 1)) * dt, G.dx, G.inv_dx);
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        un[v] = un[v] + div_cell<P2>((S.fb(v, cy, cx) - S.fb(v, cy + 1, cx)) * dt, G.dy, G.inv_dy);
+        un[v] = un[v] + div_cell<P2>((X64(S.fb(v, cy, cx)) - S.fb(v, cy + 1, cx)) * dt, G.dy, G.inv_dy);
       // IZ with the z-boundary overrides of Update.h:131-143
-      double fL[5], fR[5];
+      X64 fL[5], fR[5];
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
         fL[v] = fzL[v];
         fR[v] = fzR[v];
       }
-      const double rho_c = S.q(sk, 0, cy + 2, cx + 2);
+      const X64 rho_c = S.q(sk, 0, cy + 2, cx + 2);
       if (G.wb_flux_z && (k == 0 || k == G.nc - 1)) {
         if (k == 0) {
           fL[0] = 0.0; fL[1] = 0.0; fL[2] = 0.0; fL[4] = 0.0;
@@ -453,44 +453,44 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
       for (int v = 0; v < 5; ++v) un[v] = un[v] + div_cell<P2>((fL[v] - fR[v]) * dt, G.dz, G.inv_dz);
       if (G.gravity) {
         un[3] = un[3] + dt * rho_c * G.g;
-        un[4] = un[4] + half64(dt) * (fL[0] + fR[0]) * G.g;
+        un[4] = un[4] + half_of(dt) * (fL[0] + fR[0]) * G.g;
       }
       un[0] = fmax_bits(1.0e-6, un[0]);
 
       if (G.tc) {  // ThermalConduction.h:38-96
-        double kC, kF, kB;
+        X64 kC, kF, kB;
         if (G.kappa_z) {
           kC = G.kappa_z[3 * k];
           kF = G.kappa_z[3 * k + 1];
           kB = G.kappa_z[3 * k + 2];
         } else {
-          kC = kF = kB = half64(G.kappa + G.kappa);
+          kC = kF = kB = half_of(X64(G.kappa) + G.kappa);
         }
         const int hy = cy + 2, hx = cx + 2;
-        const double TC = S.temp(sk, hy, hx);
-        const double FL = div_cell<P2>(kC * (TC - S.temp(sk, hy, hx - 1)), G.dx, G.inv_dx);
-        const double FR = div_cell<P2>(kC * (S.temp(sk, hy, hx + 1) - TC), G.dx, G.inv_dx);
-        const double FU = div_cell<P2>(kC * (TC - S.temp(sk, hy - 1, hx)), G.dy, G.inv_dy);
-        const double FD = div_cell<P2>(kC * (S.temp(sk, hy + 1, hx) - TC), G.dy, G.inv_dy);
-        double FF = div_cell<P2>(kF * (TC - S.temp(slot_of(k - 1), hy, hx)), G.dz, G.inv_dz);
-        double FB = div_cell<P2>(kB * (S.temp(slot_of(k + 1), hy, hx) - TC), G.dz, G.inv_dz);
+        const X64 TC = S.temp(sk, hy, hx);
+        const X64 FL = div_cell<P2>(kC * (TC - S.temp(sk, hy, hx - 1)), G.dx, G.inv_dx);
+        const X64 FR = div_cell<P2>(kC * (X64(S.temp(sk, hy, hx + 1)) - TC), G.dx, G.inv_dx);
+        const X64 FU = div_cell<P2>(kC * (TC - S.temp(sk, hy - 1, hx)), G.dy, G.inv_dy);
+        const X64 FD = div_cell<P2>(kC * (X64(S.temp(sk, hy + 1, hx)) - TC), G.dy, G.inv_dy);
+        X64 FF = div_cell<P2>(kF * (TC - S.temp(slot_of(k - 1), hy, hx)), G.dz, G.inv_dz);
+        X64 FB = div_cell<P2>(kB * (X64(S.temp(slot_of(k + 1), hy, hx)) - TC), G.dz, G.inv_dz);
         if (k == 0 && G.bctc_zmin != 0) {
           if (G.bctc_zmin == 1) FF = div_cell<P2>(kF * 2.0 * (TC - G.bctc_zmin_value), G.dz, G.inv_dz);
           else FF = kF * G.bctc_zmin_value;
         }
         if (k == G.nc - 1 && G.bctc_zmax != 0) {
-          if (G.bctc_zmax == 1) FB = div_cell<P2>(kB * 2.0 * (G.bctc_zmax_value - TC), G.dz, G.inv_dz);
+          if (G.bctc_zmax == 1) FB = div_cell<P2>(kB * 2.0 * (X64(G.bctc_zmax_value) - TC), G.dz, G.inv_dz);
           else FB = kB * G.bctc_zmax_value;
         }
-        const double dtdx = div_cell<P2>(dt, G.dx, G.inv_dx);
-        const double dtdy = div_cell<P2>(dt, G.dy, G.inv_dy);
-        const double dtdz = div_cell<P2>(dt, G.dz, G.inv_dz);
+        const X64 dtdx = div_cell<P2>(dt, G.dx, G.inv_dx);
+        const X64 dtdy = div_cell<P2>(dt, G.dy, G.inv_dy);
+        const X64 dtdz = div_cell<P2>(dt, G.dz, G.inv_dz);
         un[4] = un[4] + (dtdx * (FR - FL) + dtdy * (FD - FU) + dtdz * (FB - FF));
       }
       if (G.visc && !vsh) {  // Viscosity.h:145-151
         const RingVel P{S, k, cy + 2, cx + 2};
-        double vf[3][5];
-        viscous3d<CORR, double>(P, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, vf);
+        X64 vf[3][5];
+        viscous3d<CORR, X64>(P, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, vf);
         if (CORR) {  // the flux differences divided by the cell sizes
 #pragma unroll
           for (int v = 1; v < 5; ++v)
@@ -505,32 +505,32 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
     if (vsh) {  // viscosity with the face-only branches solved once per face
       __syncthreads();  // every cell is done with the hydro fluxes in FA / FB
       for (int it = tid; it < kNFA_PAD + kNFB; it += kThreads) {
-        double g[4];
+        X64 g[4];
         if (it < kNFA_PAD) {
           if (it >= kNFA) continue;
           const int fy = it / (kTX + 1), fx = it - fy * (kTX + 1);
           viscous_face3d<0>(RingVel{S, k, fy + 2, fx + 2}, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, g);
 #pragma unroll
-          for (int v = 0; v < 4; ++v) S.fa(v, fy, fx) = g[v];
+          for (int v = 0; v < 4; ++v) S.fa(v, fy, fx) = g[v].v;
         } else {
           const int j = it - kNFA_PAD;
           const int fy = j / kTX, fx = j - fy * kTX;
           viscous_face3d<1>(RingVel{S, k, fy + 2, fx + 2}, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, g);
 #pragma unroll
-          for (int v = 0; v < 4; ++v) S.fb(v, fy, fx) = g[v];
+          for (int v = 0; v < 4; ++v) S.fb(v, fy, fx) = g[v].v;
         }
       }
       __syncthreads();
       if (own) {  // vf[d][v+1] = (0 + (-g_lower)) + g_upper, then IZ per cell (Viscosity.h:145-151)
-        double vf[3][5];
+        X64 vf[3][5];
 #pragma unroll
         for (int d = 0; d < 3; ++d)
 #pragma unroll
           for (int v = 0; v < 5; ++v) vf[d][v] = 0.0;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          vf[0][v + 1] = plus_zero(-S.fa(v, cy, cx)) + S.fa(v, cy, cx + 1);
-          vf[1][v + 1] = plus_zero(-S.fb(v, cy, cx)) + S.fb(v, cy + 1, cx);
+          vf[0][v + 1] = plus_zero(-X64(S.fa(v, cy, cx))) + S.fa(v, cy, cx + 1);
+          vf[1][v + 1] = plus_zero(-X64(S.fb(v, cy, cx))) + S.fb(v, cy + 1, cx);
         }
         viscous_iz3d(RingVel{S, k, cy + 2, cx + 2}, G.inv_dx, G.inv_dz, G.mu, vf[2]);
 #pragma unroll
@@ -540,13 +540,13 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
     if (own) {
       if (kind == STAGE_RK_2) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) un[v] = half64(u0.f[v][o] + un[v]);
+        for (int v = 0; v < 5; ++v) un[v] = half_of(X64(u0.f[v][o]) + un[v]);
       }
 #pragma unroll
-      for (int v = 0; v < 5; ++v) uout.f[v][o] = un[v];
+      for (int v = 0; v < 5; ++v) uout.f[v][o] = un[v].v;
       if (kind != STAGE_RK_1) {
-        double q[5];
-        const double inv = inv_dt_hyp64<PLANE_XY, true, P2>(un, G, q);
+        X64 q[5];
+        const double inv = inv_dt_hyp64<PLANE_XY, true, P2>(un, G, q).v;
         const unsigned long long b = (unsigned long long)__double_as_longlong(inv);
         red = b > red ? b : red;
         if (above_bits(inv, 1.0e300)) atomicOr(&ctrl->err, 1);
@@ -554,11 +554,11 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
           const long long h = ((long long)k * G.nb + y) * G.na + x;
 #pragma unroll
           for (int v = 0; v < 5; ++v)
-            if (hout.f[v]) hout.f[v][h] = q[v];
+            if (hout.f[v]) hout.f[v][h] = q[v].v;
         }
         if (qout) {
 #pragma unroll
-          for (int v = 0; v < 5; ++v) qout->f[v][o] = q[v];
+          for (int v = 0; v < 5; ++v) qout->f[v][o] = q[v].v;
         }
       }
 #pragma unroll
@@ -609,11 +609,16 @@ __device__ __forceinline__ unsigned long long march3d(const Grid& G, const Field
 // at once; a CTA marches each column block of its range over its layers.
 template <int RS, int KIND, bool CORR>
 __global__ void __launch_bounds__(kThreads, FV_3D64_MIN_CTAS)
-stage3d_fp64(const Grid G, const Fields uin, const Fields u0, const Fields uout, StepCtrl* __restrict__ ctrl,
+stage3d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u0, const Fields uout, StepCtrl* __restrict__ ctrl,
              long long units, const Fields hout, const Fields qin, const Fields qout) {
   extern __shared__ double smem_raw[];
   __shared__ unsigned long long s_red[kThreads / 32];
+  __shared__ Grid s_grid;
+  const Grid& G = s_grid;
+  param_to_shared(grid, s_grid);
+  opaque64_init();
   pdl_wait();
+  __syncthreads();
   const long long ub = units * blockIdx.x / gridDim.x, ue = units * (blockIdx.x + 1) / gridDim.x;
   const int active = ctrl->active, parity = ctrl->parity;
   // the primitive copy of uin, when the last stage that wrote uin left one
@@ -700,6 +705,7 @@ batch_stage3d64(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsi
   __shared__ BatchInst s_inst;
   __shared__ int s_tile;
   const Fields none{};
+  opaque64_init();  // the first use follows the __syncthreads below
   pdl_wait();
   for (;;) {
     __syncthreads();  // the previous item is finished with s_tile, s_inst and smem

@@ -91,7 +91,7 @@ struct TileSmem {
 // depend on the side.  Accumulates into vz[1..4].
 template <class T, class PA>
 __device__ __forceinline__ void viscous_iz_xy(const PA& P, T odx, T odz, T mu, T vz[5]) {
-  const T two_thirds = T(2.0 / 3.0);
+  const T two_thirds = two_thirds_of<T>();
   const T c4x = half_of(half_of(odx)), c4z = half_of(half_of(odz));
   const int U = 1, V = 2, W = 3;
   const T cu = P(1, 1, U), cv = P(1, 1, V), cw = P(1, 1, W);
@@ -99,16 +99,16 @@ __device__ __forceinline__ void viscous_iz_xy(const PA& P, T odx, T odz, T mu, T
   const T dwdy = c4z * (P(2, 1, V) - P(0, 1, W) + P(2, 1, V) - P(0, 1, W));
 #pragma unroll
   for (int s = 1; s < 3; ++s) {
-    const T sign = s == 1 ? T(-1) : T(1);
+    const T sm = s == 1 ? -mu : mu;
     const T dudx = c4x * (P(1, 2, U) - P(s, 0, U) + P(1, 2, U) - P(s - 1, 0, U));
     const T dwdx = c4x * (P(1, 2, V) - P(s, 0, W) + P(1, 2, V) - P(s - 1, 0, W));
     const T tau_zz = -(two_thirds * (dudx + dvdy));
     const T tau_xz = dwdx;
     const T tau_yz = dwdy;
-    vz[1] += sign * mu * tau_xz;
-    vz[2] += sign * mu * tau_yz;
-    vz[3] += sign * mu * tau_zz;
-    vz[4] += sign * mu * (tau_xz * cu + tau_yz * cv + tau_zz * cw);
+    vz[1] += sm * tau_xz;
+    vz[2] += sm * tau_yz;
+    vz[3] += sm * tau_zz;
+    vz[4] += sm * (tau_xz * cu + tau_yz * cv + tau_zz * cw);
   }
 }
 
@@ -117,13 +117,13 @@ __device__ __forceinline__ void viscous_iz_xy(const PA& P, T odx, T odz, T mu, T
 // flux belongs to the cell, not to the face.  Accumulates into vz[1..4].
 template <class T, class PA>
 __device__ __forceinline__ void viscous_iz_xz(const PA& P, T odx, T odz, T mu, T vz[5]) {
-  const T four_thirds = T(4.0 / 3.0);
-  const T two_thirds = T(2.0 / 3.0);
+  const T four_thirds = four_thirds_of<T>();
+  const T two_thirds = two_thirds_of<T>();
   const T c4x = half_of(half_of(odx)), c4z = half_of(half_of(odz));
   const int U = 1, V = 2, W = 3;
 #pragma unroll
   for (int s = 1; s < 3; ++s) {
-    const T sign = s == 1 ? T(-1) : T(1);
+    const T sm = s == 1 ? -mu : mu;
     const T qiu = half_of(P(s, 1, U) + P(s - 1, 1, U));
     const T qiv = half_of(P(s, 1, V) + P(s - 1, 1, V));
     const T qiw = half_of(P(s, 1, W) + P(s - 1, 1, W));
@@ -137,10 +137,10 @@ __device__ __forceinline__ void viscous_iz_xz(const PA& P, T odx, T odz, T mu, T
     const T tau_zz = four_thirds * dwdz - two_thirds * (dudx + dvdy);
     const T tau_xz = dudz + dwdx;
     const T tau_yz = dvdz + dwdy;
-    vz[1] += sign * mu * tau_xz;
-    vz[2] += sign * mu * tau_yz;
-    vz[3] += sign * mu * tau_zz;
-    vz[4] += sign * mu * (tau_xz * qiu + tau_yz * qiv + tau_zz * qiw);
+    vz[1] += sm * tau_xz;
+    vz[2] += sm * tau_yz;
+    vz[3] += sm * tau_zz;
+    vz[4] += sm * (tau_xz * qiu + tau_yz * qiv + tau_zz * qiw);
   }
 }
 
@@ -157,8 +157,8 @@ __device__ __forceinline__ void viscous_iz_xz(const PA& P, T odx, T odz, T mu, T
 // computed once on the host.
 template <int PLANE, class T, class PA>
 __device__ __forceinline__ void viscous_plane(const PA& P, T odx, T ody, T odz, T mu, T vf[3][5]) {
-  const T four_thirds = T(4.0 / 3.0);
-  const T two_thirds = T(2.0 / 3.0);
+  const T four_thirds = four_thirds_of<T>();
+  const T two_thirds = two_thirds_of<T>();
   const T c4x = half_of(half_of(odx)), c4y = half_of(half_of(ody)), c4z = half_of(half_of(odz));
   const int U = 1, V = 2, W = 3;
 #pragma unroll
@@ -168,7 +168,7 @@ __device__ __forceinline__ void viscous_plane(const PA& P, T odx, T ody, T odz, 
   if (PLANE == PLANE_XY) {
 #pragma unroll
     for (int s = 1; s < 3; ++s) {  // IX (Viscosity.h:163-186), z-derivatives vanish
-      const T sign = s == 1 ? T(-1) : T(1);
+      const T sm = s == 1 ? -mu : mu;
       const T qiu = half_of(P(1, s, U) + P(1, s - 1, U));
       const T qiv = half_of(P(1, s, V) + P(1, s - 1, V));
       const T qiw = half_of(P(1, s, W) + P(1, s - 1, W));
@@ -180,14 +180,14 @@ __device__ __forceinline__ void viscous_plane(const PA& P, T odx, T ody, T odz, 
       const T tau_xx = four_thirds * dudx - two_thirds * dvdy;
       const T tau_xy = dvdx + dudy;
       const T tau_xz = dwdx;
-      vf[0][1] += sign * mu * tau_xx;
-      vf[0][2] += sign * mu * tau_xy;
-      vf[0][3] += sign * mu * tau_xz;
-      vf[0][4] += sign * mu * (tau_xx * qiu + tau_xy * qiv + tau_xz * qiw);
+      vf[0][1] += sm * tau_xx;
+      vf[0][2] += sm * tau_xy;
+      vf[0][3] += sm * tau_xz;
+      vf[0][4] += sm * (tau_xx * qiu + tau_xy * qiv + tau_xz * qiw);
     }
 #pragma unroll
     for (int s = 1; s < 3; ++s) {  // IY (Viscosity.h:188-213), z-derivatives vanish
-      const T sign = s == 1 ? T(-1) : T(1);
+      const T sm = s == 1 ? -mu : mu;
       const T qiu = half_of(P(s, 1, U) + P(s - 1, 1, U));
       const T qiv = half_of(P(s, 1, V) + P(s - 1, 1, V));
       const T qiw = half_of(P(s, 1, W) + P(s - 1, 1, W));
@@ -199,16 +199,16 @@ __device__ __forceinline__ void viscous_plane(const PA& P, T odx, T ody, T odz, 
       const T tau_yy = four_thirds * dvdy - two_thirds * dudx;
       const T tau_xy = dvdx + dudy;
       const T tau_yz = dwdy;
-      vf[1][1] += sign * mu * tau_xy;
-      vf[1][2] += sign * mu * tau_yy;
-      vf[1][3] += sign * mu * tau_yz;
-      vf[1][4] += sign * mu * (tau_xy * qiu + tau_yy * qiv + tau_yz * qiw);
+      vf[1][1] += sm * tau_xy;
+      vf[1][2] += sm * tau_yy;
+      vf[1][3] += sm * tau_yz;
+      vf[1][4] += sm * (tau_xy * qiu + tau_yy * qiv + tau_yz * qiw);
     }
     viscous_iz_xy(P, odx, odz, mu, vf[2]);
   } else {
 #pragma unroll
     for (int s = 1; s < 3; ++s) {  // IX, y-derivatives vanish
-      const T sign = s == 1 ? T(-1) : T(1);
+      const T sm = s == 1 ? -mu : mu;
       const T qiu = half_of(P(1, s, U) + P(1, s - 1, U));
       const T qiv = half_of(P(1, s, V) + P(1, s - 1, V));
       const T qiw = half_of(P(1, s, W) + P(1, s - 1, W));
@@ -220,10 +220,10 @@ __device__ __forceinline__ void viscous_plane(const PA& P, T odx, T ody, T odz, 
       const T tau_xx = four_thirds * dudx - two_thirds * dwdz;
       const T tau_xy = dvdx;
       const T tau_xz = dwdx + dudz;
-      vf[0][1] += sign * mu * tau_xx;
-      vf[0][2] += sign * mu * tau_xy;
-      vf[0][3] += sign * mu * tau_xz;
-      vf[0][4] += sign * mu * (tau_xx * qiu + tau_xy * qiv + tau_xz * qiw);
+      vf[0][1] += sm * tau_xx;
+      vf[0][2] += sm * tau_xy;
+      vf[0][3] += sm * tau_xz;
+      vf[0][4] += sm * (tau_xx * qiu + tau_xy * qiv + tau_xz * qiw);
     }
     // IY on the one-cell axis: every term is side-independent and cancels.
     viscous_iz_xz(P, odx, odz, mu, vf[2]);
@@ -231,11 +231,11 @@ __device__ __forceinline__ void viscous_plane(const PA& P, T odx, T ody, T odz, 
 }
 
 // Plane accessor for viscous_plane over a TileSmem primitive tile.
-template <int PLANE, class SM>
+template <int PLANE, class SM, class T>
 struct PlaneVel {
   SM s;
   int hy, hx;
-  __device__ __forceinline__ auto operator()(int r, int c, int var) const {
+  __device__ __forceinline__ T operator()(int r, int c, int var) const {
     return s.q(phys_slot<PLANE>(var), hy + r - 1, hx + c - 1);
   }
 };
@@ -250,8 +250,8 @@ struct PlaneVel {
 // the face (the s = 1 side of Viscosity.h's loop).
 template <int PLANE, int DIR, class T, class PA>
 __device__ __forceinline__ void viscous_face(const PA& P, T odx, T ody, T odz, T mu, T g[4]) {
-  const T four_thirds = T(4.0 / 3.0);
-  const T two_thirds = T(2.0 / 3.0);
+  const T four_thirds = four_thirds_of<T>();
+  const T two_thirds = two_thirds_of<T>();
   const int U = 1, V = 2, W = 3;
   if (DIR == 0) {
     const T qiu = half_of(P(1, 1, U) + P(1, 0, U));
@@ -301,10 +301,13 @@ __device__ __forceinline__ void viscous_face(const PA& P, T odx, T ody, T odz, T
 }
 
 // 0.0 + x without the FP64 pipe: x itself, except that -0 becomes +0.
-__device__ __forceinline__ double plus_zero(double x) {
-  const long long b = __double_as_longlong(x);
-  return b == (long long)0x8000000000000000ull ? 0.0 : x;
+__device__ __forceinline__ X64 plus_zero(X64 x) {
+  const long long b = __double_as_longlong(x.v);
+  return b == (long long)0x8000000000000000ull ? X64(0.0) : x;
 }
+// The value a shared array holds (its element type) of either arithmetic type.
+__device__ __forceinline__ double stored(X64 x) { return x.v; }
+__device__ __forceinline__ float stored(float x) { return x; }
 __device__ __forceinline__ float plus_zero(float x) { return 0.0f + x; }
 
 // viscous_plane with the face-only branches taken from shared face fluxes:
@@ -345,18 +348,18 @@ __device__ __forceinline__ void visc_faces(const PV& V, T odx, T ody, T odz, T m
     if (it < nfa_pad) {
       if (it >= nfa) continue;
       const int fy = it / (TX + 1), fx = it - fy * (TX + 1);
-      const PlaneVel<PLANE, PV> P{V, fy + 2, fx + 2};  // the cell right of a face
-      viscous_face<PLANE, 0>(P, odx, ody, odz, mu, g);
+      const PlaneVel<PLANE, PV, T> P{V, fy + 2, fx + 2};  // the cell right of a face
+      viscous_face<PLANE, 0, T>(P, odx, ody, odz, mu, g);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) V.va(k, fy, fx) = g[k];
+      for (int k = 0; k < 4; ++k) V.va(k, fy, fx) = stored(g[k]);
     } else {
       const int j = it - nfa_pad;
       const int jy = j / TX, fx = j - jy * TX;
       const int fy = fb0 + jy;
-      const PlaneVel<PLANE, PV> P{V, fy + 2, fx + 2};  // the cell above b face fy
-      viscous_face<PLANE, 1>(P, odx, ody, odz, mu, g);
+      const PlaneVel<PLANE, PV, T> P{V, fy + 2, fx + 2};  // the cell above b face fy
+      viscous_face<PLANE, 1, T>(P, odx, ody, odz, mu, g);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) V.vb(k, fy, fx) = g[k];
+      for (int k = 0; k < 4; ++k) V.vb(k, fy, fx) = stored(g[k]);
     }
   }
 }
@@ -364,7 +367,7 @@ __device__ __forceinline__ void visc_faces(const PV& V, T odx, T ody, T odz, T m
 // The shared-face viscous fluxes of cell (cy, cx) of a block.
 template <int PLANE, class T, class PV>
 __device__ __forceinline__ void visc_cell_shared(const PV& V, int cy, int cx, T odx, T odz, T mu, T vf[3][5]) {
-  const PlaneVel<PLANE, PV> P{V, cy + 2, cx + 2};
+  const PlaneVel<PLANE, PV, T> P{V, cy + 2, cx + 2};
   T gl[2][4], gr[2][4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -373,7 +376,7 @@ __device__ __forceinline__ void visc_cell_shared(const PV& V, int cy, int cx, T 
     gl[1][k] = PLANE == PLANE_XY ? V.vb(k, cy, cx) : T(0);
     gr[1][k] = PLANE == PLANE_XY ? V.vb(k, cy + 1, cx) : T(0);
   }
-  viscous_plane_shared<PLANE>(P, gl, gr, odx, odz, mu, vf);
+  viscous_plane_shared<PLANE, T>(P, gl, gr, odx, odz, mu, vf);
 }
 
 // Slots of a sweep (swap_component, States.h:104-111) from storage order
@@ -416,10 +419,10 @@ __device__ __forceinline__ void from_slots(const T f[5], T out[5]) {
 // c[k][v] holds variable v of the four cells around the face (left-left,
 // left, right, right-right).
 template <int PLANE, bool WACT, int DIR>
-__device__ __forceinline__ void face_flux64(const double c[4][5], int rs, bool plm, bool wb_z, const Grid& G,
-                                            const Consts64& K, double out[5]) {
+__device__ __forceinline__ void face_flux64(const X64 c[4][5], int rs, bool plm, bool wb_z, const Grid& G,
+                                            const Consts64& K, X64 out[5]) {
   constexpr int ZS = WACT ? 0 : (PLANE == PLANE_XY ? 2 : 1);
-  double qL[5], qR[5];
+  X64 qL[5], qR[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     if (v == 3 && !WACT) {
@@ -428,7 +431,7 @@ __device__ __forceinline__ void face_flux64(const double c[4][5], int rs, bool p
       continue;
     }
     if (plm) {
-      const double d01 = c[1][v] - c[0][v], d12 = c[2][v] - c[1][v], d23 = c[3][v] - c[2][v];
+      const X64 d01 = c[1][v] - c[0][v], d12 = c[2][v] - c[1][v], d23 = c[3][v] - c[2][v];
       qL[v] = recon_plus(c[1][v], minmod_exact(d01, d12));
       qR[v] = recon_minus(c[2][v], minmod_exact(d12, d23));
     } else {
@@ -437,11 +440,11 @@ __device__ __forceinline__ void face_flux64(const double c[4][5], int rs, bool p
     }
   }
   if (DIR == 1 && wb_z) {  // PCM_WB hydrostatic pressure in z (Update.h:27)
-    qL[4] = qL[4] + half64(1.0 * qL[0] * G.g * G.dz);
-    qR[4] = qR[4] + half64(-1.0 * qR[0] * G.g * G.dz);
+    qL[4] = qL[4] + half_of(qL[0] * G.g * G.dz);
+    qR[4] = qR[4] + half_of(-qR[0] * G.g * G.dz);
   }
-  const Slots<double> L = to_slots<PLANE, DIR>(qL), R = to_slots<PLANE, DIR>(qR);
-  double f[5];
+  const Slots<X64> L = to_slots<PLANE, DIR>(qL), R = to_slots<PLANE, DIR>(qR);
+  X64 f[5];
   if (rs == 0)
     hll64<ZS>(L, R, K, f);
   else
@@ -497,7 +500,7 @@ __device__ __forceinline__ void load_prims64(const Grid& G, const Fields& uin, c
     const int sa = bc_source(x0 + hx - 2, G.na, G.bc_a, fa);
     const int sb = bc_source(y0 + hy - 2, G.nb, G.bc_b, fb);
     const long long o = (long long)sb * G.pitch + sa;
-    double u[5], q[5], y = 0.0;
+    X64 u[5], q[5], y = 0.0;
     u[0] = uin.f[0][o];
     u[1] = uin.f[1][o];
     u[2] = uin.f[2][o];
@@ -506,7 +509,7 @@ __device__ __forceinline__ void load_prims64(const Grid& G, const Fields& uin, c
     if (prims) {
 #pragma unroll
       for (int v = 0; v < 5; ++v) q[v] = u[v];
-      if (G.tc) y = 1.0 / q[0];
+      if (G.tc) y = rcp64(q[0]);
     } else {
       cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
     }
@@ -514,8 +517,8 @@ __device__ __forceinline__ void load_prims64(const Grid& G, const Fields& uin, c
     if (fb) q[2] = -q[2];
 #pragma unroll
     for (int v = 0; v < 5; ++v)
-      if (WACT || v != 3) V.q(v, hy, hx) = q[v];
-    if (G.tc) V.temp(hy, hx) = div_by_rcp(q[4], q[0], y);
+      if (WACT || v != 3) V.q(v, hy, hx) = q[v].v;
+    if (G.tc) V.temp(hy, hx) = div_by_rcp(q[4], q[0], y).v;
   }
 }
 
@@ -533,11 +536,11 @@ __device__ __forceinline__ void convert_rows64(const Grid& G, const PV& V, int h
     const int r = idx / HX, hx = idx - r * HX;
     const int hy = h0 + r;
     if (prims) {  // only the temperature
-      const double r = V.q(0, hy, hx), p = V.q(4, hy, hx);
-      V.temp(hy, hx) = div_by_rcp(p, r, 1.0 / r);
+      const X64 r = V.q(0, hy, hx), p = V.q(4, hy, hx);
+      V.temp(hy, hx) = div_by_rcp(p, r, rcp64(r)).v;
       continue;
     }
-    double u[5], q[5], y;
+    X64 u[5], q[5], y;
     u[0] = V.q(0, hy, hx);
     u[1] = V.q(1, hy, hx);
     u[2] = V.q(2, hy, hx);
@@ -546,8 +549,8 @@ __device__ __forceinline__ void convert_rows64(const Grid& G, const PV& V, int h
     cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
 #pragma unroll
     for (int v = 0; v < 5; ++v)
-      if (WACT || v != 3) V.q(v, hy, hx) = q[v];
-    if (G.tc) V.temp(hy, hx) = div_by_rcp(q[4], q[0], y);
+      if (WACT || v != 3) V.q(v, hy, hx) = q[v].v;
+    if (G.tc) V.temp(hy, hx) = div_by_rcp(q[4], q[0], y).v;
   }
 }
 
@@ -593,7 +596,7 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
   const int nfa_pad = (nfa + 31) & ~31;  // keeps each warp on one face kind
   const int n = nfa_pad + TX * (nr + 1 - fb0);
   for (int it = tid; it < n; it += kTileThreads) {
-    double c[4][5], f[5];
+    X64 c[4][5], f[5];
     if (it < nfa_pad) {
       if (it >= nfa) continue;
       const int fy = it / (TX + 1), fx = it - fy * (TX + 1);
@@ -604,7 +607,7 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
       face_flux64<PLANE, WACT, 0>(c, rs, plm, wb_z, G, K, f);
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        if (WACT || v != 3) V.fa(v, fy, fx) = f[v];
+        if (WACT || v != 3) V.fa(v, fy, fx) = f[v].v;
     } else {
       const int j = it - nfa_pad;
       const int jy = j / TX, fx = j - jy * TX;
@@ -616,10 +619,10 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
       face_flux64<PLANE, WACT, 1>(c, rs, plm, wb_z, G, K, f);
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        if (WACT || v != 3) V.fb(v, fy, fx) = f[v];
+        if (WACT || v != 3) V.fb(v, fy, fx) = f[v].v;
     }
   }
-  if (VSH && WACT && G.visc) visc_faces<PLANE, TL>(V, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, nr, fb0, tid);
+  if (VSH && WACT && G.visc) visc_faces<PLANE, TL, X64>(V, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, nr, fb0, tid);
 }
 
 // Phase 3-5: the cells of rows 0..nr-1 of the block -- conservative update,
@@ -629,12 +632,13 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
 // also written there, in the state's own layout, for the next step's load.
 template <int PLANE, bool WACT, class TL, bool P2, bool VSH, class PV>
 __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Fields& uin, const Fields& u0,
-                                         const Fields& uout, StepCtrl* ctrl, int kind, double dt, int x0, int y0,
+                                         const Fields& uout, StepCtrl* ctrl, int kind, double dt_step, int x0, int y0,
                                          int nr, int tid, const Fields* hout, unsigned long long& red,
                                          const Fields* qout = nullptr) {
   constexpr int TX = TL::TX;
-  const double db = PLANE == PLANE_XY ? G.dy : G.dz;
-  const double inv_db = PLANE == PLANE_XY ? G.inv_dy : G.inv_dz;
+  const X64 dt = dt_step;
+  const X64 db = PLANE == PLANE_XY ? G.dy : G.dz;
+  const X64 inv_db = PLANE == PLANE_XY ? G.inv_dy : G.inv_dz;
   const int ncell = TX * nr;
 #pragma unroll 1
   for (int cidx = tid; cidx < ncell; cidx += kTileThreads) {
@@ -642,7 +646,7 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
     const int x = x0 + cx, y = y0 + cy;
     if (x >= G.na || y >= G.nb) continue;
     const long long o = (long long)y * G.pitch + x;
-    double un[5];
+    X64 un[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) un[v] = (WACT || v != 3) ? uin.f[v][o] : 0.0;
 
@@ -650,37 +654,37 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       if (WACT || v != 3)
-        un[v] = un[v] + div_cell<P2>((V.fa(v, cy, cx) - V.fa(v, cy, cx + 1)) * dt, G.dx, G.inv_dx);
+        un[v] = un[v] + div_cell<P2>((X64(V.fa(v, cy, cx)) - V.fa(v, cy, cx + 1)) * dt, G.dx, G.inv_dx);
     // IY sweep (x-y plane) or IZ sweep (x-z plane), gravity on IZ
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       if (WACT || v != 3)
-        un[v] = un[v] + div_cell<P2>((V.fb(v, cy, cx) - V.fb(v, cy + 1, cx)) * dt, db, inv_db);
+        un[v] = un[v] + div_cell<P2>((X64(V.fb(v, cy, cx)) - V.fb(v, cy + 1, cx)) * dt, db, inv_db);
     if (PLANE == PLANE_XZ && G.gravity) {
       un[2] = un[2] + dt * V.q(0, cy + 2, cx + 2) * G.g;
-      un[4] = un[4] + half64(dt) * (V.fb(0, cy, cx) + V.fb(0, cy + 1, cx)) * G.g;
+      un[4] = un[4] + half_of(dt) * (X64(V.fb(0, cy, cx)) + V.fb(0, cy + 1, cx)) * G.g;
     }
     un[0] = fmax_bits(1.0e-6, un[0]);
 
     if (G.tc) {  // ThermalConduction.h:47-95, constant kappa, 2-D
-      const double kf = half64(G.kappa + G.kappa);
+      const X64 kf = half_of(X64(G.kappa) + G.kappa);
       const int hy = cy + 2, hx = cx + 2;
-      const double TC = V.temp(hy, hx);
-      const double FL = div_cell<P2>(kf * (TC - V.temp(hy, hx - 1)), G.dx, G.inv_dx);
-      const double FR = div_cell<P2>(kf * (V.temp(hy, hx + 1) - TC), G.dx, G.inv_dx);
-      const double FU = div_cell<P2>(kf * (TC - V.temp(hy - 1, hx)), db, inv_db);
-      const double FD = div_cell<P2>(kf * (V.temp(hy + 1, hx) - TC), db, inv_db);
-      const double dtdx = div_cell<P2>(dt, G.dx, G.inv_dx);
-      const double dtdb = div_cell<P2>(dt, db, inv_db);
+      const X64 TC = V.temp(hy, hx);
+      const X64 FL = div_cell<P2>(kf * (TC - V.temp(hy, hx - 1)), G.dx, G.inv_dx);
+      const X64 FR = div_cell<P2>(kf * (X64(V.temp(hy, hx + 1)) - TC), G.dx, G.inv_dx);
+      const X64 FU = div_cell<P2>(kf * (TC - V.temp(hy - 1, hx)), db, inv_db);
+      const X64 FD = div_cell<P2>(kf * (X64(V.temp(hy + 1, hx)) - TC), db, inv_db);
+      const X64 dtdx = div_cell<P2>(dt, G.dx, G.inv_dx);
+      const X64 dtdb = div_cell<P2>(dt, db, inv_db);
       un[4] = un[4] + (dtdx * (FR - FL) + dtdb * (FD - FU));
     }
     if (WACT && G.visc) {  // Viscosity.h:245-251
-      PlaneVel<PLANE, PV> P{V, cy + 2, cx + 2};
-      double vf[3][5];
+      X64 vf[3][5];
       if (VSH) {
-        visc_cell_shared<PLANE>(V, cy, cx, G.inv_dx, G.inv_dz, G.mu, vf);
+        visc_cell_shared<PLANE, X64>(V, cy, cx, G.inv_dx, G.inv_dz, G.mu, vf);
       } else {
-        viscous_plane<PLANE, double>(P, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, vf);
+        PlaneVel<PLANE, PV, X64> P{V, cy + 2, cx + 2};
+        viscous_plane<PLANE, X64>(P, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, vf);
       }
 #pragma unroll
       for (int var = 1; var < 5; ++var) {
@@ -691,14 +695,14 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
     if (kind == STAGE_RK_2) {
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        if (WACT || v != 3) un[v] = half64(u0.f[v][o] + un[v]);
+        if (WACT || v != 3) un[v] = half_of(X64(u0.f[v][o]) + un[v]);
     }
 #pragma unroll
     for (int v = 0; v < 5; ++v)
-      if (WACT || v != 3) uout.f[v][o] = un[v];
+      if (WACT || v != 3) uout.f[v][o] = un[v].v;
     if (kind != STAGE_RK_1) {
-      double q[5];
-      const double inv = inv_dt_hyp64<PLANE, WACT, P2>(un, G, q);
+      X64 q[5];
+      const double inv = inv_dt_hyp64<PLANE, WACT, P2>(un, G, q).v;
       const unsigned long long b = (unsigned long long)__double_as_longlong(inv);
       red = b > red ? b : red;
       if (above_bits(inv, 1.0e300)) atomicOr(&ctrl->err, 1);
@@ -706,12 +710,12 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
         const long long h = (long long)y * G.na + x;
 #pragma unroll
         for (int v = 0; v < 5; ++v)
-          if (hout->f[v]) hout->f[v][h] = q[v];
+          if (hout->f[v]) hout->f[v][h] = q[v].v;
       }
       if (qout) {
 #pragma unroll
         for (int v = 0; v < 5; ++v)
-          if (WACT || v != 3) qout->f[v][o] = q[v];
+          if (WACT || v != 3) qout->f[v][o] = q[v].v;
       }
     }
   }
@@ -845,8 +849,8 @@ __device__ __forceinline__ void stage_strip64(const Grid& G, const Fields& uin, 
 // stencil[dk][dj][di][var].
 template <bool CORR, class T, class PA>
 __device__ __forceinline__ void viscous3d(const PA& P, T odx, T ody, T odz, T mu, T vf[3][5]) {
-  const T four_thirds = T(4.0 / 3.0);
-  const T two_thirds = T(2.0 / 3.0);
+  const T four_thirds = four_thirds_of<T>();
+  const T two_thirds = two_thirds_of<T>();
   const T c4x = half_of(half_of(odx)), c4y = half_of(half_of(ody)), c4z = half_of(half_of(odz));
   const int U = 1, V = 2, W = 3;
 #pragma unroll
@@ -855,7 +859,7 @@ __device__ __forceinline__ void viscous3d(const PA& P, T odx, T ody, T odz, T mu
     for (int v = 0; v < 5; ++v) vf[d][v] = T(0);
 #pragma unroll
   for (int s = 1; s < 3; ++s) {  // IX
-    const T sm = (s == 1 ? T(-1) : T(1)) * mu;
+    const T sm = s == 1 ? -mu : mu;
     const T qiu = half_of(P(1, 1, s, U) + P(1, 1, s - 1, U));
     const T qiv = half_of(P(1, 1, s, V) + P(1, 1, s - 1, V));
     const T qiw = half_of(P(1, 1, s, W) + P(1, 1, s - 1, W));
@@ -876,7 +880,7 @@ __device__ __forceinline__ void viscous3d(const PA& P, T odx, T ody, T odz, T mu
   }
 #pragma unroll
   for (int s = 1; s < 3; ++s) {  // IY
-    const T sm = (s == 1 ? T(-1) : T(1)) * mu;
+    const T sm = s == 1 ? -mu : mu;
     const T qiu = half_of(P(1, s, 1, U) + P(1, s - 1, 1, U));
     const T qiv = half_of(P(1, s, 1, V) + P(1, s - 1, 1, V));
     const T qiw = half_of(P(1, s, 1, W) + P(1, s - 1, 1, W));
@@ -897,7 +901,7 @@ __device__ __forceinline__ void viscous3d(const PA& P, T odx, T ody, T odz, T mu
   }
 #pragma unroll
   for (int s = 1; s < 3; ++s) {  // IZ, with the reference's mix-ups
-    const T sm = (s == 1 ? T(-1) : T(1)) * mu;
+    const T sm = s == 1 ? -mu : mu;
     const T qiu = half_of(P(s, 1, 1, U) + P(s - 1, 1, 1, U));
     const T qiv = half_of(P(s, 1, 1, V) + P(s - 1, 1, 1, V));
     const T qiw = half_of(P(s, 1, 1, W) + P(s - 1, 1, 1, W));
