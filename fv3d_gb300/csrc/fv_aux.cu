@@ -22,6 +22,8 @@ __global__ void __launch_bounds__(256) reduce2d_fp64(const Grid G, const Fields 
   __shared__ unsigned long long s_red[8];
   opaque64_init();
   __syncthreads();
+  cell_div_init(G);
+  __syncthreads();
   unsigned long long red = 0ull;
   const long long n = (long long)G.na * G.rows;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
@@ -85,6 +87,8 @@ __global__ void __launch_bounds__(256) prim_to_cons_from(const Grid G, const Fie
   __shared__ unsigned long long s_red[8];
   opaque64_init();
   __syncthreads();
+  cell_div_init(G);
+  __syncthreads();
   unsigned long long red = 0ull;
   const long long n = (long long)G.na * G.rows;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
@@ -112,8 +116,8 @@ __global__ void __launch_bounds__(256) prim_to_cons_from(const Grid G, const Fie
         red = b > red ? b : red;
         if (!(inv <= 1.0e300)) atomicOr(&ctrl->err, 1);
       } else {
-        X64 y;
-        cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
+        Div64 D;
+        cons_to_prim64<PLANE, WACT>(u, G.gm1, q, D);
       }
       if (qout.f[0]) {
 #pragma unroll

@@ -83,12 +83,10 @@ batch_stage64(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsign
       continue;
     }
     unsigned long long red = 0ull;
-    if (I.G.pow2_all)
-      stage_segment64<PLANE, WACT, TL, true>(I.G, uin, u0, uout, ctrl, I.rs, kind, ctrl->dt_cur, x0, ya, yb, smem_raw,
-                                             nullptr, red, nullptr, nullptr, nullptr, qi, qo);
-    else
-      stage_segment64<PLANE, WACT, TL, false>(I.G, uin, u0, uout, ctrl, I.rs, kind, ctrl->dt_cur, x0, ya, yb,
-                                              smem_raw, nullptr, red, nullptr, nullptr, nullptr, qi, qo);
+    cell_div_init(I.G);
+    __syncthreads();
+    stage_segment64<PLANE, WACT, TL>(I.G, uin, u0, uout, ctrl, I.rs, kind, ctrl->dt_cur, x0, ya, yb, smem_raw, nullptr,
+                                     red, nullptr, nullptr, nullptr, qi, qo);
     if (kind != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[ctrl->parity ^ 1], s_red);
     // the copy is complete once this launch is (the next reader is a later kernel)
     if (qo && threadIdx.x == 0) ctrl->q_valid = 1;

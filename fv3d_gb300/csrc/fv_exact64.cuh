@@ -6,14 +6,6 @@
 // returns bit-for-bit the value of the reference expression it stands for
 // (for finite operands away from the subnormal range), so the FP64 stage
 // kernel stays bit-identical to the reference's CPU arithmetic.
-//
-// Division by a value whose correctly rounded reciprocal is known uses
-// Markstein's correction (P. Markstein, "Computation of elementary functions
-// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990; see
-// also Muller et al., Handbook of Floating-Point Arithmetic, the theorem on
-// correcting a quotient with a fused multiply-add): with y = RN(1/b) and
-// q0 = RN(a*y), which lies within one ulp of a/b, the residual
-// r = a - b*q0 is exactly representable (one fma) and RN(q0 + r*y) = RN(a/b).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -85,28 +77,150 @@ __device__ __forceinline__ X64 two_thirds_of<X64>() { return s_op64.two_thirds; 
 template <>
 __device__ __forceinline__ X64 four_thirds_of<X64>() { return s_op64.four_thirds; }
 
-// RN(a / b) given y = RN(1 / b): three fused operations instead of a full
-// IEEE division.
-__device__ __forceinline__ X64 div_by_rcp(X64 a, X64 b, X64 y) {
-  const X64 q0 = a * y;
-  const double r = fma(-b.v, q0.v, a.v);
-  return fma(r, y.v, q0.v);
+// ---- correctly rounded quotients and square roots, two FP64 operations each --
+// CUDA's FP64 division and square root take 137 and 143 cycles of the FP64
+// pipe per warp and SM, a reciprocal 86; the FP32 and integer pipes beside it
+// are all but idle (32 other instructions per DFMA cost nothing: 497 G
+// DFMA/s with them, 498 without).  So the result is first formed to about
+// 2^-45 from FP32 operations on the significands, split into an unevaluated
+// pair of floats (T. J. Dekker, "A floating-point technique for extending the
+// available precision", Numer. Math. 18, 1971), and made a double Q by
+// integer additions.  Then, for a quotient a / b,
+//     r = fma(-b, Q, a),   result = fma(r, y, Q),   y = 1/b to 2^-24,
+// (a square root: r = fma(-G, G, x), result = fma(r, h, G), h = 1/(2 sqrt x)):
+// the value rounded by the last operation is within 2^-15 units in the last
+// place of the exact one.  Whether that decides the rounding is tested (A.
+// Ziv, "Fast evaluation of elementary mathematical functions with correctly
+// rounded last bit", ACM TOMS 17(3), 1991): r y in units in the last place of
+// Q, computed in FP32 (error below 2^-13), must lie at least 2^-12 away from
+// every half.  Where it does not (one result in 2,048), and for operands
+// outside 2^-256 .. 2^256, the IEEE operation itself is called.  A result
+// beside a power of two, where the spacing changes, is taken only if r is
+// zero (an exact quotient).
+static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
+static __device__ __noinline__ double sqrt_ieee(double x) { return sqrt(x); }
+
+// The significand of x as h + l 2^-23: h in [1, 2) (23 bits after the point),
+// l in [0, 1) the next 23 of the 29 bits left.
+__device__ __forceinline__ void split_significand(unsigned hi, unsigned lo, unsigned expo, float& h, float& l) {
+  h = __uint_as_float((expo << 23) | (__funnelshift_l(lo, hi, 3) & 0x007fffffu));
+  l = __uint_as_float(0x3f800000u | ((lo >> 6) & 0x007fffffu)) - 1.0f;
 }
 
-// Correctly rounded reciprocal, quotient and square root.
-__device__ __forceinline__ X64 rcp64(X64 x) { return 1.0 / x.v; }
-__device__ __forceinline__ X64 div64(X64 a, X64 b) { return a.v / b.v; }
-__device__ __forceinline__ X64 sqrt64(X64 x) { return sqrt(x.v); }
-
-// (x) / d for a cell size d: an exact multiplication by 1/d when d is a power
-// of two (then 1/d is exact and scaling by it rounds nowhere), else the
-// corrected quotient above (exact for any d).  P2 is a compile-time choice:
-// the kernels branch once, uniformly, on "every cell size is a power of two",
-// because a per-call select would issue both forms.
-template <bool P2>
-__device__ __forceinline__ X64 div_cell(X64 x, X64 d, X64 inv_d) {
-  return P2 ? x * inv_d : div_by_rcp(x, d, inv_d);
+// Whether the fraction of t >= 0 (a correction in units in the last place)
+// stays 2^-12 clear of a half.
+__device__ __forceinline__ bool clear_of_half(float t) {
+  const float n = __fadd_rn(t, 12582912.0f) - 12582912.0f;  // nearest integer (t < 2^12)
+  return fabsf(t - n) < 0.5f - 0x1p-12f;
 }
+
+// A divisor prepared for several quotients.
+struct Div64 {
+  double b, y;  // the divisor, 1/b to 2^-24
+  float h, l;   // its significand (split_significand; l scaled by 2^-23)
+  float r;      // 1/(h + l) to 2^-24
+  bool ok;      // 2^-256 <= |b| < 2^256
+};
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+__device__ __forceinline__ Div64 prepare_div(X64 b) {
+  Div64 D;
+  D.b = b.v;
+  const unsigned hi = (unsigned)__double2hiint(b.v), lo = (unsigned)__double2loint(b.v);
+  const unsigned e = hi & 0x7ff00000u;
+  D.ok = e - (767u << 20) < (512u << 20);
+  split_significand(hi, lo, 127u, D.h, D.l);
+  D.l *= 0x1p-23f;
+  const float r0 = rcp_approx(D.h);
+  const float err = __fmaf_rn(-D.l, r0, __fmaf_rn(-D.h, r0, 1.0f));
+  D.r = __fmaf_rn(r0, err, r0);
+  const unsigned rb = __float_as_uint(D.r);  // 2^-1 < r <= 1
+  D.y = __hiloint2double((int)(((rb >> 3) + ((896u + 1023u) << 20) - e) | (hi & 0x80000000u)), (int)(rb << 29));
+  return D;
+}
+
+// Out of line, as the square root: inlined into every face and cell these two
+// made a translation unit take minutes to compile, and the call costs only
+// instruction issue, of which there is plenty.
+static __device__ __noinline__ double quot_call(double a_, double b_, double y_, float h_, float l_, float r_, bool ok_) {
+  const X64 a = a_;
+  const Div64 D{b_, y_, h_, l_, r_, ok_};
+  const unsigned ahi = (unsigned)__double2hiint(a.v), alo = (unsigned)__double2loint(a.v);
+  const unsigned bhi = (unsigned)__double2hiint(D.b);
+  const unsigned ea = ahi & 0x7ff00000u, eb = bhi & 0x7ff00000u;
+  float ah, al;
+  split_significand(ahi, alo, 127u, ah, al);
+  const float qh = __fmul_rn(ah, D.r);
+  const float rem = __fmaf_rn(al, 0x1p-23f, __fmaf_rn(-qh, D.l, __fmaf_rn(-qh, D.h, ah)));
+  const float ql = __fmul_rn(rem, D.r);
+  const unsigned qb = __float_as_uint(qh);
+  const bool big = qb >= 0x3f800000u;  // qh in [1, 2), else in [1/2, 1)
+  const int n = __float2int_rn(__fmul_rn(ql, big ? 0x1p49f : 0x1p50f));  // ql in units of 8 last places
+  const long long q = (((long long)((qb >> 3) + (896u << 20) + ea - eb) << 32) | (long long)(qb << 29)) +
+                      ((long long)n << 3);
+  const unsigned sign = (ahi ^ bhi) & 0x80000000u;
+  const double Q = __longlong_as_double(q ^ ((long long)sign << 32));
+  const double res = fma(-D.b, Q, a.v);
+  double out = fma(res, D.y, Q);
+  // the rounding test
+  const unsigned rhi = (unsigned)__double2hiint(res) & 0x7fffffffu, rlo = (unsigned)__double2loint(res);
+  const int x = (int)(rhi - ea + ((127u + 52u) << 20));
+  float t = __fmul_rn(x > 0 ? __uint_as_float(__funnelshift_l(rlo, (unsigned)x, 3)) : 0.0f, D.r);
+  t = big ? t : t + t;
+  const bool edge = ((qb + 1u) & 0x007fffffu) <= 1u && (rhi | rlo) != 0u;
+  const bool good = D.ok && ea - (767u << 20) < (512u << 20) && x < (int)((127u + 12u) << 20) && clear_of_half(t) &&
+                    !edge;
+  if (((ahi << 1) | alo) == 0u && D.ok) return __hiloint2double((int)sign, 0);  // 0 / b
+  if (!good) out = div_ieee(a.v, D.b);
+  return out;
+}
+
+// RN(a / D.b).
+__device__ __forceinline__ X64 quot(X64 a, const Div64& D) { return quot_call(a.v, D.b, D.y, D.h, D.l, D.r, D.ok); }
+
+// RN(a / b) for a divisor used once.
+__device__ __forceinline__ X64 div64(X64 a, X64 b) { return quot(a, prepare_div(b)); }
+
+static __device__ __noinline__ double sqrt_call(double x_) {
+  const X64 x = x_;
+  const unsigned hi = (unsigned)__double2hiint(x.v), lo = (unsigned)__double2loint(x.v);
+  const int e = (int)(hi >> 20) - 1023;
+  const int odd = e & 1, half_e = (e - odd) >> 1;
+  float mh, ml;  // x = (mh + ml) 4^half_e, mh in [1, 4)
+  split_significand(hi, lo, (unsigned)(127 + odd), mh, ml);
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(mh));
+  const float g0 = __fmul_rn(mh, y0);
+  const float y1 = __fmaf_rn(__fmul_rn(0.5f, y0), __fmaf_rn(-g0, y0, 1.0f), y0);
+  const float h = __fmul_rn(0.5f, y1);
+  const float rem = __fmaf_rn(ml, odd ? 0x1p-22f : 0x1p-23f, __fmaf_rn(-g0, g0, mh));
+  const float c = __fmul_rn(rem, h);
+  const float gl = __fmaf_rn(__fmul_rn(c, c), h, c);  // (g0 + gl)^2 = mh + ml
+  const unsigned gb = __float_as_uint(g0), hb = __float_as_uint(h);
+  const int n = __float2int_rn(__fmul_rn(gl, 0x1p49f));
+  const long long g = (((long long)((gb >> 3) + (896u << 20) + ((unsigned)half_e << 20)) << 32) |
+                       (long long)(gb << 29)) + ((long long)n << 3);
+  const double G = __longlong_as_double(g);
+  const double H = __hiloint2double((int)((hb >> 3) + (896u << 20) - ((unsigned)half_e << 20)), (int)(hb << 29));
+  const double res = fma(-G, G, x.v);
+  double out = fma(res, H, G);
+  const unsigned rhi = (unsigned)__double2hiint(res) & 0x7fffffffu, rlo = (unsigned)__double2loint(res);
+  const int s = (int)(rhi - ((unsigned)(2 * half_e + 1023) << 20) + ((127u + 52u) << 20));
+  const float t = __fmul_rn(s > 0 ? __uint_as_float(__funnelshift_l(rlo, (unsigned)s, 3)) : 0.0f, h);
+  const bool inside = gb - 0x3f800001u < 0x007ffffeu;  // 1 < g0 < 2, not beside either
+  const bool good = hi - (767u << 20) < (512u << 20) && s < (int)((127u + 12u) << 20) && clear_of_half(t) &&
+                    (inside || (rhi | rlo) == 0u);
+  if (!good) out = sqrt_ieee(x.v);
+  return out;
+}
+
+// RN(sqrt(x)).
+__device__ __forceinline__ X64 sqrt64(X64 x) { return sqrt_call(x.v); }
 
 // The reference formula of minmod, out of line: the rare operands that reach
 // it (NaN, infinities, a product that may underflow) take a real branch, so
@@ -211,7 +325,6 @@ __device__ __forceinline__ X64 recon_minus(X64 q, X64 slope) { return fma(-slope
 // arithmetic exactly as the reference evaluates them.
 struct Consts64 {
   X64 gamma;     // gamma0
-  X64 gm1;       // gamma0 - 1 (exact for 1 < gamma0 < 3)
   X64 inv_gm1;   // RN(1 / (gamma0 - 1)), also HLLC's `entho`
 };
 

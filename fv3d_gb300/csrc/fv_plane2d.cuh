@@ -12,6 +12,36 @@
 
 namespace fv {
 
+// The constant divisors of a problem -- cell sizes and gamma - 1 -- prepared
+// in shared memory once per kernel (or work item).
+struct CellDiv64 {
+  Div64 d[3];     // dx, dy, dz
+  Div64 gm1;
+  double inv[3];  // RN(1/d)
+  int pow2;       // every cell size is a power of two: 1/d is exact
+};
+static __shared__ CellDiv64 s_cell64;
+
+// Every thread calls it, after a __syncthreads that follows opaque64_init and
+// the store of G; another must come before the first division.
+__device__ __forceinline__ void cell_div_init(const Grid& G) {
+  const int t = threadIdx.x;
+  if (t < 3) {
+    s_cell64.d[t] = prepare_div(t == 0 ? G.dx : (t == 1 ? G.dy : G.dz));
+    s_cell64.inv[t] = t == 0 ? G.inv_dx : (t == 1 ? G.inv_dy : G.inv_dz);
+  }
+  if (t == 3) s_cell64.gm1 = prepare_div(G.gm1);
+  if (t == 4) s_cell64.pow2 = G.pow2_all;
+}
+
+// x / d for the cell size of an axis: an exact multiplication by 1/d when the
+// cell sizes are powers of two (then 1/d is exact and scaling by it rounds
+// nowhere; a uniform branch), else a quotient.
+__device__ __forceinline__ X64 div_cell(X64 x, int axis) {
+  if (s_cell64.pow2) return x * s_cell64.inv[axis];
+  return quot(x, s_cell64.d[axis]);
+}
+
 // Storage slot (1 = a, 2 = b, 3 = c) of the reference's physical velocity
 // component var (1 = x, 2 = y, 3 = z).
 template <int PLANE>
@@ -20,18 +50,17 @@ __device__ __forceinline__ constexpr int phys_slot(int var) {
 }
 
 // consToPrim (States.h:34-45) of a state held in storage order; returns
-// (rho, u_a, u_b, u_c, p) and, through y, RN(1/rho).  The kinetic energy sums
+// (rho, u_a, u_b, u_c, p) and, through D, the prepared density.  The kinetic energy sums
 // the physical x, y, z velocities in the reference's order; with WACT false
 // the degenerate velocity is exactly zero and its (exact) zero terms are
-// dropped.  The three divisions by rho share one correctly rounded
-// reciprocal (Markstein correction, fv_exact64.cuh).
+// dropped.  The divisions by rho share its preparation (quot, fv_exact64.cuh).
 template <int PLANE, bool WACT>
-__device__ __forceinline__ void cons_to_prim64(const X64 u[5], X64 gm1, X64 q[5], X64& y) {
+__device__ __forceinline__ void cons_to_prim64(const X64 u[5], X64 gm1, X64 q[5], Div64& D) {
   const X64 r = u[0];
-  y = rcp64(r);
-  const X64 va = div_by_rcp(u[1], r, y);
-  const X64 vb = div_by_rcp(u[2], r, y);
-  const X64 vc = WACT ? div_by_rcp(u[3], r, y) : X64(0.0);
+  D = prepare_div(r);
+  const X64 va = quot(u[1], D);
+  const X64 vb = quot(u[2], D);
+  const X64 vc = WACT ? quot(u[3], D) : X64(0.0);
   X64 ke;
   if (WACT) {
     const X64 vx = va, vy = PLANE == PLANE_XY ? vb : vc, vz = PLANE == PLANE_XY ? vc : vb;
@@ -50,19 +79,20 @@ __device__ __forceinline__ void cons_to_prim64(const X64 u[5], X64 gm1, X64 q[5]
 // Hyperbolic inverse time step of one cell, ComputeDt.h:49-52:
 // (cs + |u|)/dx + (cs + |v|)/dy + (cs + |w|)/dz with cs = sqrt(p*gamma/rho).
 // qout, when given, receives the primitives consToPrim computes on the way.
-template <int PLANE, bool WACT, bool P2 = false>
+template <int PLANE, bool WACT>
 __device__ __forceinline__ X64 inv_dt_hyp64(const X64 u[5], const Grid& G, X64* qout = nullptr) {
-  X64 q[5], y;
-  cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
+  X64 q[5];
+  Div64 D;
+  cons_to_prim64<PLANE, WACT>(u, G.gm1, q, D);
   if (qout) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) qout[v] = q[v];
   }
-  const X64 cs = sqrt64(div_by_rcp(q[4] * G.gamma, q[0], y));
+  const X64 cs = sqrt64(quot(q[4] * G.gamma, D));
   const X64 vx = q[1], vy = PLANE == PLANE_XY ? q[2] : q[3], vz = PLANE == PLANE_XY ? q[3] : q[2];
-  const X64 tx = div_cell<P2>(cs + fabs(vx.v), G.dx, G.inv_dx);
-  const X64 ty = div_cell<P2>(cs + fabs(vy.v), G.dy, G.inv_dy);
-  const X64 tz = div_cell<P2>(cs + fabs(vz.v), G.dz, G.inv_dz);
+  const X64 tx = div_cell(cs + fabs(vx.v), 0);
+  const X64 ty = div_cell(cs + fabs(vy.v), 1);
+  const X64 tz = div_cell(cs + fabs(vz.v), 2);
   return tx + ty + tz;
 }
 

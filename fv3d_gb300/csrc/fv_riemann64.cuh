@@ -6,11 +6,10 @@
 // that is identically zero in a 2-D run without a third velocity (1: t1,
 // 2: t2, 0: none); its terms are exact zeros in the reference arithmetic and
 // are dropped.  Cheaper-but-identical steps, each returning the same bits:
-//   - p/(gamma-1) via the corrected quotient with RN(1/(gamma-1));
-//   - the five HLL flux components share one reciprocal of SR-SL, and each
-//     state's sound speed and kinetic energy share one reciprocal of rho;
+//   - quotients and square roots by FP32-seeded two-operation forms (quot,
+//     sqrt64 in fv_exact64.cuh), a divisor prepared once for its quotients;
 //   - HLLC's max(cL, cR) as sqrt(max(cL^2, cR^2)) (sqrt is monotone and
-//     correctly rounded), and u*, p* / the star state share reciprocals;
+//     correctly rounded);
 //   - products with 0.5 by exponent arithmetic (half64, exact);
 //   - wave-speed min / max and region tests on bit patterns (fmin_bits,
 //     gt0_bits, ...: integer pipe, same results; an FP64 comparison takes 19
@@ -18,7 +17,7 @@
 #pragma once
 
 #include "fv_device.cuh"
-#include "fv_exact64.cuh"
+#include "fv_plane2d.cuh"
 
 namespace fv {
 
@@ -42,14 +41,14 @@ __device__ __forceinline__ void euler_flux64(const Slots<X64>& q, X64 e, X64 F[5
   F[4] = (q.p + E) * q.un;
 }
 
-// primToCons (States.h:20-31) given e = p/(gamma-1) and y = RN(1/rho).
+// primToCons (States.h:20-31) given e = p/(gamma-1) and the prepared density.
 template <int ZS>
-__device__ __forceinline__ void prim_to_cons64(const Slots<X64>& q, X64 e, X64 y, X64 u[5]) {
+__device__ __forceinline__ void prim_to_cons64(const Slots<X64>& q, X64 e, const Div64& rho, X64 u[5]) {
   u[0] = q.r;
   u[1] = q.r * q.un;
   u[2] = ZS == 1 ? 0.0 : q.r * q.t1;
   u[3] = ZS == 2 ? 0.0 : q.r * q.t2;
-  const X64 Ek = div_by_rcp(half_of(ke_sum3<ZS>(u[1], u[2], u[3])), q.r, y);
+  const X64 Ek = quot(half_of(ke_sum3<ZS>(u[1], u[2], u[3])), rho);
   u[4] = Ek + e;
 }
 
@@ -59,15 +58,15 @@ __device__ __forceinline__ void prim_to_cons64(const Slots<X64>& q, X64 e, X64 y
 template <int ZS>
 __device__ __forceinline__ void hll64(const Slots<X64>& L, const Slots<X64>& R, const Consts64& K,
                                       X64 flux[5], X64* pout = nullptr) {
-  // one correctly rounded reciprocal of each density serves both quotients by
-  // it (the sound speed's p*gamma/rho and, in the star region, Ek/rho)
-  const X64 yL = rcp64(L.r), yR = rcp64(R.r);
-  const X64 aL = sqrt64(div_by_rcp(L.p * K.gamma, L.r, yL));
-  const X64 aR = sqrt64(div_by_rcp(R.p * K.gamma, R.r, yR));
+  // each density, prepared once, divides twice (the sound speed's p*gamma and,
+  // in the star region, the kinetic energy)
+  const Div64 rhoL = prepare_div(L.r), rhoR = prepare_div(R.r);
+  const X64 aL = sqrt64(quot(L.p * K.gamma, rhoL));
+  const X64 aR = sqrt64(quot(R.p * K.gamma, rhoR));
   const X64 SL = fmin_bits(L.un - aL, R.un - aR);
   const X64 SR = fmax_bits(L.un + aL, R.un + aR);
-  const X64 eL = div_by_rcp(L.p, K.gm1, K.inv_gm1);
-  const X64 eR = div_by_rcp(R.p, K.gm1, K.inv_gm1);
+  const X64 eL = quot(L.p, s_cell64.gm1);
+  const X64 eR = quot(R.p, s_cell64.gm1);
   X64 FL[5], FR[5];
   euler_flux64<ZS>(L, eL, FL);
   euler_flux64<ZS>(R, eR, FR);
@@ -82,18 +81,17 @@ __device__ __forceinline__ void hll64(const Slots<X64>& L, const Slots<X64>& R, 
   } else {
     if (pout) *pout = half_of(L.p + R.p);
     X64 uL[5], uR[5];
-    prim_to_cons64<ZS>(L, eL, yL, uL);
-    prim_to_cons64<ZS>(R, eR, yR, uR);
+    prim_to_cons64<ZS>(L, eL, rhoL, uL);
+    prim_to_cons64<ZS>(R, eR, rhoR, uR);
     const X64 slsr = SL * SR;
-    const X64 den = SR - SL;
-    const X64 y = rcp64(den);
+    const Div64 den = prepare_div(SR - SL);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       if ((ZS == 1 && v == 2) || (ZS == 2 && v == 3)) {
         flux[v] = 0.0;
         continue;
       }
-      flux[v] = div_by_rcp((FL[v] * SR - FR[v] * SL) + (uR[v] - uL[v]) * slsr, den, y);
+      flux[v] = quot((FL[v] * SR - FR[v] * SL) + (uR[v] - uL[v]) * slsr, den);
     }
   }
 }
@@ -118,10 +116,9 @@ __device__ __forceinline__ void hllc64(const Slots<X64>& L, const Slots<X64>& R,
   const X64 SR = fmax_bits(uL, uR) + cmax;
   const X64 rcL = rL * (uL - SL);
   const X64 rcR = rR * (SR - uR);
-  const X64 D = rcR + rcL;
-  const X64 yD = rcp64(D);
-  const X64 uS = div_by_rcp(rcR * uR + rcL * uL + (pL - pR), D, yD);
-  const X64 pS = div_by_rcp(rcR * pL + rcL * pR + rcL * rcR * (uL - uR), D, yD);
+  const Div64 D = prepare_div(rcR + rcL);
+  const X64 uS = quot(rcR * uR + rcL * uL + (pL - pR), D);
+  const X64 pS = quot(rcR * pL + rcL * pR + rcL * rcR * (uL - uR), D);
   X64 sr, su, st1, st2, sp, E;
   if (gt0_bits(SL)) {
     sr = rL; su = uL; st1 = L.t1; st2 = L.t2; sp = pL; E = EL;
@@ -131,10 +128,9 @@ __device__ __forceinline__ void hllc64(const Slots<X64>& L, const Slots<X64>& R,
     const bool left = gt0_bits(uS);
     const X64 rK = left ? rL : rR, uK = left ? uL : uR, pK = left ? pL : pR, EK = left ? EL : ER;
     const X64 SK = left ? SL : SR;
-    const X64 den = SK - uS;
-    const X64 y = rcp64(den);
-    sr = div_by_rcp(rK * (SK - uK), den, y);
-    E = div_by_rcp((SK - uK) * EK - pK * uK + pS * uS, den, y);
+    const Div64 den = prepare_div(SK - uS);
+    sr = quot(rK * (SK - uK), den);
+    E = quot((SK - uK) * EK - pK * uK + pS * uS, den);
     su = uS;
     sp = pS;
     st1 = left ? L.t1 : R.t1;

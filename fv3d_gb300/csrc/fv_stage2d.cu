@@ -42,6 +42,8 @@ stage2d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u
     }
   }
   __syncthreads();
+  cell_div_init(G);
+  __syncthreads();
   // the primitive copy of uin, when the last stage that wrote uin left one
   const bool prims = qin.f[0] != nullptr && ctrl->q_valid != 0;
   const Fields* qi = prims ? &qin : nullptr;
@@ -49,12 +51,8 @@ stage2d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u
   const TmaState* tp = prims ? (use_tq ? &tq : nullptr) : (use_tma ? &tin : nullptr);
   const Fields* ho = hout.f[0] ? &hout : nullptr;
   const long long ub = units * blockIdx.x / gridDim.x, ue = units * (blockIdx.x + 1) / gridDim.x;
-  if (G.pow2_all)
-    stage_strip64<PLANE, WACT, SingleTile, true>(G, uin, u0, uout, ctrl, RS, KIND, ub, ue, smem, s_red, ho, tp,
-                                                 &s_mbar, qi, qo);
-  else
-    stage_strip64<PLANE, WACT, SingleTile, false>(G, uin, u0, uout, ctrl, RS, KIND, ub, ue, smem, s_red, ho, tp,
-                                                  &s_mbar, qi, qo);
+  stage_strip64<PLANE, WACT, SingleTile>(G, uin, u0, uout, ctrl, RS, KIND, ub, ue, smem, s_red, ho, tp, &s_mbar, qi,
+                                         qo);
   pdl_trigger();
 }
 

@@ -65,21 +65,21 @@ struct Smem3 {
 // Ring slot of z layer kg (kg >= -2).
 __device__ __forceinline__ int slot_of(int kg) { return (kg + 4) & 3; }
 
-// consToPrim of one stored cell (x, y, z storage order), RN(1/rho) in y.
-// With qsrc (the primitive copy of u, the same bits) the primitives are read
-// and y is computed only when need_y.
+// consToPrim of one stored cell (x, y, z storage order), the prepared density
+// in D.  With qsrc (the primitive copy of u, the same bits) the primitives are
+// read and D is prepared only when need_d.
 __device__ __forceinline__ void load_prim(const Fields& u, const Fields* qsrc, long long o, X64 gm1, X64 q[5],
-                                          X64& y, bool need_y = false) {
+                                          Div64& D, bool need_d = false) {
   if (qsrc) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) q[v] = qsrc->f[v][o];
-    y = need_y ? rcp64(q[0]) : X64(0.0);
+    if (need_d) D = prepare_div(q[0]);
     return;
   }
   X64 w[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) w[v] = u.f[v][o];
-  cons_to_prim64<PLANE_XY, true>(w, gm1, q, y);
+  cons_to_prim64<PLANE_XY, true>(w, gm1, q, D);
 }
 
 // fillC91 (BoundaryConditions.h:87-134) for ghost layer kg of column (sa, sb)
@@ -90,9 +90,10 @@ __device__ __forceinline__ void c91_ghost(const Grid& G, const Fields& u, const 
                                           bool fb, int kg, X64 res[5]) {
   const int kref = kg < 0 ? 0 : G.nc - 1;
   const int ksym = kg < 0 ? -kg - 1 : 2 * G.nc - kg - 1;
-  X64 qref[5], qsym[5], y;
-  load_prim(u, qsrc, (long long)kref * G.nb * G.pitch + col, G.gm1, qref, y);
-  load_prim(u, qsrc, (long long)ksym * G.nb * G.pitch + col, G.gm1, qsym, y);
+  X64 qref[5], qsym[5];
+  Div64 D;
+  load_prim(u, qsrc, (long long)kref * G.nb * G.pitch + col, G.gm1, qref, D);
+  load_prim(u, qsrc, (long long)ksym * G.nb * G.pitch + col, G.gm1, qsym, D);
   if (fa) {
     qref[1] = -qref[1];
     qsym[1] = -qsym[1];
@@ -149,12 +150,12 @@ __device__ __forceinline__ void load_layer(const Grid& G, const Fields& u, const
     X64 q[5];
     X64 T = 0.0;
     if (!c91) {
-      X64 y;
-      load_prim(u, qsrc, zoff + col, G.gm1, q, y, G.tc != 0);
+      Div64 D;
+      load_prim(u, qsrc, zoff + col, G.gm1, q, D, G.tc != 0);
       if (fa) q[1] = -q[1];
       if (fb) q[2] = -q[2];
       if (fz) q[3] = -q[3];
-      if (G.tc) T = div_by_rcp(q[4], q[0], y);
+      if (G.tc) T = quot(q[4], D);
     } else {
       c91_ghost(G, u, qsrc, col, fa, fb, kg, q);
       if (G.tc) T = div64(q[4], q[0]);
@@ -327,7 +328,7 @@ __device__ __forceinline__ void viscous_iz3d(const PA& P, X64 odx, X64 odz, X64 
 // branch on it once, uniformly).  Every thread of the CTA must call it; the
 // CFL maximum is folded into red (the caller reduces it once per CTA or work
 // item).
-template <bool P2, bool CORR>
+template <bool CORR>
 __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin, const Fields& u0,
                                                 const Fields& uout, StepCtrl* __restrict__ ctrl, int rs, int kind,
                                                 int bx, int by, int k0, int k1, const Fields& hout, double* smem_raw,
@@ -353,7 +354,7 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
     return;
   }
   const X64 dt = ctrl->dt_cur;
-  const Consts64 K{G.gamma, G.gm1, G.inv_gm1};
+  const Consts64 K{G.gamma, G.inv_gm1};
   const int recon = G.recon;
   const bool need_pout = G.wb_flux_z || G.bc_c == DBC_C91;
   const bool vsh = !CORR && G.visc;  // shared-face viscous fluxes (FA / FB reused)
@@ -420,10 +421,10 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
       // IX, IY: un += (F(-1/2) - F(+1/2)) * dt / d
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        un[v] = un[v] + div_cell<P2>((X64(S.fa(v, cy, cx)) - S.fa(v, cy, cx + 1)) * dt, G.dx, G.inv_dx);
+        un[v] = un[v] + div_cell((X64(S.fa(v, cy, cx)) - S.fa(v, cy, cx + 1)) * dt, 0);
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        un[v] = un[v] + div_cell<P2>((X64(S.fb(v, cy, cx)) - S.fb(v, cy + 1, cx)) * dt, G.dy, G.inv_dy);
+        un[v] = un[v] + div_cell((X64(S.fb(v, cy, cx)) - S.fb(v, cy + 1, cx)) * dt, 1);
       // IZ with the z-boundary overrides of Update.h:131-143
       X64 fL[5], fR[5];
 #pragma unroll
@@ -450,7 +451,7 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
         }
       }
 #pragma unroll
-      for (int v = 0; v < 5; ++v) un[v] = un[v] + div_cell<P2>((fL[v] - fR[v]) * dt, G.dz, G.inv_dz);
+      for (int v = 0; v < 5; ++v) un[v] = un[v] + div_cell((fL[v] - fR[v]) * dt, 2);
       if (G.gravity) {
         un[3] = un[3] + dt * rho_c * G.g;
         un[4] = un[4] + half_of(dt) * (fL[0] + fR[0]) * G.g;
@@ -468,23 +469,23 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
         }
         const int hy = cy + 2, hx = cx + 2;
         const X64 TC = S.temp(sk, hy, hx);
-        const X64 FL = div_cell<P2>(kC * (TC - S.temp(sk, hy, hx - 1)), G.dx, G.inv_dx);
-        const X64 FR = div_cell<P2>(kC * (X64(S.temp(sk, hy, hx + 1)) - TC), G.dx, G.inv_dx);
-        const X64 FU = div_cell<P2>(kC * (TC - S.temp(sk, hy - 1, hx)), G.dy, G.inv_dy);
-        const X64 FD = div_cell<P2>(kC * (X64(S.temp(sk, hy + 1, hx)) - TC), G.dy, G.inv_dy);
-        X64 FF = div_cell<P2>(kF * (TC - S.temp(slot_of(k - 1), hy, hx)), G.dz, G.inv_dz);
-        X64 FB = div_cell<P2>(kB * (X64(S.temp(slot_of(k + 1), hy, hx)) - TC), G.dz, G.inv_dz);
+        const X64 FL = div_cell(kC * (TC - S.temp(sk, hy, hx - 1)), 0);
+        const X64 FR = div_cell(kC * (X64(S.temp(sk, hy, hx + 1)) - TC), 0);
+        const X64 FU = div_cell(kC * (TC - S.temp(sk, hy - 1, hx)), 1);
+        const X64 FD = div_cell(kC * (X64(S.temp(sk, hy + 1, hx)) - TC), 1);
+        X64 FF = div_cell(kF * (TC - S.temp(slot_of(k - 1), hy, hx)), 2);
+        X64 FB = div_cell(kB * (X64(S.temp(slot_of(k + 1), hy, hx)) - TC), 2);
         if (k == 0 && G.bctc_zmin != 0) {
-          if (G.bctc_zmin == 1) FF = div_cell<P2>(kF * 2.0 * (TC - G.bctc_zmin_value), G.dz, G.inv_dz);
+          if (G.bctc_zmin == 1) FF = div_cell(kF * 2.0 * (TC - G.bctc_zmin_value), 2);
           else FF = kF * G.bctc_zmin_value;
         }
         if (k == G.nc - 1 && G.bctc_zmax != 0) {
-          if (G.bctc_zmax == 1) FB = div_cell<P2>(kB * 2.0 * (X64(G.bctc_zmax_value) - TC), G.dz, G.inv_dz);
+          if (G.bctc_zmax == 1) FB = div_cell(kB * 2.0 * (X64(G.bctc_zmax_value) - TC), 2);
           else FB = kB * G.bctc_zmax_value;
         }
-        const X64 dtdx = div_cell<P2>(dt, G.dx, G.inv_dx);
-        const X64 dtdy = div_cell<P2>(dt, G.dy, G.inv_dy);
-        const X64 dtdz = div_cell<P2>(dt, G.dz, G.inv_dz);
+        const X64 dtdx = div_cell(dt, 0);
+        const X64 dtdy = div_cell(dt, 1);
+        const X64 dtdz = div_cell(dt, 2);
         un[4] = un[4] + (dtdx * (FR - FL) + dtdy * (FD - FU) + dtdz * (FB - FF));
       }
       if (G.visc && !vsh) {  // Viscosity.h:145-151
@@ -494,8 +495,8 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
         if (CORR) {  // the flux differences divided by the cell sizes
 #pragma unroll
           for (int v = 1; v < 5; ++v)
-            un[v] = un[v] + dt * (div_cell<P2>(vf[0][v], G.dx, G.inv_dx) + div_cell<P2>(vf[1][v], G.dy, G.inv_dy) +
-                                  div_cell<P2>(vf[2][v], G.dz, G.inv_dz));
+            un[v] = un[v] + dt * (div_cell(vf[0][v], 0) + div_cell(vf[1][v], 1) +
+                                  div_cell(vf[2][v], 2));
         } else {
 #pragma unroll
           for (int v = 1; v < 5; ++v) un[v] = un[v] + dt * (vf[0][v] + vf[1][v] + vf[2][v]);
@@ -546,7 +547,7 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
       for (int v = 0; v < 5; ++v) uout.f[v][o] = un[v].v;
       if (kind != STAGE_RK_1) {
         X64 q[5];
-        const double inv = inv_dt_hyp64<PLANE_XY, true, P2>(un, G, q).v;
+        const double inv = inv_dt_hyp64<PLANE_XY, true>(un, G, q).v;
         const unsigned long long b = (unsigned long long)__double_as_longlong(inv);
         red = b > red ? b : red;
         if (above_bits(inv, 1.0e300)) atomicOr(&ctrl->err, 1);
@@ -571,7 +572,7 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
 
 // One stage for the columns (bx, by) and z chunk bz of tz layers, reduced
 // (the batch kernel's work item).
-template <bool P2, bool CORR>
+template <bool CORR>
 __device__ __forceinline__ void stage3d_body(const Grid& G, const Fields& uin, const Fields& u0, const Fields& uout,
                                              StepCtrl* __restrict__ ctrl, int rs, int kind, int bx, int by, int bz,
                                              int tz, const Fields& hout, double* smem_raw,
@@ -580,13 +581,13 @@ __device__ __forceinline__ void stage3d_body(const Grid& G, const Fields& uin, c
   const int k0 = bz * tz;
   const int k1 = min(k0 + tz, G.nc);
   unsigned long long red = 0ull;
-  stage3d_segment<P2, CORR>(G, uin, u0, uout, ctrl, rs, kind, bx, by, k0, k1, hout, smem_raw, red);
+  stage3d_segment<CORR>(G, uin, u0, uout, ctrl, rs, kind, bx, by, k0, k1, hout, smem_raw, red);
   if (active && kind != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[parity ^ 1], s_red);
 }
 
 // Units [ub, ue) of the (column block, z layer) numbering, column block by
 // column block; returns the CTA's CFL maximum.
-template <bool P2, bool CORR, int RS, int KIND>
+template <bool CORR, int RS, int KIND>
 __device__ __forceinline__ unsigned long long march3d(const Grid& G, const Fields& uin, const Fields& u0,
                                                       const Fields& uout, StepCtrl* __restrict__ ctrl, long long ub,
                                                       long long ue, const Fields& hout, double* smem_raw,
@@ -598,7 +599,7 @@ __device__ __forceinline__ unsigned long long march3d(const Grid& G, const Field
     const int k0 = (int)(u - (long long)cb * G.nc);
     const int k1 = (int)(k0 + (ue - u) < (long long)G.nc ? k0 + (ue - u) : (long long)G.nc);
     u += k1 - k0;
-    stage3d_segment<P2, CORR>(G, uin, u0, uout, ctrl, RS, KIND, cb % tiles_x, cb / tiles_x, k0, k1, hout, smem_raw,
+    stage3d_segment<CORR>(G, uin, u0, uout, ctrl, RS, KIND, cb % tiles_x, cb / tiles_x, k0, k1, hout, smem_raw,
                               red, qin, qout);
   }
   return red;
@@ -619,14 +620,15 @@ stage3d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u
   opaque64_init();
   pdl_wait();
   __syncthreads();
+  cell_div_init(G);
+  __syncthreads();
   const long long ub = units * blockIdx.x / gridDim.x, ue = units * (blockIdx.x + 1) / gridDim.x;
   const int active = ctrl->active, parity = ctrl->parity;
   // the primitive copy of uin, when the last stage that wrote uin left one
   const Fields* qi = qin.f[0] && ctrl->q_valid ? &qin : nullptr;
   const Fields* qo = qout.f[0] ? &qout : nullptr;
   const unsigned long long red =
-      G.pow2_all ? march3d<true, CORR, RS, KIND>(G, uin, u0, uout, ctrl, ub, ue, hout, smem_raw, qi, qo)
-                 : march3d<false, CORR, RS, KIND>(G, uin, u0, uout, ctrl, ub, ue, hout, smem_raw, qi, qo);
+      march3d<CORR, RS, KIND>(G, uin, u0, uout, ctrl, ub, ue, hout, smem_raw, qi, qo);
   if (active && KIND != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[parity ^ 1], s_red);
   // the copy is complete once this launch is (the next reader is a later kernel)
   if (active && qo && threadIdx.x == 0) ctrl->q_valid = 1;
@@ -741,11 +743,10 @@ batch_stage3d64(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsi
     } else {
       uin = flip ? I.B : I.A; u0 = uin; uout = flip ? I.A : I.B;
     }
-    // the group shares the solver (RS); the cell-size form is a uniform branch
-    if (I.G.pow2_all)
-      stage3d_body<true, CORR>(I.G, uin, u0, uout, I.ctrl, RS, kind, bx, by, bz, I.tz, none, smem_raw, s_red);
-    else
-      stage3d_body<false, CORR>(I.G, uin, u0, uout, I.ctrl, RS, kind, bx, by, bz, I.tz, none, smem_raw, s_red);
+    cell_div_init(I.G);
+    __syncthreads();
+    // the group shares the solver (RS)
+    stage3d_body<CORR>(I.G, uin, u0, uout, I.ctrl, RS, kind, bx, by, bz, I.tz, none, smem_raw, s_red);
   }
 }
 

@@ -500,7 +500,8 @@ __device__ __forceinline__ void load_prims64(const Grid& G, const Fields& uin, c
     const int sa = bc_source(x0 + hx - 2, G.na, G.bc_a, fa);
     const int sb = bc_source(y0 + hy - 2, G.nb, G.bc_b, fb);
     const long long o = (long long)sb * G.pitch + sa;
-    X64 u[5], q[5], y = 0.0;
+    X64 u[5], q[5];
+    Div64 D;
     u[0] = uin.f[0][o];
     u[1] = uin.f[1][o];
     u[2] = uin.f[2][o];
@@ -509,16 +510,16 @@ __device__ __forceinline__ void load_prims64(const Grid& G, const Fields& uin, c
     if (prims) {
 #pragma unroll
       for (int v = 0; v < 5; ++v) q[v] = u[v];
-      if (G.tc) y = rcp64(q[0]);
+      if (G.tc) D = prepare_div(q[0]);
     } else {
-      cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
+      cons_to_prim64<PLANE, WACT>(u, G.gm1, q, D);
     }
     if (fa) q[1] = -q[1];
     if (fb) q[2] = -q[2];
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       if (WACT || v != 3) V.q(v, hy, hx) = q[v].v;
-    if (G.tc) V.temp(hy, hx) = div_by_rcp(q[4], q[0], y).v;
+    if (G.tc) V.temp(hy, hx) = quot(q[4], D).v;
   }
 }
 
@@ -537,20 +538,21 @@ __device__ __forceinline__ void convert_rows64(const Grid& G, const PV& V, int h
     const int hy = h0 + r;
     if (prims) {  // only the temperature
       const X64 r = V.q(0, hy, hx), p = V.q(4, hy, hx);
-      V.temp(hy, hx) = div_by_rcp(p, r, rcp64(r)).v;
+      V.temp(hy, hx) = div64(p, r).v;
       continue;
     }
-    X64 u[5], q[5], y;
+    X64 u[5], q[5];
+    Div64 D;
     u[0] = V.q(0, hy, hx);
     u[1] = V.q(1, hy, hx);
     u[2] = V.q(2, hy, hx);
     u[3] = WACT ? V.q(3, hy, hx) : 0.0;
     u[4] = V.q(4, hy, hx);
-    cons_to_prim64<PLANE, WACT>(u, G.gm1, q, y);
+    cons_to_prim64<PLANE, WACT>(u, G.gm1, q, D);
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       if (WACT || v != 3) V.q(v, hy, hx) = q[v].v;
-    if (G.tc) V.temp(hy, hx) = div_by_rcp(q[4], q[0], y).v;
+    if (G.tc) V.temp(hy, hx) = quot(q[4], D).v;
   }
 }
 
@@ -630,15 +632,14 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
 //
 // qout (optional, last stage of a step): the primitives of the result are
 // also written there, in the state's own layout, for the next step's load.
-template <int PLANE, bool WACT, class TL, bool P2, bool VSH, class PV>
+template <int PLANE, bool WACT, class TL, bool VSH, class PV>
 __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Fields& uin, const Fields& u0,
                                          const Fields& uout, StepCtrl* ctrl, int kind, double dt_step, int x0, int y0,
                                          int nr, int tid, const Fields* hout, unsigned long long& red,
                                          const Fields* qout = nullptr) {
   constexpr int TX = TL::TX;
   const X64 dt = dt_step;
-  const X64 db = PLANE == PLANE_XY ? G.dy : G.dz;
-  const X64 inv_db = PLANE == PLANE_XY ? G.inv_dy : G.inv_dz;
+  constexpr int kB = PLANE == PLANE_XY ? 1 : 2;  // the axis of b
   const int ncell = TX * nr;
 #pragma unroll 1
   for (int cidx = tid; cidx < ncell; cidx += kTileThreads) {
@@ -654,12 +655,12 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       if (WACT || v != 3)
-        un[v] = un[v] + div_cell<P2>((X64(V.fa(v, cy, cx)) - V.fa(v, cy, cx + 1)) * dt, G.dx, G.inv_dx);
+        un[v] = un[v] + div_cell((X64(V.fa(v, cy, cx)) - V.fa(v, cy, cx + 1)) * dt, 0);
     // IY sweep (x-y plane) or IZ sweep (x-z plane), gravity on IZ
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       if (WACT || v != 3)
-        un[v] = un[v] + div_cell<P2>((X64(V.fb(v, cy, cx)) - V.fb(v, cy + 1, cx)) * dt, db, inv_db);
+        un[v] = un[v] + div_cell((X64(V.fb(v, cy, cx)) - V.fb(v, cy + 1, cx)) * dt, kB);
     if (PLANE == PLANE_XZ && G.gravity) {
       un[2] = un[2] + dt * V.q(0, cy + 2, cx + 2) * G.g;
       un[4] = un[4] + half_of(dt) * (X64(V.fb(0, cy, cx)) + V.fb(0, cy + 1, cx)) * G.g;
@@ -670,12 +671,12 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
       const X64 kf = half_of(X64(G.kappa) + G.kappa);
       const int hy = cy + 2, hx = cx + 2;
       const X64 TC = V.temp(hy, hx);
-      const X64 FL = div_cell<P2>(kf * (TC - V.temp(hy, hx - 1)), G.dx, G.inv_dx);
-      const X64 FR = div_cell<P2>(kf * (X64(V.temp(hy, hx + 1)) - TC), G.dx, G.inv_dx);
-      const X64 FU = div_cell<P2>(kf * (TC - V.temp(hy - 1, hx)), db, inv_db);
-      const X64 FD = div_cell<P2>(kf * (X64(V.temp(hy + 1, hx)) - TC), db, inv_db);
-      const X64 dtdx = div_cell<P2>(dt, G.dx, G.inv_dx);
-      const X64 dtdb = div_cell<P2>(dt, db, inv_db);
+      const X64 FL = div_cell(kf * (TC - V.temp(hy, hx - 1)), 0);
+      const X64 FR = div_cell(kf * (X64(V.temp(hy, hx + 1)) - TC), 0);
+      const X64 FU = div_cell(kf * (TC - V.temp(hy - 1, hx)), kB);
+      const X64 FD = div_cell(kf * (X64(V.temp(hy + 1, hx)) - TC), kB);
+      const X64 dtdx = div_cell(dt, 0);
+      const X64 dtdb = div_cell(dt, kB);
       un[4] = un[4] + (dtdx * (FR - FL) + dtdb * (FD - FU));
     }
     if (WACT && G.visc) {  // Viscosity.h:245-251
@@ -702,7 +703,7 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
       if (WACT || v != 3) uout.f[v][o] = un[v].v;
     if (kind != STAGE_RK_1) {
       X64 q[5];
-      const double inv = inv_dt_hyp64<PLANE, WACT, P2>(un, G, q).v;
+      const double inv = inv_dt_hyp64<PLANE, WACT>(un, G, q).v;
       const unsigned long long b = (unsigned long long)__double_as_longlong(inv);
       red = b > red ? b : red;
       if (above_bits(inv, 1.0e300)) atomicOr(&ctrl->err, 1);
@@ -755,7 +756,7 @@ __device__ __forceinline__ void pass_on64(const Grid& G, const Fields& uin, cons
 // qin (optional): the primitive copy of uin; the halo is then read (or
 // staged, tin then describing qin) from it and only the temperature is
 // computed.  qout (optional): receives the primitives of uout (update64).
-template <int PLANE, bool WACT, class TL, bool P2>
+template <int PLANE, bool WACT, class TL>
 __device__ __forceinline__ void stage_segment64(const Grid& G, const Fields& uin, const Fields& u0,
                                                 const Fields& uout, StepCtrl* ctrl, int rs, int kind, double dt,
                                                 int x0, int ya, int yb, double* smem, const Fields* hout,
@@ -767,7 +768,7 @@ __device__ __forceinline__ void stage_segment64(const Grid& G, const Fields& uin
   using SM = TileSmem<double, NV, TL>;
   const SM S{smem};
   const int tid = threadIdx.x;
-  const Consts64 K{G.gamma, G.gm1, G.inv_gm1};
+  const Consts64 K{G.gamma, G.inv_gm1};
   const bool vsh = WACT && G.visc;
   int base = 0;
   for (int y0 = ya; y0 < yb; y0 += TY) {
@@ -797,7 +798,7 @@ __device__ __forceinline__ void stage_segment64(const Grid& G, const Fields& uin
     __syncthreads();
     faces64<PLANE, WACT, TL, WACT>(G, K, V, rs, nr, first ? 0 : 1, tid);
     __syncthreads();
-    update64<PLANE, WACT, TL, P2, WACT>(G, V, uin, u0, uout, ctrl, kind, dt, x0, y0, nr, tid, hout, red, qout);
+    update64<PLANE, WACT, TL, WACT>(G, V, uin, u0, uout, ctrl, kind, dt, x0, y0, nr, tid, hout, red, qout);
     __syncthreads();
     base += TY;
     if (base >= HY) base -= HY;
@@ -811,7 +812,7 @@ __device__ __forceinline__ void stage_segment64(const Grid& G, const Fields& uin
 // once, which balances the FP64 work per SM whatever the grid shape.
 // qin / qout: the primitive copy of the state read in place of uin's
 // conversion (when ctrl->q_valid) / written by the last stage of a step.
-template <int PLANE, bool WACT, class TL, bool P2>
+template <int PLANE, bool WACT, class TL>
 __device__ __forceinline__ void stage_strip64(const Grid& G, const Fields& uin, const Fields& u0, const Fields& uout,
                                               StepCtrl* ctrl, int rs, int kind, long long u0_, long long u1_,
                                               double* smem, unsigned long long* s_red, const Fields* hout,
@@ -834,7 +835,7 @@ __device__ __forceinline__ void stage_strip64(const Grid& G, const Fields& uin, 
       if (kind == STAGE_EULER) pass_on64<WACT, TX>(G, uin, uout, x0, ya, yb, tid);
       continue;
     }
-    stage_segment64<PLANE, WACT, TL, P2>(G, uin, u0, uout, ctrl, rs, kind, dt, x0, ya, yb, smem, hout, red, tin,
+    stage_segment64<PLANE, WACT, TL>(G, uin, u0, uout, ctrl, rs, kind, dt, x0, ya, yb, smem, hout, red, tin,
                                          mbar, &phase, qin, qout);
   }
   if (active && kind != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[parity ^ 1], s_red);
