@@ -230,6 +230,14 @@ static __device__ __noinline__ double minmod_rare(double dL, double dR) {
   return fabs(dL) < fabs(dR) ? dL : dR;
 }
 
+// Bits of x without the sign, shifted up by one: they order like |x|.  (A
+// mask in place of the shift is recognised as an absolute value and issued as
+// a DADD.)
+__device__ __forceinline__ unsigned long long abs_key(double x) {
+  return (unsigned long long)__double_as_longlong(x) << 1;
+}
+constexpr unsigned long long kInfKey = 0xffe0000000000000ull;
+
 // minmod of Update.h:73-80 -- 0 if dL*dR < 0, else the argument of smaller
 // magnitude, ties to dR -- decided on the bit patterns without FP64
 // instructions.  The sign test equals `dL*dR < 0` whenever the product cannot
@@ -238,16 +246,20 @@ static __device__ __noinline__ double minmod_rare(double dL, double dR) {
 // like their bit patterns.  The remaining cases take the reference formula.
 __device__ __forceinline__ X64 minmod_exact(X64 xL, X64 xR) {
   const double dL = xL.v, dR = xR.v;
-  const unsigned long long a = (unsigned long long)__double_as_longlong(dL);
-  const unsigned long long b = (unsigned long long)__double_as_longlong(dR);
-  const unsigned long long ma = a & 0x7fffffffffffffffull, mb = b & 0x7fffffffffffffffull;
-  const unsigned long long kInf = 0x7ff0000000000000ull;
-  if (ma <= kInf && mb <= kInf) {
-    if (ma == 0ull || mb == 0ull || ((a ^ b) >> 63) == 0ull) return ma < mb ? dL : dR;
-    const unsigned ea = (unsigned)(ma >> 52), eb = (unsigned)(mb >> 52);
+  const unsigned long long ma = abs_key(dL), mb = abs_key(dR);
+  if (ma <= kInfKey && mb <= kInfKey) {
+    const bool opposite = (__double2hiint(dL) ^ __double2hiint(dR)) < 0;
+    if (!opposite || ma == 0ull || mb == 0ull) return ma < mb ? dL : dR;
+    const unsigned ea = (unsigned)(ma >> 53), eb = (unsigned)(mb >> 53);
     if (ea != 0u && eb != 0u && ea + eb >= 972u) return 0.0;  // |dL*dR| >= 2^-1074
   }
   return minmod_rare(dL, dR);
+}
+
+// x with its sign flipped when f (integer: a negation selected by a flag is
+// issued as a DADD).
+__device__ __forceinline__ X64 flip_sign(X64 x, bool f) {
+  return __hiloint2double(__double2hiint(x.v) ^ (f ? (int)0x80000000 : 0), __double2loint(x.v));
 }
 
 // Comparisons and C99 fmin / fmax on bit patterns (integer pipe; the FP64
@@ -257,7 +269,7 @@ __device__ __forceinline__ X64 minmod_exact(X64 xL, X64 xR) {
 // may differ, which none of the callers can observe (their results do not
 // depend on the sign of a zero speed or of a zero compared with zero).  A
 // NaN operand is handled as fmin / fmax and the IEEE comparisons do.
-__device__ __forceinline__ bool is_nan_bits(long long b) { return (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL; }
+__device__ __forceinline__ bool is_nan_bits(long long b) { return ((unsigned long long)b << 1) > kInfKey; }
 
 // Signed-integer key that orders like the double (negative values reversed).
 __device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }

@@ -152,9 +152,9 @@ __device__ __forceinline__ void load_layer(const Grid& G, const Fields& u, const
     if (!c91) {
       Div64 D;
       load_prim(u, qsrc, zoff + col, G.gm1, q, D, G.tc != 0);
-      if (fa) q[1] = -q[1];
-      if (fb) q[2] = -q[2];
-      if (fz) q[3] = -q[3];
+      q[1] = flip_sign(q[1], fa);
+      q[2] = flip_sign(q[2], fb);
+      q[3] = flip_sign(q[3], fz);
       if (G.tc) T = quot(q[4], D);
     } else {
       c91_ghost(G, u, qsrc, col, fa, fb, kg, q);
@@ -530,8 +530,8 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
           for (int v = 0; v < 5; ++v) vf[d][v] = 0.0;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          vf[0][v + 1] = plus_zero(-X64(S.fa(v, cy, cx))) + S.fa(v, cy, cx + 1);
-          vf[1][v + 1] = plus_zero(-X64(S.fb(v, cy, cx))) + S.fb(v, cy + 1, cx);
+          vf[0][v + 1] = plus_zero(negated(X64(S.fa(v, cy, cx)))) + S.fa(v, cy, cx + 1);
+          vf[1][v + 1] = plus_zero(negated(X64(S.fb(v, cy, cx)))) + S.fb(v, cy + 1, cx);
         }
         viscous_iz3d(RingVel{S, k, cy + 2, cx + 2}, G.inv_dx, G.inv_dz, G.mu, vf[2]);
 #pragma unroll

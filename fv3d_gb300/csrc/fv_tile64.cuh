@@ -309,6 +309,8 @@ __device__ __forceinline__ X64 plus_zero(X64 x) {
 __device__ __forceinline__ double stored(X64 x) { return x.v; }
 __device__ __forceinline__ float stored(float x) { return x; }
 __device__ __forceinline__ float plus_zero(float x) { return 0.0f + x; }
+__device__ __forceinline__ X64 negated(X64 x) { return flip_sign(x, true); }
+__device__ __forceinline__ float negated(float x) { return -x; }
 
 // viscous_plane with the face-only branches taken from shared face fluxes:
 // gl[d] / gr[d] are viscous_face of the cell's lower / upper face along
@@ -324,10 +326,10 @@ __device__ __forceinline__ void viscous_plane_shared(const PA& P, const T gl[2][
 #pragma unroll
     for (int v = 0; v < 5; ++v) vf[d][v] = T(0);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) vf[0][k + 1] = plus_zero(-gl[0][k]) + gr[0][k];
+  for (int k = 0; k < 4; ++k) vf[0][k + 1] = plus_zero(negated(gl[0][k])) + gr[0][k];
   if (PLANE == PLANE_XY) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) vf[1][k + 1] = plus_zero(-gl[1][k]) + gr[1][k];
+    for (int k = 0; k < 4; ++k) vf[1][k + 1] = plus_zero(negated(gl[1][k])) + gr[1][k];
     viscous_iz_xy(P, odx, odz, mu, vf[2]);
   } else {
     viscous_iz_xz(P, odx, odz, mu, vf[2]);
@@ -514,8 +516,8 @@ __device__ __forceinline__ void load_prims64(const Grid& G, const Fields& uin, c
     } else {
       cons_to_prim64<PLANE, WACT>(u, G.gm1, q, D);
     }
-    if (fa) q[1] = -q[1];
-    if (fb) q[2] = -q[2];
+    q[1] = flip_sign(q[1], fa);
+    q[2] = flip_sign(q[2], fb);
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       if (WACT || v != 3) V.q(v, hy, hx) = q[v].v;
