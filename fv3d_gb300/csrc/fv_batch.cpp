@@ -226,8 +226,8 @@ std::string GroupKey(const fv_batch* b, const Group& g) {
     cells += (long long)s.first * s.second;
   }
   std::ostringstream k;
-  // the FP32-mixed 2-D groups' kernels (marched by warps) have a key of their own
-  k << "p" << b->precision << (b->precision != FV_PREC_FP64 && g.ndim == 2 ? "m" : "") << "_d" << g.ndim << "_co" << (g.rs >= 2) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
+  // k2: the generation of the stage kernels; a choice tuned on others is not taken over
+  k << "p" << b->precision << "k2_d" << g.ndim << "_co" << (g.rs >= 2) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
     << rs_mask << "_ts" << b->ts << "_n" << g.members.size() << "_c" << cells << "_h" << std::hex << h;
   return k.str();
 }

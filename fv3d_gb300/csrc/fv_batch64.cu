@@ -76,16 +76,17 @@ batch_stage64(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsign
     // the primitive copy: read by stage 1 while valid, written by stage 2
     const Fields* qi = kind == STAGE_RK_1 && I.Q.f[0] && ctrl->q_valid ? &I.Q : nullptr;
     const Fields* qo = kind == STAGE_RK_2 && I.Q.f[0] ? &I.Q : nullptr;
-    const int x0 = bx * TL::TX, ya = by * I.tz;  // tz: rows per work item
+    const int x0 = bx * TL::TX, w = min(TL::TX, I.G.na - x0);
+    const int ya = by * I.tz;  // tz: rows per work item
     const int yb = ya + I.tz < I.G.nb ? ya + I.tz : I.G.nb;
     if (!ctrl->active) {
-      if (kind == STAGE_EULER) pass_on64<WACT, TL::TX>(I.G, uin, uout, x0, ya, yb, threadIdx.x);
+      if (kind == STAGE_EULER) pass_on64<WACT>(I.G, uin, uout, x0, w, ya, yb, threadIdx.x);
       continue;
     }
     unsigned long long red = 0ull;
     cell_div_init(I.G);
     __syncthreads();
-    stage_segment64<PLANE, WACT, TL>(I.G, uin, u0, uout, ctrl, I.rs, kind, ctrl->dt_cur, x0, ya, yb, smem_raw, nullptr,
+    stage_segment64<PLANE, WACT, TL>(I.G, uin, u0, uout, ctrl, I.rs, kind, ctrl->dt_cur, x0, w, ya, yb, smem_raw, nullptr,
                                      red, nullptr, nullptr, nullptr, qi, qo);
     if (kind != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[ctrl->parity ^ 1], s_red);
     // the copy is complete once this launch is (the next reader is a later kernel)

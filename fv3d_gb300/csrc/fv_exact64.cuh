@@ -93,8 +93,10 @@ __device__ __forceinline__ X64 four_thirds_of<X64>() { return s_op64.four_thirds
 // Ziv, "Fast evaluation of elementary mathematical functions with correctly
 // rounded last bit", ACM TOMS 17(3), 1991): r y in units in the last place of
 // Q, computed in FP32 (error below 2^-13), must lie at least 2^-12 away from
-// every half.  Where it does not (one result in 2,048), and for operands
-// outside 2^-256 .. 2^256, the IEEE operation itself is called.  A result
+// every half.  Where it does not (one result in 2,048), and for operands so
+// small or large that a step could leave the normal range (divisors outside
+// 2^-150 .. 2^150, numerators outside 2^-750 .. 2^800, roots outside 2^-700 ..
+// 2^700), the IEEE operation itself is called.  A result
 // beside a power of two, where the spacing changes, is taken only if r is
 // zero (an exact quotient).
 static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
@@ -119,7 +121,7 @@ struct Div64 {
   double b, y;  // the divisor, 1/b to 2^-24
   float h, l;   // its significand (split_significand; l scaled by 2^-23)
   float r;      // 1/(h + l) to 2^-24
-  bool ok;      // 2^-256 <= |b| < 2^256
+  bool ok;      // 2^-150 <= |b| < 2^150
 };
 
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -133,7 +135,7 @@ __device__ __forceinline__ Div64 prepare_div(X64 b) {
   D.b = b.v;
   const unsigned hi = (unsigned)__double2hiint(b.v), lo = (unsigned)__double2loint(b.v);
   const unsigned e = hi & 0x7ff00000u;
-  D.ok = e - (767u << 20) < (512u << 20);
+  D.ok = e - (873u << 20) < (300u << 20);
   split_significand(hi, lo, 127u, D.h, D.l);
   D.l *= 0x1p-23f;
   const float r0 = rcp_approx(D.h);
@@ -144,13 +146,9 @@ __device__ __forceinline__ Div64 prepare_div(X64 b) {
   return D;
 }
 
-// Out of line, as the square root: inlined into every face and cell these two
-// made a translation unit take minutes to compile, and the call costs only
-// instruction issue, of which there is plenty.
-static __device__ __noinline__ double quot_call(double a_, double b_, double y_, float h_, float l_, float r_, bool ok_) {
-  const X64 a = a_;
-  const Div64 D{b_, y_, h_, l_, r_, ok_};
-  const unsigned ahi = (unsigned)__double2hiint(a.v), alo = (unsigned)__double2loint(a.v);
+// RN(a / D.b) where `good`; else the caller takes the IEEE operation.
+__device__ __forceinline__ double quot_core(double a, const Div64& D, bool& good) {
+  const unsigned ahi = (unsigned)__double2hiint(a), alo = (unsigned)__double2loint(a);
   const unsigned bhi = (unsigned)__double2hiint(D.b);
   const unsigned ea = ahi & 0x7ff00000u, eb = bhi & 0x7ff00000u;
   float ah, al;
@@ -165,30 +163,78 @@ static __device__ __noinline__ double quot_call(double a_, double b_, double y_,
                       ((long long)n << 3);
   const unsigned sign = (ahi ^ bhi) & 0x80000000u;
   const double Q = __longlong_as_double(q ^ ((long long)sign << 32));
-  const double res = fma(-D.b, Q, a.v);
-  double out = fma(res, D.y, Q);
+  const double res = fma(-D.b, Q, a);
+  const double out = fma(res, D.y, Q);
   // the rounding test
   const unsigned rhi = (unsigned)__double2hiint(res) & 0x7fffffffu, rlo = (unsigned)__double2loint(res);
   const int x = (int)(rhi - ea + ((127u + 52u) << 20));
   float t = __fmul_rn(x > 0 ? __uint_as_float(__funnelshift_l(rlo, (unsigned)x, 3)) : 0.0f, D.r);
   t = big ? t : t + t;
   const bool edge = ((qb + 1u) & 0x007fffffu) <= 1u && (rhi | rlo) != 0u;
-  const bool good = D.ok && ea - (767u << 20) < (512u << 20) && x < (int)((127u + 12u) << 20) && clear_of_half(t) &&
-                    !edge;
-  if (((ahi << 1) | alo) == 0u && D.ok) return __hiloint2double((int)sign, 0);  // 0 / b
-  if (!good) out = div_ieee(a.v, D.b);
-  return out;
+  const bool zero = ((ahi << 1) | alo) == 0u;  // 0 / b
+  good = D.ok && (zero || (ea - (273u << 20) < (1550u << 20) && x < (int)((127u + 12u) << 20) && clear_of_half(t) &&
+                           !edge));
+  return zero ? __hiloint2double((int)sign, 0) : out;
 }
 
-// RN(a / D.b).
-__device__ __forceinline__ X64 quot(X64 a, const Div64& D) { return quot_call(a.v, D.b, D.y, D.h, D.l, D.r, D.ok); }
+// Out of line, as the square roots: inlined into every face and cell these
+// made a translation unit take minutes to compile, and a call costs only
+// instruction issue, of which there is plenty.  One call takes as many
+// quotients as the code has at hand: they overlap in it (a quotient alone
+// takes 356 cycles from operands to result), calls do not.
+template <int N>
+struct Vals {
+  double v[N];
+};
+template <int N>
+static __device__ __noinline__ Vals<N> quots_call(Vals<N> a, Div64 D) {
+  Vals<N> q;
+  bool good[N], all = true;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    q.v[i] = quot_core(a.v[i], D, good[i]);
+    all = all && good[i];
+  }
+  if (!all) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (!good[i]) q.v[i] = div_ieee(a.v[i], D.b);
+  }
+  return q;
+}
+static __device__ __noinline__ Vals<2> quot_pair_call(double a, Div64 A, double b, Div64 B) {
+  Vals<2> q;
+  bool ga, gb;
+  q.v[0] = quot_core(a, A, ga);
+  q.v[1] = quot_core(b, B, gb);
+  if (!ga) q.v[0] = div_ieee(a, A.b);
+  if (!gb) q.v[1] = div_ieee(b, B.b);
+  return q;
+}
+
+// RN(a / D.b); of several numerators, in place; of two with a divisor each.
+__device__ __forceinline__ X64 quot(X64 a, const Div64& D) { return quots_call<1>(Vals<1>{{a.v}}, D).v[0]; }
+template <int N>
+__device__ __forceinline__ void quots(X64 (&a)[N], const Div64& D) {
+  Vals<N> x;
+#pragma unroll
+  for (int i = 0; i < N; ++i) x.v[i] = a[i].v;
+  x = quots_call<N>(x, D);
+#pragma unroll
+  for (int i = 0; i < N; ++i) a[i] = x.v[i];
+}
+__device__ __forceinline__ void quot_pair(X64& a, const Div64& A, X64& b, const Div64& B) {
+  const Vals<2> q = quot_pair_call(a.v, A, b.v, B);
+  a = q.v[0];
+  b = q.v[1];
+}
 
 // RN(a / b) for a divisor used once.
 __device__ __forceinline__ X64 div64(X64 a, X64 b) { return quot(a, prepare_div(b)); }
 
-static __device__ __noinline__ double sqrt_call(double x_) {
-  const X64 x = x_;
-  const unsigned hi = (unsigned)__double2hiint(x.v), lo = (unsigned)__double2loint(x.v);
+// RN(sqrt(x)) where `good`.
+__device__ __forceinline__ double sqrt_core(double x, bool& good) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const int e = (int)(hi >> 20) - 1023;
   const int odd = e & 1, half_e = (e - odd) >> 1;
   float mh, ml;  // x = (mh + ml) 4^half_e, mh in [1, 4)
@@ -207,20 +253,39 @@ static __device__ __noinline__ double sqrt_call(double x_) {
                        (long long)(gb << 29)) + ((long long)n << 3);
   const double G = __longlong_as_double(g);
   const double H = __hiloint2double((int)((hb >> 3) + (896u << 20) - ((unsigned)half_e << 20)), (int)(hb << 29));
-  const double res = fma(-G, G, x.v);
-  double out = fma(res, H, G);
+  const double res = fma(-G, G, x);
+  const double out = fma(res, H, G);
   const unsigned rhi = (unsigned)__double2hiint(res) & 0x7fffffffu, rlo = (unsigned)__double2loint(res);
   const int s = (int)(rhi - ((unsigned)(2 * half_e + 1023) << 20) + ((127u + 52u) << 20));
   const float t = __fmul_rn(s > 0 ? __uint_as_float(__funnelshift_l(rlo, (unsigned)s, 3)) : 0.0f, h);
   const bool inside = gb - 0x3f800001u < 0x007ffffeu;  // 1 < g0 < 2, not beside either
-  const bool good = hi - (767u << 20) < (512u << 20) && s < (int)((127u + 12u) << 20) && clear_of_half(t) &&
+  good = hi - (323u << 20) < (1400u << 20) && s < (int)((127u + 12u) << 20) && clear_of_half(t) &&
                     (inside || (rhi | rlo) == 0u);
-  if (!good) out = sqrt_ieee(x.v);
   return out;
+}
+
+static __device__ __noinline__ double sqrt_call(double x) {
+  bool good;
+  const double s = sqrt_core(x, good);
+  return good ? s : sqrt_ieee(x);
+}
+static __device__ __noinline__ Vals<2> sqrt_pair_call(double a, double b) {
+  Vals<2> s;
+  bool ga, gb;
+  s.v[0] = sqrt_core(a, ga);
+  s.v[1] = sqrt_core(b, gb);
+  if (!ga) s.v[0] = sqrt_ieee(a);
+  if (!gb) s.v[1] = sqrt_ieee(b);
+  return s;
 }
 
 // RN(sqrt(x)).
 __device__ __forceinline__ X64 sqrt64(X64 x) { return sqrt_call(x.v); }
+__device__ __forceinline__ void sqrt_pair(X64& a, X64& b) {
+  const Vals<2> s = sqrt_pair_call(a.v, b.v);
+  a = s.v[0];
+  b = s.v[1];
+}
 
 // The reference formula of minmod, out of line: the rare operands that reach
 // it (NaN, infinities, a product that may underflow) take a real branch, so

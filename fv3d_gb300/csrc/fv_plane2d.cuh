@@ -42,6 +42,32 @@ __device__ __forceinline__ X64 div_cell(X64 x, int axis) {
   return quot(x, s_cell64.d[axis]);
 }
 
+// x[v] / d of several values, in place.
+template <int N>
+__device__ __forceinline__ void div_cells(X64 (&x)[N], int axis) {
+  if (s_cell64.pow2) {
+#pragma unroll
+    for (int v = 0; v < N; ++v) x[v] = x[v] * s_cell64.inv[axis];
+  } else {
+    quots(x, s_cell64.d[axis]);
+  }
+}
+
+// u[v] += x[v] / d for the cell size of an axis and N values: with powers of
+// two one fused operation each (the product is exact, so it rounds as the
+// quotient and the sum do).
+template <int N>
+__device__ __forceinline__ void add_div_cell(X64 (&u)[N], X64 (&x)[N], int axis) {
+  if (s_cell64.pow2) {
+#pragma unroll
+    for (int v = 0; v < N; ++v) u[v] = fma(x[v].v, s_cell64.inv[axis], u[v].v);
+  } else {
+    quots(x, s_cell64.d[axis]);
+#pragma unroll
+    for (int v = 0; v < N; ++v) u[v] = u[v] + x[v];
+  }
+}
+
 // Storage slot (1 = a, 2 = b, 3 = c) of the reference's physical velocity
 // component var (1 = x, 2 = y, 3 = z).
 template <int PLANE>
@@ -58,9 +84,10 @@ template <int PLANE, bool WACT>
 __device__ __forceinline__ void cons_to_prim64(const X64 u[5], X64 gm1, X64 q[5], Div64& D) {
   const X64 r = u[0];
   D = prepare_div(r);
-  const X64 va = quot(u[1], D);
-  const X64 vb = quot(u[2], D);
-  const X64 vc = WACT ? quot(u[3], D) : X64(0.0);
+  X64 m[WACT ? 3 : 2] = {u[1], u[2]};
+  if (WACT) m[2] = u[3];
+  quots(m, D);
+  const X64 va = m[0], vb = m[1], vc = WACT ? m[2] : X64(0.0);
   X64 ke;
   if (WACT) {
     const X64 vx = va, vy = PLANE == PLANE_XY ? vb : vc, vz = PLANE == PLANE_XY ? vc : vb;
@@ -90,10 +117,11 @@ __device__ __forceinline__ X64 inv_dt_hyp64(const X64 u[5], const Grid& G, X64* 
   }
   const X64 cs = sqrt64(quot(q[4] * G.gamma, D));
   const X64 vx = q[1], vy = PLANE == PLANE_XY ? q[2] : q[3], vz = PLANE == PLANE_XY ? q[3] : q[2];
-  const X64 tx = div_cell(cs + fabs(vx.v), 0);
-  const X64 ty = div_cell(cs + fabs(vy.v), 1);
-  const X64 tz = div_cell(cs + fabs(vz.v), 2);
-  return tx + ty + tz;
+  X64 tx = cs + fabs(vx.v), ty = cs + fabs(vy.v), tz = cs + fabs(vz.v);
+  if (s_cell64.pow2)  // exact products: each fused operation rounds as quotient and sum do
+    return fma(tz.v, s_cell64.inv[2], fma(ty.v, s_cell64.inv[1], (tx * s_cell64.inv[0]).v));
+  quot_pair(tx, s_cell64.d[0], ty, s_cell64.d[1]);
+  return tx + ty + quot(tz, s_cell64.d[2]);
 }
 
 // Block-wide max of non-negative doubles held as bit patterns (IEEE order of

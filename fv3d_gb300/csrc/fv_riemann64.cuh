@@ -41,15 +41,15 @@ __device__ __forceinline__ void euler_flux64(const Slots<X64>& q, X64 e, X64 F[5
   F[4] = (q.p + E) * q.un;
 }
 
-// primToCons (States.h:20-31) given e = p/(gamma-1) and the prepared density.
+// primToCons (States.h:20-31) without the internal energy: u[4] = the sum of
+// the squared momenta / 2, still to be divided by the density.
 template <int ZS>
-__device__ __forceinline__ void prim_to_cons64(const Slots<X64>& q, X64 e, const Div64& rho, X64 u[5]) {
+__device__ __forceinline__ void prim_to_cons64(const Slots<X64>& q, X64 u[5]) {
   u[0] = q.r;
   u[1] = q.r * q.un;
-  u[2] = ZS == 1 ? 0.0 : q.r * q.t1;
-  u[3] = ZS == 2 ? 0.0 : q.r * q.t2;
-  const X64 Ek = quot(half_of(ke_sum3<ZS>(u[1], u[2], u[3])), rho);
-  u[4] = Ek + e;
+  u[2] = ZS == 1 ? X64(0.0) : q.r * q.t1;
+  u[3] = ZS == 2 ? X64(0.0) : q.r * q.t2;
+  u[4] = half_of(ke_sum3<ZS>(u[1], u[2], u[3]));
 }
 
 // HLL with Davis wave speeds, RiemannSolvers.h:6-36.
@@ -61,12 +61,14 @@ __device__ __forceinline__ void hll64(const Slots<X64>& L, const Slots<X64>& R, 
   // each density, prepared once, divides twice (the sound speed's p*gamma and,
   // in the star region, the kinetic energy)
   const Div64 rhoL = prepare_div(L.r), rhoR = prepare_div(R.r);
-  const X64 aL = sqrt64(quot(L.p * K.gamma, rhoL));
-  const X64 aR = sqrt64(quot(R.p * K.gamma, rhoR));
+  X64 aL = L.p * K.gamma, aR = R.p * K.gamma;
+  quot_pair(aL, rhoL, aR, rhoR);
+  sqrt_pair(aL, aR);
   const X64 SL = fmin_bits(L.un - aL, R.un - aR);
   const X64 SR = fmax_bits(L.un + aL, R.un + aR);
-  const X64 eL = quot(L.p, s_cell64.gm1);
-  const X64 eR = quot(R.p, s_cell64.gm1);
+  X64 e[2] = {L.p, R.p};
+  quots(e, s_cell64.gm1);
+  const X64 eL = e[0], eR = e[1];
   X64 FL[5], FR[5];
   euler_flux64<ZS>(L, eL, FL);
   euler_flux64<ZS>(R, eR, FR);
@@ -81,18 +83,25 @@ __device__ __forceinline__ void hll64(const Slots<X64>& L, const Slots<X64>& R, 
   } else {
     if (pout) *pout = half_of(L.p + R.p);
     X64 uL[5], uR[5];
-    prim_to_cons64<ZS>(L, eL, rhoL, uL);
-    prim_to_cons64<ZS>(R, eR, rhoR, uR);
+    prim_to_cons64<ZS>(L, uL);
+    prim_to_cons64<ZS>(R, uR);
+    quot_pair(uL[4], rhoL, uR[4], rhoR);
+    uL[4] = uL[4] + eL;
+    uR[4] = uR[4] + eR;
     const X64 slsr = SL * SR;
     const Div64 den = prepare_div(SR - SL);
+    constexpr int N = ZS ? 4 : 5;
+    X64 f[N];
+    int n = 0;
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      if ((ZS == 1 && v == 2) || (ZS == 2 && v == 3)) {
-        flux[v] = 0.0;
-        continue;
-      }
-      flux[v] = quot((FL[v] * SR - FR[v] * SL) + (uR[v] - uL[v]) * slsr, den);
+      if ((ZS == 1 && v == 2) || (ZS == 2 && v == 3)) continue;
+      f[n++] = (FL[v] * SR - FR[v] * SL) + (uR[v] - uL[v]) * slsr;
     }
+    quots(f, den);
+    n = 0;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) flux[v] = (ZS == 1 && v == 2) || (ZS == 2 && v == 3) ? X64(0.0) : f[n++];
   }
 }
 
@@ -109,16 +118,17 @@ __device__ __forceinline__ void hllc64(const Slots<X64>& L, const Slots<X64>& R,
   const X64 kR = KE3 ? ke_sum3<ZS>(uR, R.t1, R.t2) : (ZS == 1 ? uR * uR : uR * uR + R.t1 * R.t1);
   const X64 EL = half_of(rL) * kL + pL * K.inv_gm1;
   const X64 ER = half_of(rR) * kR + pR * K.inv_gm1;
-  const X64 c2L = div64(pL * K.gamma, rL);
-  const X64 c2R = div64(pR * K.gamma, rR);
+  X64 c2L = pL * K.gamma, c2R = pR * K.gamma;
+  quot_pair(c2L, prepare_div(rL), c2R, prepare_div(rR));
   const X64 cmax = sqrt64(fmax_bits(c2L, c2R));
   const X64 SL = fmin_bits(uL, uR) - cmax;
   const X64 SR = fmax_bits(uL, uR) + cmax;
   const X64 rcL = rL * (uL - SL);
   const X64 rcR = rR * (SR - uR);
   const Div64 D = prepare_div(rcR + rcL);
-  const X64 uS = quot(rcR * uR + rcL * uL + (pL - pR), D);
-  const X64 pS = quot(rcR * pL + rcL * pR + rcL * rcR * (uL - uR), D);
+  X64 s[2] = {rcR * uR + rcL * uL + (pL - pR), rcR * pL + rcL * pR + rcL * rcR * (uL - uR)};
+  quots(s, D);
+  const X64 uS = s[0], pS = s[1];
   X64 sr, su, st1, st2, sp, E;
   if (gt0_bits(SL)) {
     sr = rL; su = uL; st1 = L.t1; st2 = L.t2; sp = pL; E = EL;
@@ -129,8 +139,10 @@ __device__ __forceinline__ void hllc64(const Slots<X64>& L, const Slots<X64>& R,
     const X64 rK = left ? rL : rR, uK = left ? uL : uR, pK = left ? pL : pR, EK = left ? EL : ER;
     const X64 SK = left ? SL : SR;
     const Div64 den = prepare_div(SK - uS);
-    sr = quot(rK * (SK - uK), den);
-    E = quot((SK - uK) * EK - pK * uK + pS * uS, den);
+    X64 k[2] = {rK * (SK - uK), (SK - uK) * EK - pK * uK + pS * uS};
+    quots(k, den);
+    sr = k[0];
+    E = k[1];
     su = uS;
     sp = pS;
     st1 = left ? L.t1 : R.t1;

@@ -4,6 +4,8 @@
 // the reference).  The strip rows are split evenly over as many CTAs as the
 // GPU holds at once, so every SM gets the same FP64 work.
 #include "fv_tile64.cuh"
+#include <algorithm>
+#include <cmath>
 #include <cudaTypedefs.h>  // PFN_cuTensorMapEncodeTiled
 
 namespace fv {
@@ -11,10 +13,6 @@ namespace fv {
 namespace {
 
 using SingleTile = Tile<kTileX, kTileY>;
-#ifndef FV_STRIP_MIN_ROWS
-#define FV_STRIP_MIN_ROWS 4
-#endif
-constexpr int kMinRowsPerCta = FV_STRIP_MIN_ROWS;  // fewer CTAs than that many rows each on small grids
 
 // Dynamic shared memory is over-allocated by this much and aligned up, so
 // that tensor copies land on 128-byte boundaries.
@@ -23,7 +21,7 @@ constexpr size_t kSmemAlign = 128;
 template <int PLANE, int RS, int KIND, bool WACT>
 __global__ void __launch_bounds__(kTileThreads, WACT ? FV_FP64_MIN_CTAS_W : FV_FP64_MIN_CTAS)
 stage2d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u0, const Fields uout, StepCtrl* __restrict__ ctrl,
-             const Fields hout, long long units, const __grid_constant__ TmaState tin, int use_tma, const Fields qin,
+             const Fields hout, int width, long long units, const __grid_constant__ TmaState tin, int use_tma, const Fields qin,
              const Fields qout, const __grid_constant__ TmaState tq, int use_tq) {
   extern __shared__ __align__(128) unsigned char smem_bytes[];
   __shared__ unsigned long long s_red[kTileThreads / 32];
@@ -51,8 +49,8 @@ stage2d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u
   const TmaState* tp = prims ? (use_tq ? &tq : nullptr) : (use_tma ? &tin : nullptr);
   const Fields* ho = hout.f[0] ? &hout : nullptr;
   const long long ub = units * blockIdx.x / gridDim.x, ue = units * (blockIdx.x + 1) / gridDim.x;
-  stage_strip64<PLANE, WACT, SingleTile>(G, uin, u0, uout, ctrl, RS, KIND, ub, ue, smem, s_red, ho, tp, &s_mbar, qi,
-                                         qo);
+  stage_strip64<PLANE, WACT, SingleTile>(G, uin, u0, uout, ctrl, RS, KIND, width, ub, ue, smem, s_red, ho, tp,
+                                         &s_mbar, qi, qo);
   pdl_trigger();
 }
 
@@ -64,6 +62,55 @@ int sm_count() {
       n = 1;
   }
   return n;
+}
+
+// The split of a plane into strips of `width` columns whose rows (units) are
+// shared out evenly over `ctas` CTAs.
+struct Strips {
+  int width;
+  long long units, ctas;
+};
+
+// The width and CTA count with the least estimated time of the busiest SM.
+// Large grids take full strips on every CTA the GPU holds at once: the fewest
+// faces solved twice.  On small grids that left SMs idle (a 64^2 grid made 32
+// CTAs of 32 x 4 cells): narrower strips and fewer rows per CTA spread the
+// FP64 work, which bounds an SM, over all of them.  The estimate counts FP64
+// warp operations per phase (a warp with idle lanes costs a whole one) for the
+// faces, conversions and cell updates of a CTA and divides the SM's sum by the
+// share of the pipe its CTAs keep busy between their barriers: 60 % for one,
+// 95 % for two against three (1024^2: 1,330, 850 and 813 us a step).
+Strips split_strips(const Grid& G, int rs, bool wact, int resident) {
+  const int sms = sm_count();
+  const bool visc = wact && G.visc;
+  const double face = (rs == 0 ? 110 : 75) + (wact ? 12 : 0) + (visc ? 30 : 0);
+  const double cell = 55 + (G.tc ? 20 : 0) + (visc ? 40 : 0), conv = 8;
+  const double phase = 7000.0 / 16.0;  // latency of a block's phases, in FP64 warp operations
+  const double busy[3] = {0.60, 0.95, 1.0};
+  Strips best{};
+  double best_t = 0.0;
+  for (int w0 : {kTileX, 24, 16, 12, 8}) {
+    const int n_strips = (G.na + w0 - 1) / w0;
+    // strips of equal width; full ones where that saves none (they are staged by tensor copies)
+    int w = (G.na + n_strips - 1) / n_strips;
+    if (w0 == kTileX && G.na >= 8 * kTileX) w = kTileX;
+    const long long units = (long long)n_strips * G.nb;
+    for (int per_sm = 1; per_sm <= resident; ++per_sm) {
+      const long long ctas = std::min(units, (long long)per_sm * sms);
+      const long long rows = (units + ctas - 1) / ctas;  // of the busiest CTA
+      const double blocks = std::ceil((double)rows / kTileY);
+      auto warps = [](double lanes) { return std::ceil(lanes / 32.0); };
+      const double work = face * (warps((w + 1.0) * rows) + warps(w * (rows + 1.0))) + cell * warps((double)w * rows) +
+                          conv * warps((w + 4.0) * (rows + 4.0));
+      const long long on_sm = (ctas + sms - 1) / sms;
+      const double t = std::max(work * on_sm / busy[std::min(on_sm, 3LL) - 1], phase * blocks);
+      if (best.ctas == 0 || t < best_t * 0.995) {
+        best = Strips{w, units, ctas};
+        best_t = t;
+      }
+    }
+  }
+  return best;
 }
 
 template <int PLANE, int RS, int KIND, bool WACT>
@@ -86,15 +133,11 @@ cudaError_t launch_one(const Grid& G, Fields uin, Fields u0, Fields uout, StepCt
     if (e != cudaSuccess) return e;
     if (resident[cfg] < 1) resident[cfg] = 1;
   }
-  const long long units = (long long)((G.na + kTileX - 1) / kTileX) * G.nb;
-  long long ctas = units / kMinRowsPerCta;
-  const long long slots = (long long)resident[cfg] * sm_count();
-  if (ctas > slots) ctas = slots;
-  if (ctas < 1) ctas = 1;
+  const Strips p = split_strips(G, RS, WACT, resident[cfg]);
   const Fields none{};
   static const TmaState no_tma{};
-  const cudaError_t e = launch_pdl(kern, dim3((unsigned)ctas), dim3(kTileThreads), smem, st, G, uin, u0, uout, ctrl,
-                                   hout ? *hout : none, units, tin ? *tin : no_tma, tin ? 1 : 0,
+  const cudaError_t e = launch_pdl(kern, dim3((unsigned)p.ctas), dim3(kTileThreads), smem, st, G, uin, u0, uout, ctrl,
+                                   hout ? *hout : none, p.width, p.units, tin ? *tin : no_tma, tin ? 1 : 0,
                                    pc.qin ? *pc.qin : none, pc.qout ? *pc.qout : none, pc.tq ? *pc.tq : no_tma,
                                    pc.tq ? 1 : 0);
   return e != cudaSuccess ? e : cudaGetLastError();

@@ -419,12 +419,13 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
 #pragma unroll
       for (int v = 0; v < 5; ++v) un[v] = uin.f[v][o];
       // IX, IY: un += (F(-1/2) - F(+1/2)) * dt / d
+      X64 dF[5];
 #pragma unroll
-      for (int v = 0; v < 5; ++v)
-        un[v] = un[v] + div_cell((X64(S.fa(v, cy, cx)) - S.fa(v, cy, cx + 1)) * dt, 0);
+      for (int v = 0; v < 5; ++v) dF[v] = (X64(S.fa(v, cy, cx)) - S.fa(v, cy, cx + 1)) * dt;
+      add_div_cell(un, dF, 0);
 #pragma unroll
-      for (int v = 0; v < 5; ++v)
-        un[v] = un[v] + div_cell((X64(S.fb(v, cy, cx)) - S.fb(v, cy + 1, cx)) * dt, 1);
+      for (int v = 0; v < 5; ++v) dF[v] = (X64(S.fb(v, cy, cx)) - S.fb(v, cy + 1, cx)) * dt;
+      add_div_cell(un, dF, 1);
       // IZ with the z-boundary overrides of Update.h:131-143
       X64 fL[5], fR[5];
 #pragma unroll
@@ -451,7 +452,8 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
         }
       }
 #pragma unroll
-      for (int v = 0; v < 5; ++v) un[v] = un[v] + div_cell((fL[v] - fR[v]) * dt, 2);
+      for (int v = 0; v < 5; ++v) dF[v] = (fL[v] - fR[v]) * dt;
+      add_div_cell(un, dF, 2);
       if (G.gravity) {
         un[3] = un[3] + dt * rho_c * G.g;
         un[4] = un[4] + half_of(dt) * (fL[0] + fR[0]) * G.g;
@@ -469,12 +471,14 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
         }
         const int hy = cy + 2, hx = cx + 2;
         const X64 TC = S.temp(sk, hy, hx);
-        const X64 FL = div_cell(kC * (TC - S.temp(sk, hy, hx - 1)), 0);
-        const X64 FR = div_cell(kC * (X64(S.temp(sk, hy, hx + 1)) - TC), 0);
-        const X64 FU = div_cell(kC * (TC - S.temp(sk, hy - 1, hx)), 1);
-        const X64 FD = div_cell(kC * (X64(S.temp(sk, hy + 1, hx)) - TC), 1);
-        X64 FF = div_cell(kF * (TC - S.temp(slot_of(k - 1), hy, hx)), 2);
-        X64 FB = div_cell(kB * (X64(S.temp(slot_of(k + 1), hy, hx)) - TC), 2);
+        X64 fx[3] = {kC * (TC - S.temp(sk, hy, hx - 1)), kC * (X64(S.temp(sk, hy, hx + 1)) - TC), dt};
+        X64 fy[3] = {kC * (TC - S.temp(sk, hy - 1, hx)), kC * (X64(S.temp(sk, hy + 1, hx)) - TC), dt};
+        X64 fz[3] = {kF * (TC - S.temp(slot_of(k - 1), hy, hx)), kB * (X64(S.temp(slot_of(k + 1), hy, hx)) - TC), dt};
+        div_cells(fx, 0);
+        div_cells(fy, 1);
+        div_cells(fz, 2);
+        const X64 FL = fx[0], FR = fx[1], FU = fy[0], FD = fy[1], dtdx = fx[2], dtdy = fy[2], dtdz = fz[2];
+        X64 FF = fz[0], FB = fz[1];
         if (k == 0 && G.bctc_zmin != 0) {
           if (G.bctc_zmin == 1) FF = div_cell(kF * 2.0 * (TC - G.bctc_zmin_value), 2);
           else FF = kF * G.bctc_zmin_value;
@@ -483,9 +487,6 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
           if (G.bctc_zmax == 1) FB = div_cell(kB * 2.0 * (X64(G.bctc_zmax_value) - TC), 2);
           else FB = kB * G.bctc_zmax_value;
         }
-        const X64 dtdx = div_cell(dt, 0);
-        const X64 dtdy = div_cell(dt, 1);
-        const X64 dtdz = div_cell(dt, 2);
         un[4] = un[4] + (dtdx * (FR - FL) + dtdy * (FD - FU) + dtdz * (FB - FF));
       }
       if (G.visc && !vsh) {  // Viscosity.h:145-151

@@ -600,7 +600,7 @@ __device__ __forceinline__ void stage_segment32(const Grid& G, const MixedFields
     __syncthreads();
     faces32<PLANE, WACT, TL>(G, V, rs, nr, first ? 0 : 1, tid);
     if (VF && WACT && G.visc)
-      visc_faces<PLANE, TL, float>(V, G.inv_dx_f, G.inv_dy_f, G.inv_dz_f, G.mu_f, nr, first ? 0 : 1, tid);
+      visc_faces<PLANE, TL, float>(V, G.inv_dx_f, G.inv_dy_f, G.inv_dz_f, G.mu_f, TX, nr, first ? 0 : 1, tid);
     __syncthreads();
     update32<PLANE, WACT, TL, VF>(G, V, M, src, dst, kind, dt, x0, y0, nr, tid, red, bad);
     __syncthreads();

@@ -56,6 +56,16 @@ struct Tile {
   static constexpr int CELLS = TX * TY;
 };
 
+// Division of small indices by a strip's width, known only at run time: exact
+// for i < 2^12 and d <= 128: (i + 1/2) / d lies at least 1/256 off every integer,
+// far more than the rounding of the product.
+struct SmallDiv {
+  int d;
+  float r;
+  __device__ __forceinline__ explicit SmallDiv(int d_) : d(d_), r(1.0f / (float)d_) {}
+  __device__ __forceinline__ int quotient(int i) const { return (int)(((float)i + 0.5f) * r); }
+};
+
 // Shared-memory layout for NV stored variables of element type T:
 //   Q [NV][HY][HX]   primitives of tile + halo
 //   FA[NV][TY][TX+1] a-face fluxes (storage order)
@@ -336,27 +346,27 @@ __device__ __forceinline__ void viscous_plane_shared(const PA& P, const T gl[2][
   }
 }
 
-// Viscous fluxes of the face-only branches for the faces of a block: a
+// Viscous fluxes of the face-only branches for the faces of a block of w columns: a
 // faces of cell rows 0..nr-1 along IX; b faces of face rows fb0..nr along IY
 // in the x-y plane (the x-z plane's IZ branch belongs to the cells).
 template <int PLANE, class TL, class T, class PV>
-__device__ __forceinline__ void visc_faces(const PV& V, T odx, T ody, T odz, T mu, int nr, int fb0, int tid) {
-  constexpr int TX = TL::TX;
-  const int nfa = (TX + 1) * nr;
+__device__ __forceinline__ void visc_faces(const PV& V, T odx, T ody, T odz, T mu, int w, int nr, int fb0, int tid) {
+  const SmallDiv by_wa(w + 1), by_w(w);
+  const int nfa = (w + 1) * nr;
   const int nfa_pad = (nfa + 31) & ~31;
-  const int n = nfa_pad + (PLANE == PLANE_XY ? TX * (nr + 1 - fb0) : 0);
+  const int n = nfa_pad + (PLANE == PLANE_XY ? w * (nr + 1 - fb0) : 0);
   for (int it = tid; it < n; it += kTileThreads) {
     T g[4];
     if (it < nfa_pad) {
       if (it >= nfa) continue;
-      const int fy = it / (TX + 1), fx = it - fy * (TX + 1);
+      const int fy = by_wa.quotient(it), fx = it - fy * (w + 1);
       const PlaneVel<PLANE, PV, T> P{V, fy + 2, fx + 2};  // the cell right of a face
       viscous_face<PLANE, 0, T>(P, odx, ody, odz, mu, g);
 #pragma unroll
       for (int k = 0; k < 4; ++k) V.va(k, fy, fx) = stored(g[k]);
     } else {
       const int j = it - nfa_pad;
-      const int jy = j / TX, fx = j - jy * TX;
+      const int jy = by_w.quotient(j), fx = j - jy * w;
       const int fy = fb0 + jy;
       const PlaneVel<PLANE, PV, T> P{V, fy + 2, fx + 2};  // the cell above b face fy
       viscous_face<PLANE, 1, T>(P, odx, ody, odz, mu, g);
@@ -483,7 +493,7 @@ struct PrimView {
 };
 
 // Phase 1: halo rows [h0, h1) of the block whose first cell is (x0, y0),
-// columns x0-2 .. x0+TX+1: conserved state -> primitives (and temperature),
+// columns x0-2 .. x0+w+1: conserved state -> primitives (and temperature),
 // ghost cells synthesised by index remapping (X-then-Y fill of
 // BoundaryConditions.h:146-192, corners included).
 //
@@ -492,11 +502,11 @@ struct PrimView {
 // temperature's reciprocal is computed.
 template <int PLANE, bool WACT, class TL, class PV>
 __device__ __forceinline__ void load_prims64(const Grid& G, const Fields& uin, const PV& V, int x0, int y0, int h0,
-                                             int h1, int tid, bool prims = false) {
-  constexpr int HX = TL::HX;
-  const int n = (h1 - h0) * HX;
+                                             int h1, int w, int tid, bool prims = false) {
+  const SmallDiv by_hx(w + 4);
+  const int n = (h1 - h0) * (w + 4);
   for (int idx = tid; idx < n; idx += kTileThreads) {
-    const int r = idx / HX, hx = idx - r * HX;
+    const int r = by_hx.quotient(idx), hx = idx - r * (w + 4);
     const int hy = h0 + r;
     bool fa, fb;
     const int sa = bc_source(x0 + hx - 2, G.na, G.bc_a, fa);
@@ -591,19 +601,19 @@ __device__ __forceinline__ bool stage_rows_tma(const TmaState* tin, const PV& V,
 // the block (b face row fy lies between cell rows fy-1 and fy), each solved
 // once; with VSH, their viscous fluxes too.
 template <int PLANE, bool WACT, class TL, bool VSH, class PV>
-__device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const PV& V, int rs, int nr, int fb0,
-                                        int tid) {
-  constexpr int TX = TL::TX;
+__device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const PV& V, int rs, int w, int nr,
+                                        int fb0, int tid) {
+  const SmallDiv by_wa(w + 1), by_w(w);
   const bool plm = G.recon == R_PLM;
   const bool wb_z = PLANE == PLANE_XZ && G.recon == R_PCM_WB;
-  const int nfa = (TX + 1) * nr;
+  const int nfa = (w + 1) * nr;
   const int nfa_pad = (nfa + 31) & ~31;  // keeps each warp on one face kind
-  const int n = nfa_pad + TX * (nr + 1 - fb0);
+  const int n = nfa_pad + w * (nr + 1 - fb0);
   for (int it = tid; it < n; it += kTileThreads) {
     X64 c[4][5], f[5];
     if (it < nfa_pad) {
       if (it >= nfa) continue;
-      const int fy = it / (TX + 1), fx = it - fy * (TX + 1);
+      const int fy = by_wa.quotient(it), fx = it - fy * (w + 1);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
 #pragma unroll
@@ -614,7 +624,7 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
         if (WACT || v != 3) V.fa(v, fy, fx) = f[v].v;
     } else {
       const int j = it - nfa_pad;
-      const int jy = j / TX, fx = j - jy * TX;
+      const int jy = by_w.quotient(j), fx = j - jy * w;
       const int fy = fb0 + jy;
 #pragma unroll
       for (int k = 0; k < 4; ++k)
@@ -626,7 +636,7 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
         if (WACT || v != 3) V.fb(v, fy, fx) = f[v].v;
     }
   }
-  if (VSH && WACT && G.visc) visc_faces<PLANE, TL, X64>(V, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, nr, fb0, tid);
+  if (VSH && WACT && G.visc) visc_faces<PLANE, TL, X64>(V, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, w, nr, fb0, tid);
 }
 
 // Phase 3-5: the cells of rows 0..nr-1 of the block -- conservative update,
@@ -637,32 +647,42 @@ __device__ __forceinline__ void faces64(const Grid& G, const Consts64& K, const 
 template <int PLANE, bool WACT, class TL, bool VSH, class PV>
 __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Fields& uin, const Fields& u0,
                                          const Fields& uout, StepCtrl* ctrl, int kind, double dt_step, int x0, int y0,
-                                         int nr, int tid, const Fields* hout, unsigned long long& red,
+                                         int w, int nr, int tid, const Fields* hout, unsigned long long& red,
                                          const Fields* qout = nullptr) {
-  constexpr int TX = TL::TX;
+  const SmallDiv by_w(w);
   const X64 dt = dt_step;
   constexpr int kB = PLANE == PLANE_XY ? 1 : 2;  // the axis of b
-  const int ncell = TX * nr;
+  const int ncell = w * nr;
 #pragma unroll 1
   for (int cidx = tid; cidx < ncell; cidx += kTileThreads) {
-    const int cx = cidx % TX, cy = cidx / TX;
+    const int cy = by_w.quotient(cidx), cx = cidx - cy * w;
     const int x = x0 + cx, y = y0 + cy;
-    if (x >= G.na || y >= G.nb) continue;
     const long long o = (long long)y * G.pitch + x;
     X64 un[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) un[v] = (WACT || v != 3) ? uin.f[v][o] : 0.0;
 
-    // IX sweep: un += (F(i-1/2) - F(i+1/2)) * dt / dx
+    // IX sweep: un += (F(i-1/2) - F(i+1/2)) * dt / dx; then IY (x-y plane) or
+    // IZ (x-z plane), gravity on IZ
+    {
+      constexpr int N = WACT ? 5 : 4;  // the stored variables
+      X64 u[N], x[N];
 #pragma unroll
-    for (int v = 0; v < 5; ++v)
-      if (WACT || v != 3)
-        un[v] = un[v] + div_cell((X64(V.fa(v, cy, cx)) - V.fa(v, cy, cx + 1)) * dt, 0);
-    // IY sweep (x-y plane) or IZ sweep (x-z plane), gravity on IZ
+      for (int n = 0; n < N; ++n) {
+        const int v = WACT || n < 3 ? n : 4;
+        u[n] = un[v];
+        x[n] = (X64(V.fa(v, cy, cx)) - V.fa(v, cy, cx + 1)) * dt;
+      }
+      add_div_cell(u, x, 0);
 #pragma unroll
-    for (int v = 0; v < 5; ++v)
-      if (WACT || v != 3)
-        un[v] = un[v] + div_cell((X64(V.fb(v, cy, cx)) - V.fb(v, cy + 1, cx)) * dt, kB);
+      for (int n = 0; n < N; ++n) {
+        const int v = WACT || n < 3 ? n : 4;
+        x[n] = (X64(V.fb(v, cy, cx)) - V.fb(v, cy + 1, cx)) * dt;
+      }
+      add_div_cell(u, x, kB);
+#pragma unroll
+      for (int n = 0; n < N; ++n) un[WACT || n < 3 ? n : 4] = u[n];
+    }
     if (PLANE == PLANE_XZ && G.gravity) {
       un[2] = un[2] + dt * V.q(0, cy + 2, cx + 2) * G.g;
       un[4] = un[4] + half_of(dt) * (X64(V.fb(0, cy, cx)) + V.fb(0, cy + 1, cx)) * G.g;
@@ -673,12 +693,11 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
       const X64 kf = half_of(X64(G.kappa) + G.kappa);
       const int hy = cy + 2, hx = cx + 2;
       const X64 TC = V.temp(hy, hx);
-      const X64 FL = div_cell(kf * (TC - V.temp(hy, hx - 1)), 0);
-      const X64 FR = div_cell(kf * (X64(V.temp(hy, hx + 1)) - TC), 0);
-      const X64 FU = div_cell(kf * (TC - V.temp(hy - 1, hx)), kB);
-      const X64 FD = div_cell(kf * (X64(V.temp(hy + 1, hx)) - TC), kB);
-      const X64 dtdx = div_cell(dt, 0);
-      const X64 dtdb = div_cell(dt, kB);
+      X64 fx[3] = {kf * (TC - V.temp(hy, hx - 1)), kf * (X64(V.temp(hy, hx + 1)) - TC), dt};
+      X64 fb[3] = {kf * (TC - V.temp(hy - 1, hx)), kf * (X64(V.temp(hy + 1, hx)) - TC), dt};
+      div_cells(fx, 0);
+      div_cells(fb, kB);
+      const X64 FL = fx[0], FR = fx[1], dtdx = fx[2], FU = fb[0], FD = fb[1], dtdb = fb[2];
       un[4] = un[4] + (dtdx * (FR - FL) + dtdb * (FD - FU));
     }
     if (WACT && G.visc) {  // Viscosity.h:245-251
@@ -726,13 +745,13 @@ __device__ __forceinline__ void update64(const Grid& G, const PV& V, const Field
 
 // An inactive Euler step still hands its state on (ping-pong buffers); RK2
 // stages leave everything in place.  Copies cell rows [y0, y1) of columns
-// [x0, x0 + TX).
-template <bool WACT, int TX>
-__device__ __forceinline__ void pass_on64(const Grid& G, const Fields& uin, const Fields& uout, int x0, int y0,
+// [x0, x0 + w).
+template <bool WACT>
+__device__ __forceinline__ void pass_on64(const Grid& G, const Fields& uin, const Fields& uout, int x0, int w, int y0,
                                           int y1, int tid) {
-  const int n = TX * (y1 - y0);
+  const int n = w * (y1 - y0);
   for (int c = tid; c < n; c += kTileThreads) {
-    const int x = x0 + c % TX, y = y0 + c / TX;
+    const int x = x0 + c % w, y = y0 + c / w;
     if (x < G.na && y < G.nb) {
       const long long o = (long long)y * G.pitch + x;
 #pragma unroll
@@ -742,8 +761,8 @@ __device__ __forceinline__ void pass_on64(const Grid& G, const Fields& uin, cons
   }
 }
 
-// One strip segment: cell rows [ya, yb) of the TX-wide strip whose first
-// column is x0, marched in blocks of TY rows through a ring of TY + 4
+// One strip segment: cell rows [ya, yb) of the w columns from x0 on (w <= TX;
+// only these are computed), marched in blocks of TY rows through a ring of TY + 4
 // primitive rows, so each block converts only its new rows and reuses the
 // b-face fluxes on the boundary with the previous block; with viscosity the
 // face-only viscous branches are computed once per face (viscous_face).  The
@@ -761,7 +780,7 @@ __device__ __forceinline__ void pass_on64(const Grid& G, const Fields& uin, cons
 template <int PLANE, bool WACT, class TL>
 __device__ __forceinline__ void stage_segment64(const Grid& G, const Fields& uin, const Fields& u0,
                                                 const Fields& uout, StepCtrl* ctrl, int rs, int kind, double dt,
-                                                int x0, int ya, int yb, double* smem, const Fields* hout,
+                                                int x0, int w, int ya, int yb, double* smem, const Fields* hout,
                                                 unsigned long long& red, const TmaState* tin = nullptr,
                                                 unsigned long long* mbar = nullptr, unsigned* phase = nullptr,
                                                 const Fields* qin = nullptr, const Fields* qout = nullptr) {
@@ -790,25 +809,25 @@ __device__ __forceinline__ void stage_segment64(const Grid& G, const Fields& uin
         }
     }
     const int h0 = first ? 0 : 4;
-    const bool staged = tin && nr == TY && x0 >= 2 && x0 + TX + 2 <= G.na && y0 + h0 >= 2 && y0 + TY + 2 <= G.nb;
+    const bool staged = tin && nr == TY && w == TX && x0 >= 2 && x0 + TX + 2 <= G.na && y0 + h0 >= 2 && y0 + TY + 2 <= G.nb;
     if (staged) {
       stage_rows_tma<WACT, TL>(tin, V, mbar, *phase, x0, y0, h0, TY + 4, ctrl);
       convert_rows64<PLANE, WACT, TL>(G, V, h0, TY + 4, tid, qin != nullptr);
     } else {
-      load_prims64<PLANE, WACT, TL>(G, qin ? *qin : uin, V, x0, y0, h0, nr + 4, tid, qin != nullptr);
+      load_prims64<PLANE, WACT, TL>(G, qin ? *qin : uin, V, x0, y0, h0, nr + 4, w, tid, qin != nullptr);
     }
     __syncthreads();
-    faces64<PLANE, WACT, TL, WACT>(G, K, V, rs, nr, first ? 0 : 1, tid);
+    faces64<PLANE, WACT, TL, WACT>(G, K, V, rs, w, nr, first ? 0 : 1, tid);
     __syncthreads();
-    update64<PLANE, WACT, TL, WACT>(G, V, uin, u0, uout, ctrl, kind, dt, x0, y0, nr, tid, hout, red, qout);
+    update64<PLANE, WACT, TL, WACT>(G, V, uin, u0, uout, ctrl, kind, dt, x0, y0, w, nr, tid, hout, red, qout);
     __syncthreads();
     base += TY;
     if (base >= HY) base -= HY;
   }
 }
 
-// One stage of a run of cell rows of problem G, marching down TX-wide strips.
-// The rows are numbered strip by strip (unit u = strip * nb + row) and the
+// One stage of a run of cell rows of problem G, marching down strips of
+// `width` columns (at most TX; the last strip takes what is left).  The rows are numbered strip by strip (unit u = strip * nb + row) and the
 // CTA owns units [u0_, u1_), processed as strip segments (stage_segment64).
 // Host code splits the units evenly over the CTAs that fit on the GPU at
 // once, which balances the FP64 work per SM whatever the grid shape.
@@ -816,11 +835,10 @@ __device__ __forceinline__ void stage_segment64(const Grid& G, const Fields& uin
 // conversion (when ctrl->q_valid) / written by the last stage of a step.
 template <int PLANE, bool WACT, class TL>
 __device__ __forceinline__ void stage_strip64(const Grid& G, const Fields& uin, const Fields& u0, const Fields& uout,
-                                              StepCtrl* ctrl, int rs, int kind, long long u0_, long long u1_,
-                                              double* smem, unsigned long long* s_red, const Fields* hout,
+                                              StepCtrl* ctrl, int rs, int kind, int width, long long u0_,
+                                              long long u1_, double* smem, unsigned long long* s_red, const Fields* hout,
                                               const TmaState* tin = nullptr, unsigned long long* mbar = nullptr,
                                               const Fields* qin = nullptr, const Fields* qout = nullptr) {
-  constexpr int TX = TL::TX;
   const int tid = threadIdx.x;
   const int active = ctrl->active;
   const double dt = ctrl->dt_cur;
@@ -831,13 +849,13 @@ __device__ __forceinline__ void stage_strip64(const Grid& G, const Fields& uin, 
     const int strip = (int)(u / G.nb);
     const int ya = (int)(u - (long long)strip * G.nb);
     const int yb = (int)(ya + (u1_ - u) < (long long)G.nb ? ya + (u1_ - u) : (long long)G.nb);
-    const int x0 = strip * TX;
+    const int x0 = strip * width, w = min(width, G.na - x0);
     u += yb - ya;
     if (!active) {
-      if (kind == STAGE_EULER) pass_on64<WACT, TX>(G, uin, uout, x0, ya, yb, tid);
+      if (kind == STAGE_EULER) pass_on64<WACT>(G, uin, uout, x0, w, ya, yb, tid);
       continue;
     }
-    stage_segment64<PLANE, WACT, TL>(G, uin, u0, uout, ctrl, rs, kind, dt, x0, ya, yb, smem, hout, red, tin,
+    stage_segment64<PLANE, WACT, TL>(G, uin, u0, uout, ctrl, rs, kind, dt, x0, w, ya, yb, smem, hout, red, tin,
                                          mbar, &phase, qin, qout);
   }
   if (active && kind != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[parity ^ 1], s_red);
