@@ -1,7 +1,7 @@
 // fv_stage3d.cu -- the FP64 fused stage kernel of a 3-D problem.
 //
-// One CTA owns a 16 x 16 block of (x, y) columns and marches up a chunk of
-// z layers.  A ring of four z layers of primitives (each with a 2-cell
+// One CTA owns a block of at most 16 x 16 (x, y) columns and marches up a chunk
+// of z layers.  A ring of four z layers of primitives (each with a 2-cell
 // in-plane halo) sits in shared memory; layer k+2 is loaded while the x and y
 // faces of layer k are solved, then every thread solves the z face above its
 // own column and updates its cell.  The z flux below the cell is the one the
@@ -25,14 +25,16 @@
 // Compiled without FMA contraction, operation order as in the reference, the
 // exact replacements of fv_exact64.cuh: bit-identical to the reference's FP64
 // CPU arithmetic.
+#include <algorithm>
+#include <cmath>
+
 #include "fv_tile64.cuh"
 
 namespace fv {
 
 namespace {
 
-constexpr int kTX = 16, kTY = 16;                // columns per CTA
-constexpr int kMinLayersPerCta = 8;              // the prologue loads 4 layers and one extra z face
+constexpr int kTX = 16, kTY = 16;                // most columns per CTA
 constexpr int kThreads = kTX * kTY;              // one thread per column
 constexpr int kHX = kTX + 4, kHY = kTY + 4;      // layer with halo
 constexpr int kLayer = kHX * kHY;
@@ -42,9 +44,6 @@ constexpr int kLayer = kHX * kHY;
 #define FV_3D64_MIN_CTAS 2
 #endif
 constexpr int kRing = 4;                         // z layers held
-constexpr int kNFA = (kTX + 1) * kTY;            // x faces per layer
-constexpr int kNFA_PAD = (kNFA + 31) / 32 * 32;  // keeps each warp on one face kind
-constexpr int kNFB = kTX * (kTY + 1);            // y faces per layer
 static_assert(kThreads == 256, "one thread per column");
 
 // Shared memory: Q[ring][v][hy][hx] primitives, FA[v][fy][fx] x-face and
@@ -132,17 +131,21 @@ __device__ __forceinline__ void c91_ghost(const Grid& G, const Fields& u, const 
   }
 }
 
-// Loads z layer kg of the tile at (x0, y0) into ring slot slot_of(kg)
-// (from the primitive copy qsrc of u when given).
-__device__ __forceinline__ void load_layer(const Grid& G, const Fields& u, const Fields* qsrc, int x0, int y0, int kg,
-                                           const Smem3& S, int tid) {
+// Loads z layer kg of the w x h columns at (x0, y0) and `halo` cells around
+// them into ring slot slot_of(kg) (from the primitive copy qsrc of u when
+// given).
+__device__ __forceinline__ void load_layer(const Grid& G, const Fields& u, const Fields* qsrc, int x0, int y0, int w,
+                                           int h, int halo, int kg, const Smem3& S, int tid) {
   const int s = slot_of(kg);
   const bool c91 = G.bc_c == DBC_C91 && (kg < 0 || kg >= G.nc);
   bool fz = false;
   const int sz = c91 ? 0 : bc_source(kg, G.nc, G.bc_c, fz);
   const long long zoff = (long long)sz * G.nb * G.pitch;
-  for (int idx = tid; idx < kLayer; idx += kThreads) {
-    const int hy = idx / kHX, hx = idx - hy * kHX;
+  const int nx = w + 2 * halo, n = nx * (h + 2 * halo);
+  const SmallDiv by_nx(nx);
+  for (int idx = tid; idx < n; idx += kThreads) {
+    const int r = by_nx.quotient(idx);
+    const int hy = r + 2 - halo, hx = idx - r * nx + 2 - halo;
     bool fa, fb;
     const int sa = bc_source(x0 + hx - 2, G.na, G.bc_a, fa);
     const int sb = bc_source(y0 + hy - 2, G.nb, G.bc_b, fb);
@@ -322,7 +325,7 @@ __device__ __forceinline__ void viscous_iz3d(const PA& P, X64 odx, X64 odz, X64 
   }
 }
 
-// One stage for the columns (bx, by) and z layers [k0, k1); rs 0 HLL /
+// One stage for the w x h columns from (x0, y0) on and z layers [k0, k1); rs 0 HLL /
 // 1 HLLC, kind a StageKind (constants in the one-problem kernel, per work
 // item in the batch kernel); P2: every cell size is a power of two (callers
 // branch on it once, uniformly).  Every thread of the CTA must call it; the
@@ -331,15 +334,18 @@ __device__ __forceinline__ void viscous_iz3d(const PA& P, X64 odx, X64 odz, X64 
 template <bool CORR>
 __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin, const Fields& u0,
                                                 const Fields& uout, StepCtrl* __restrict__ ctrl, int rs, int kind,
-                                                int bx, int by, int k0, int k1, const Fields& hout, double* smem_raw,
+                                                int x0, int y0, int w, int h, int k0, int k1, const Fields& hout,
+                                                double* smem_raw,
                                                 unsigned long long& red, const Fields* qin = nullptr,
                                                 const Fields* qout = nullptr) {
   const Smem3 S{smem_raw};
   const int tid = threadIdx.x;
-  const int x0 = bx * kTX, y0 = by * kTY;
-  const int cx = tid % kTX, cy = tid / kTX;
+  const SmallDiv by_w(w), by_wa(w + 1);
+  const int cy = by_w.quotient(tid), cx = tid - cy * w;
   const int x = x0 + cx, y = y0 + cy;
-  const bool own = x < G.na && y < G.nb;
+  const bool own = tid < w * h;
+  const int nfa = (w + 1) * h, nfa_pad = (nfa + 31) & ~31;  // x faces; padded to keep each warp on one face kind
+  const int nfaces = nfa_pad + w * (h + 1);
   const long long col = (long long)y * G.pitch + x;
   const long long zstride = (long long)G.nb * G.pitch;
 
@@ -358,9 +364,12 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
   const int recon = G.recon;
   const bool need_pout = G.wb_flux_z || G.bc_c == DBC_C91;
   const bool vsh = !CORR && G.visc;  // shared-face viscous fluxes (FA / FB reused)
+  // cells read around a cell: slopes reach two out; without them the faces,
+  // conduction and viscosity reach one
+  const int halo = recon == R_PLM ? 2 : 1;
 
-  // prologue: layers k0-2 .. k0+1, then the z face k0-1/2 of the own column
-  for (int kg = k0 - 2; kg <= k0 + 1; ++kg) load_layer(G, uin, qin, x0, y0, kg, S, tid);
+  // prologue: layers k0-halo .. k0+halo-1, then the z face k0-1/2 of the own column
+  for (int kg = k0 - halo; kg < k0 + halo; ++kg) load_layer(G, uin, qin, x0, y0, w, h, halo, kg, S, tid);
   __syncthreads();
   X64 fzL[5], poutL = 0.0;
   if (own) {
@@ -375,14 +384,14 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
 
 #pragma unroll 1
   for (int k = k0; k < k1; ++k) {
-    // ---- 1. layer k+2 in, x and y faces of layer k ----
-    load_layer(G, uin, qin, x0, y0, k + 2, S, tid);
+    // ---- 1. layer k+halo in, x and y faces of layer k ----
+    load_layer(G, uin, qin, x0, y0, w, h, halo, k + halo, S, tid);
     const int sk = slot_of(k);
-    for (int it = tid; it < kNFA_PAD + kNFB; it += kThreads) {
+    for (int it = tid; it < nfaces; it += kThreads) {
       X64 c[4][5], f[5];
-      if (it < kNFA_PAD) {
-        if (it >= kNFA) continue;
-        const int fy = it / (kTX + 1), fx = it - fy * (kTX + 1);
+      if (it < nfa_pad) {
+        if (it >= nfa) continue;
+        const int fy = by_wa.quotient(it), fx = it - fy * (w + 1);
 #pragma unroll
         for (int m = 0; m < 4; ++m)
 #pragma unroll
@@ -391,8 +400,8 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
 #pragma unroll
         for (int v = 0; v < 5; ++v) S.fa(v, fy, fx) = f[v].v;
       } else {
-        const int j = it - kNFA_PAD;
-        const int fy = j / kTX, fx = j - fy * kTX;
+        const int j = it - nfa_pad;
+        const int fy = by_w.quotient(j), fx = j - fy * w;
 #pragma unroll
         for (int m = 0; m < 4; ++m)
 #pragma unroll
@@ -506,17 +515,17 @@ __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin
     }
     if (vsh) {  // viscosity with the face-only branches solved once per face
       __syncthreads();  // every cell is done with the hydro fluxes in FA / FB
-      for (int it = tid; it < kNFA_PAD + kNFB; it += kThreads) {
+      for (int it = tid; it < nfaces; it += kThreads) {
         X64 g[4];
-        if (it < kNFA_PAD) {
-          if (it >= kNFA) continue;
-          const int fy = it / (kTX + 1), fx = it - fy * (kTX + 1);
+        if (it < nfa_pad) {
+          if (it >= nfa) continue;
+          const int fy = by_wa.quotient(it), fx = it - fy * (w + 1);
           viscous_face3d<0>(RingVel{S, k, fy + 2, fx + 2}, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, g);
 #pragma unroll
           for (int v = 0; v < 4; ++v) S.fa(v, fy, fx) = g[v].v;
         } else {
-          const int j = it - kNFA_PAD;
-          const int fy = j / kTX, fx = j - fy * kTX;
+          const int j = it - nfa_pad;
+          const int fy = by_w.quotient(j), fx = j - fy * w;
           viscous_face3d<1>(RingVel{S, k, fy + 2, fx + 2}, G.inv_dx, G.inv_dy, G.inv_dz, G.mu, g);
 #pragma unroll
           for (int v = 0; v < 4; ++v) S.fb(v, fy, fx) = g[v].v;
@@ -581,8 +590,10 @@ __device__ __forceinline__ void stage3d_body(const Grid& G, const Fields& uin, c
   const int active = ctrl->active, parity = ctrl->parity;
   const int k0 = bz * tz;
   const int k1 = min(k0 + tz, G.nc);
+  const int x0 = bx * kTX, y0 = by * kTY;
   unsigned long long red = 0ull;
-  stage3d_segment<CORR>(G, uin, u0, uout, ctrl, rs, kind, bx, by, k0, k1, hout, smem_raw, red);
+  stage3d_segment<CORR>(G, uin, u0, uout, ctrl, rs, kind, x0, y0, min(kTX, G.na - x0), min(kTY, G.nb - y0), k0, k1,
+                        hout, smem_raw, red);
   if (active && kind != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[parity ^ 1], s_red);
 }
 
@@ -590,29 +601,30 @@ __device__ __forceinline__ void stage3d_body(const Grid& G, const Fields& uin, c
 // column block; returns the CTA's CFL maximum.
 template <bool CORR, int RS, int KIND>
 __device__ __forceinline__ unsigned long long march3d(const Grid& G, const Fields& uin, const Fields& u0,
-                                                      const Fields& uout, StepCtrl* __restrict__ ctrl, long long ub,
-                                                      long long ue, const Fields& hout, double* smem_raw,
+                                                      const Fields& uout, StepCtrl* __restrict__ ctrl, int bw, int bh,
+                                                      long long ub, long long ue, const Fields& hout, double* smem_raw,
                                                       const Fields* qin, const Fields* qout) {
-  const int tiles_x = (G.na + kTX - 1) / kTX;
+  const int tiles_x = (G.na + bw - 1) / bw;
   unsigned long long red = 0ull;
   for (long long u = ub; u < ue;) {
     const int cb = (int)(u / G.nc);
     const int k0 = (int)(u - (long long)cb * G.nc);
     const int k1 = (int)(k0 + (ue - u) < (long long)G.nc ? k0 + (ue - u) : (long long)G.nc);
     u += k1 - k0;
-    stage3d_segment<CORR>(G, uin, u0, uout, ctrl, RS, KIND, cb % tiles_x, cb / tiles_x, k0, k1, hout, smem_raw,
-                              red, qin, qout);
+    const int x0 = cb % tiles_x * bw, y0 = cb / tiles_x * bh;
+    stage3d_segment<CORR>(G, uin, u0, uout, ctrl, RS, KIND, x0, y0, min(bw, G.na - x0), min(bh, G.nb - y0), k0, k1,
+                          hout, smem_raw, red, qin, qout);
   }
   return red;
 }
 
-// The one-problem kernel: the (column block, z layer) units, numbered column
-// block by column block, are split evenly over the CTAs that fit on the GPU
+// The one-problem kernel: the (column block, z layer) units (split_blocks),
+// numbered column block by column block, are split evenly over the CTAs that fit on the GPU
 // at once; a CTA marches each column block of its range over its layers.
 template <int RS, int KIND, bool CORR>
 __global__ void __launch_bounds__(kThreads, FV_3D64_MIN_CTAS)
 stage3d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u0, const Fields uout, StepCtrl* __restrict__ ctrl,
-             long long units, const Fields hout, const Fields qin, const Fields qout) {
+             int bw, int bh, long long units, const Fields hout, const Fields qin, const Fields qout) {
   extern __shared__ double smem_raw[];
   __shared__ unsigned long long s_red[kThreads / 32];
   __shared__ Grid s_grid;
@@ -629,7 +641,7 @@ stage3d_fp64(const __grid_constant__ Grid grid, const Fields uin, const Fields u
   const Fields* qi = qin.f[0] && ctrl->q_valid ? &qin : nullptr;
   const Fields* qo = qout.f[0] ? &qout : nullptr;
   const unsigned long long red =
-      march3d<CORR, RS, KIND>(G, uin, u0, uout, ctrl, ub, ue, hout, smem_raw, qi, qo);
+      march3d<CORR, RS, KIND>(G, uin, u0, uout, ctrl, bw, bh, ub, ue, hout, smem_raw, qi, qo);
   if (active && KIND != STAGE_RK_1) block_max_atomic(red, &ctrl->slot[parity ^ 1], s_red);
   // the copy is complete once this launch is (the next reader is a later kernel)
   if (active && qo && threadIdx.x == 0) ctrl->q_valid = 1;
@@ -644,6 +656,52 @@ int sm_count3d() {
       n = 1;
   }
   return n;
+}
+
+// The split of a grid into blocks of bw x bh columns whose (block, z layer)
+// units are shared out evenly over `ctas` CTAs.
+struct Blocks {
+  int bw, bh;
+  long long units, ctas;
+};
+
+// The blocks and CTA count with the least estimated time of the busiest SM,
+// counted in FP64 warp operations (a warp with idle lanes costs a whole one):
+// per layer the faces, conversions and cell updates of a block, per CTA the
+// prologue (its first layers and one z face).  Blocks are of equal size, so
+// that a ragged grid computes no columns it does not have (101 x 83 columns:
+// 7 x 6 blocks of 15 x 14, not of 16 x 16), and lower ones serve small grids,
+// whose units then share out more evenly.  One resident CTA keeps about 60 %
+// of the FP64 pipe busy between its barriers (as in the 2-D kernel).
+Blocks split_blocks(const Grid& G, int rs, int resident) {
+  const int sms = sm_count3d();
+  const int halo = G.recon == R_PLM ? 2 : 1;
+  const double face = (rs == 0 ? 120 : 80) - (G.recon == R_PLM ? 0 : 25);
+  const double cell = 70 + (G.tc ? 30 : 0) + (G.visc ? 110 : 0), conv = 14;
+  auto warps = [](double lanes) { return std::ceil(lanes / 32.0); };
+  Blocks best{};
+  double best_t = 0.0;
+  for (int bh0 : {kTY, 12, 8}) {
+    const int nx = (G.na + kTX - 1) / kTX, ny = (G.nb + bh0 - 1) / bh0;
+    const int bw = (G.na + nx - 1) / nx, bh = (G.nb + ny - 1) / ny;
+    const long long units = (long long)nx * ny * G.nc;
+    const double z_face = face * warps((double)bw * bh);
+    const double load = conv * warps((bw + 2.0 * halo) * (bh + 2.0 * halo));
+    const double layer = face * (warps((bw + 1.0) * bh) + warps(bw * (bh + 1.0))) + z_face +
+                         cell * warps((double)bw * bh) + load;
+    for (int per_sm = 1; per_sm <= resident; ++per_sm) {
+      const long long ctas = std::min(units, (long long)per_sm * sms);
+      const long long layers = (units + ctas - 1) / ctas;  // of the busiest CTA
+      const double starts = 1.0 + (layers - 1) / G.nc;     // column blocks it begins, about
+      const long long on_sm = (ctas + sms - 1) / sms;
+      const double t = on_sm * (layers * layer + starts * (2 * halo * load + z_face)) / (on_sm == 1 ? 0.6 : 1.0);
+      if (best.ctas == 0 || t < best_t * 0.99) {
+        best = Blocks{bw, bh, units, ctas};
+        best_t = t;
+      }
+    }
+  }
+  return best;
 }
 
 template <int RS, int KIND, bool CORR>
@@ -663,15 +721,10 @@ cudaError_t launch_one(const Grid& G, Fields uin, Fields u0, Fields uout, StepCt
     if (e != cudaSuccess) return e;
     if (resident[tc] < 1) resident[tc] = 1;
   }
-  const long long cols = (long long)((G.na + kTX - 1) / kTX) * ((G.nb + kTY - 1) / kTY);
-  const long long units = cols * G.nc;
-  long long ctas = units / kMinLayersPerCta;
-  const long long slots = (long long)resident[tc] * sm_count3d();
-  if (ctas > slots) ctas = slots;
-  if (ctas < 1) ctas = 1;
+  const Blocks p = split_blocks(G, RS, resident[tc]);
   const Fields none{};
-  const cudaError_t e = launch_pdl(kern, dim3((unsigned)ctas), dim3(kThreads), Smem3::bytes(tc), st, G, uin, u0, uout,
-                                   ctrl, units, hout ? *hout : none, pc.qin ? *pc.qin : none,
+  const cudaError_t e = launch_pdl(kern, dim3((unsigned)p.ctas), dim3(kThreads), Smem3::bytes(tc), st, G, uin, u0,
+                                   uout, ctrl, p.bw, p.bh, p.units, hout ? *hout : none, pc.qin ? *pc.qin : none,
                                    pc.qout ? *pc.qout : none);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
