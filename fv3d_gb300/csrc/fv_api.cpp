@@ -9,6 +9,7 @@
 // reads the control block back between replays.
 #include <cmath>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -476,6 +477,37 @@ const double* DeviceView(const double* p, bool* host) {
   return pageable ? p : nullptr;
 }
 
+// Takes the state from src: primitives straight out of pinned host arrays in
+// one kernel (with the primitive copy of the new state), everything else
+// through copies into A (and primToCons in place).
+int TakeState(fv_sim* s, const double* const src[5], bool prim) {
+  Fields view;
+  if (prim && fv::pinned_fields(src, (long long)s->G.na * s->G.rows, &view)) {
+    const bool keep_q = s->Q.f[0] != nullptr;
+    Timed t(s, KC_CONV);
+    // with the third momentum, so that its field holds the state's zeros too
+    cudaError_t e = fv::launch_prim_to_cons_from(s->G, true, view, s->A, nullptr, 0, s->stream,
+                                                 keep_q ? &s->Q : nullptr, keep_q ? &s->d_ctrl->q_valid : nullptr);
+    if (e != cudaSuccess) return Fail(s, FV_ERR_CUDA, "primToCons launch: %s", cudaGetErrorString(e));
+    if (keep_q) s->q_dirty = true;
+    t.done();
+    CUDA_TRY(s, cudaStreamSynchronize(s->stream));  // the caller may reuse its arrays
+    s->slot_valid = false;
+    return FV_OK;
+  }
+  int rc = CopyIn(s, s->A, src, true);
+  if (rc) return rc;
+  if (prim) {
+    Timed t(s, KC_CONV);
+    cudaError_t e = fv::launch_prim_to_cons2d(s->G, s->A, s->stream);
+    if (e != cudaSuccess) return Fail(s, FV_ERR_CUDA, "primToCons launch: %s", cudaGetErrorString(e));
+    t.done();
+  }
+  CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+  s->slot_valid = false;
+  return FV_OK;
+}
+
 int SetState(fv_sim* s, const double* const ref_fields[5], bool prim) {
   if (!s) return FV_ERR_PARAM;
   int slot_of[5];
@@ -498,16 +530,8 @@ int SetState(fv_sim* s, const double* const ref_fields[5], bool prim) {
   s->cur = 0;
   int rc = DropPrims(s);
   if (rc) return rc;
-  rc = CopyIn(s, s->A, src, true);
+  rc = TakeState(s, src, prim);
   if (rc) return rc;
-  if (prim) {
-    Timed t(s, KC_CONV);
-    cudaError_t e = fv::launch_prim_to_cons2d(s->G, s->A, s->stream);
-    if (e != cudaSuccess) return Fail(s, FV_ERR_CUDA, "primToCons launch: %s", cudaGetErrorString(e));
-    t.done();
-  }
-  CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-  s->slot_valid = false;
   s->state_set = true;
   return FV_OK;
 }
@@ -515,6 +539,25 @@ int SetState(fv_sim* s, const double* const ref_fields[5], bool prim) {
 }  // namespace
 
 namespace fv {
+
+bool pinned_fields(const double* const host[5], long long n, Fields* view) {
+  for (int v = 0; v < 5; ++v) {
+    view->f[v] = nullptr;
+    if (!host[v]) continue;
+    cudaPointerAttributes a{}, z{};
+    if (cudaPointerGetAttributes(&a, host[v]) != cudaSuccess ||
+        cudaPointerGetAttributes(&z, host[v] + (n - 1)) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    double* first = static_cast<double*>(a.devicePointer);
+    if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !first ||
+        reinterpret_cast<uintptr_t>(first) % sizeof(double) || z.devicePointer != first + (n - 1))
+      return false;
+    view->f[v] = first;
+  }
+  return true;
+}
 
 // The parameter checks and grid set-up of fvgpu_create, without allocating:
 // fills G and the constant CFL terms, or returns a status with a message.
@@ -744,6 +787,15 @@ int fvgpu_get_prim(fv_sim* s, double* rho, double* u, double* v, double* w, doub
   double* ref[5] = {rho, u, v, w, p};
   double* dst[5];
   for (int k = 0; k < 5; ++k) dst[slot_of[k]] = ref[k];
+  Fields view;
+  if (fv::pinned_fields(dst, (long long)s->G.na * s->G.rows, &view)) {  // written by the conversion itself
+    Timed t(s, KC_CONV);
+    cudaError_t e = fv::launch_cons_to_prim_to(s->G, s->wact, Current(s), view, s->stream);
+    if (e != cudaSuccess) return Fail(s, FV_ERR_CUDA, "consToPrim launch: %s", cudaGetErrorString(e));
+    t.done();
+    CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+    return FV_OK;
+  }
   {
     Timed t(s, KC_CONV);
     cudaError_t e = fv::launch_cons_to_prim2d(s->G, Current(s), s->S, s->stream);

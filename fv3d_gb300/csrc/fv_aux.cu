@@ -16,6 +16,11 @@ int grid_for(long long n, int block) {
   return b < 1 ? 1 : (int)b;
 }
 
+// Threads per CTA of a kernel with one cell per thread and FP64 arithmetic:
+// small grids spread over the SMs (the FP64 pipe bounds an SM: 256 cells take
+// it about 5 us).
+int block_for(long long n) { return n >= 152 * 256 ? 256 : (n >= 152 * 128 ? 128 : 64); }
+
 // ComputeDt.h:28-54 over the interior: max inv_dt_hyp into ctrl->slot[slot].
 template <int PLANE, bool WACT>
 __global__ void __launch_bounds__(256) reduce2d_fp64(const Grid G, const Fields u, StepCtrl* ctrl, int slot) {
@@ -94,19 +99,19 @@ __global__ void __launch_bounds__(256) prim_to_cons_from(const Grid G, const Fie
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
     const int y = (int)(c / G.na), x = (int)(c - (long long)y * G.na);
     const long long o = (long long)y * G.pitch + x;
-    const double r = src.f[0][c];
-    const double va = src.f[1] ? src.f[1][c] : 0.0, vb = src.f[2] ? src.f[2][c] : 0.0;
-    const double vc = (WACT && src.f[3]) ? src.f[3][c] : 0.0;
-    const double ma = __dmul_rn(r, va), mb = __dmul_rn(r, vb), mc = __dmul_rn(r, vc);
-    const double mx = ma, my = PLANE == PLANE_XY ? mb : mc, mz = PLANE == PLANE_XY ? mc : mb;
-    const double sq = __dadd_rn(__dadd_rn(__dmul_rn(mx, mx), __dmul_rn(my, my)), __dmul_rn(mz, mz));
-    const double Ek = __ddiv_rn(__dmul_rn(0.5, sq), r);
-    const double E = __dadd_rn(Ek, __ddiv_rn(src.f[4][c], G.gm1));
-    dst.f[0][o] = r;
-    dst.f[1][o] = ma;
-    dst.f[2][o] = mb;
-    if (WACT) dst.f[3][o] = mc;
-    dst.f[4][o] = E;
+    const X64 r = src.f[0][c];
+    const X64 va = src.f[1] ? src.f[1][c] : 0.0, vb = src.f[2] ? src.f[2][c] : 0.0;
+    const X64 vc = (WACT && src.f[3]) ? src.f[3][c] : 0.0;
+    const X64 ma = r * va, mb = r * vb, mc = r * vc;
+    const X64 mx = ma, my = PLANE == PLANE_XY ? mb : mc, mz = PLANE == PLANE_XY ? mc : mb;
+    X64 Ek = half_of(mx * mx + my * my + mz * mz), e = src.f[4][c];
+    quot_pair(Ek, prepare_div(r), e, s_cell64.gm1);
+    const X64 E = Ek + e;
+    dst.f[0][o] = r.v;
+    dst.f[1][o] = ma.v;
+    dst.f[2][o] = mb.v;
+    if (WACT) dst.f[3][o] = mc.v;
+    dst.f[4][o] = E.v;
     if (REDUCE || qout.f[0]) {
       const X64 u[5] = {r, ma, mb, mc, E};
       X64 q[5];
@@ -149,6 +154,29 @@ __global__ void cons_to_prim2d(const Grid G, const Fields src, const Fields dst)
     dst.f[2][o] = vb;
     dst.f[3][o] = vc;
     dst.f[4][o] = p;
+  }
+}
+
+// consToPrim straight into unpadded primitive arrays the GPU can address (a
+// caller's pinned host arrays; a null one is skipped).  Without the third
+// momentum its velocity is written as zero.
+template <int PLANE, bool WACT>
+__global__ void __launch_bounds__(256) cons_to_prim_to(const Grid G, const Fields src, const Fields dst) {
+  opaque64_init();
+  __syncthreads();
+  const X64 gm1 = G.gm1;
+  const long long n = (long long)G.na * G.rows;
+  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
+    const int y = (int)(c / G.na), x = (int)(c - (long long)y * G.na);
+    const long long o = (long long)y * G.pitch + x;
+    X64 u[5], q[5];
+    Div64 D;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) u[v] = (WACT || v != 3) ? src.f[v][o] : 0.0;
+    cons_to_prim64<PLANE, WACT>(u, gm1, q, D);
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      if (dst.f[v]) dst.f[v][c] = q[v].v;
   }
 }
 
@@ -228,11 +256,11 @@ cudaError_t launch_prim_to_cons2d(const Grid& G, Fields u, cudaStream_t st) {
 template <int PLANE, bool WACT>
 cudaError_t launch_p2c_from(const Grid& G, Fields src, Fields dst, StepCtrl* ctrl, int slot, const Fields& qout,
                             int* q_valid, cudaStream_t st) {
-  const int grid = grid_for((long long)G.na * G.rows, 256);
+  const int block = block_for((long long)G.na * G.rows), grid = grid_for((long long)G.na * G.rows, block);
   if (ctrl)
-    prim_to_cons_from<PLANE, WACT, true><<<grid, 256, 0, st>>>(G, src, dst, ctrl, slot, qout, q_valid);
+    prim_to_cons_from<PLANE, WACT, true><<<grid, block, 0, st>>>(G, src, dst, ctrl, slot, qout, q_valid);
   else
-    prim_to_cons_from<PLANE, WACT, false><<<grid, 256, 0, st>>>(G, src, dst, ctrl, slot, qout, q_valid);
+    prim_to_cons_from<PLANE, WACT, false><<<grid, block, 0, st>>>(G, src, dst, ctrl, slot, qout, q_valid);
   return cudaGetLastError();
 }
 
@@ -251,6 +279,18 @@ cudaError_t launch_cons_to_prim2d(const Grid& G, Fields src, Fields dst, cudaStr
   const int grid = grid_for((long long)G.na * G.rows, 256);
   if (G.plane == PLANE_XY) cons_to_prim2d<PLANE_XY><<<grid, 256, 0, st>>>(G, src, dst);
   else cons_to_prim2d<PLANE_XZ><<<grid, 256, 0, st>>>(G, src, dst);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_cons_to_prim_to(const Grid& G, bool wact, Fields src, Fields dst, cudaStream_t st) {
+  const int block = block_for((long long)G.na * G.rows), grid = grid_for((long long)G.na * G.rows, block);
+  if (G.plane == PLANE_XY) {
+    if (wact) cons_to_prim_to<PLANE_XY, true><<<grid, block, 0, st>>>(G, src, dst);
+    else cons_to_prim_to<PLANE_XY, false><<<grid, block, 0, st>>>(G, src, dst);
+  } else {
+    if (wact) cons_to_prim_to<PLANE_XZ, true><<<grid, block, 0, st>>>(G, src, dst);
+    else cons_to_prim_to<PLANE_XZ, false><<<grid, block, 0, st>>>(G, src, dst);
+  }
   return cudaGetLastError();
 }
 

@@ -875,6 +875,19 @@ int fvgpu_batch_set_prim(fv_batch* b, int inst, const double* rho, const double*
   if (!b->prepared) ReleaseGroups(b);
   if (b->Q[inst].f[0])  // the primitive copy no longer matches the state
     BCUDA(b, cudaMemsetAsync(&b->d_ctrl[inst].q_valid, 0, sizeof(int), b->stream));
+  Fields view;
+  if (fv::pinned_fields(src, (long long)G.na * G.rows, &view)) {  // read in place by one kernel
+    const cudaError_t pe =
+        b->precision == FV_PREC_FP64
+            ? fv::launch_prim_to_cons_from(G, true, view, Current(b, inst), nullptr, 0, b->stream)
+            : fv::launch_prim_to_pairs_from(G, view, Current(b, inst), b->stream);
+    if (pe != cudaSuccess) return Fail(b, FV_ERR_CUDA, "set_prim: %s", cudaGetErrorString(pe));
+    b->launches += 1;
+    BCUDA(b, cudaStreamSynchronize(b->stream));
+    b->state_set[inst] = 1;
+    b->slot_valid[inst] = 0;
+    return FV_OK;
+  }
   // FP64 values into the staging buffer (the current state for FP64, scratch
   // for the mixed form), primToCons in place, then split into pairs (mixed)
   Fields stage = b->precision == FV_PREC_FP64 ? Current(b, inst) : Fields();
@@ -955,6 +968,15 @@ int fvgpu_batch_get_prim(fv_batch* b, int inst, double* rho, double* u, double* 
   double* ref[5] = {rho, u, v, w, pr};
   double* dst[5];
   for (int k = 0; k < 5; ++k) dst[slot_of[k]] = ref[k];
+  Fields view;
+  if (fv::pinned_fields(dst, (long long)G.na * G.rows, &view)) {  // written in place by the conversion
+    const cudaError_t pe = b->precision == FV_PREC_FP64
+                               ? fv::launch_cons_to_prim_to(G, b->wact[inst], Current(b, inst), view, b->stream)
+                               : fv::launch_pairs_to_prim_to(G, b->wact[inst], Current(b, inst), view, b->stream);
+    if (pe != cudaSuccess) return Fail(b, FV_ERR_CUDA, "get_prim: %s", cudaGetErrorString(pe));
+    BCUDA(b, cudaStreamSynchronize(b->stream));
+    return FV_OK;
+  }
   Fields S;
   for (int k = 0; k < 5; ++k) S.f[k] = b->scratch + (size_t)k * G.fstride;
   cudaError_t e;

@@ -250,6 +250,58 @@ __global__ void double_from_pairs(const Grid G, const Fields src, const Fields d
   }
 }
 
+// primToCons (States.h:20-31) of a caller's unpadded primitive arrays (a null
+// field reads as zero), in FP64, split into pairs as pairs_from_double.
+template <int PLANE>
+__global__ void __launch_bounds__(256) prim_to_pairs_from(const Grid G, const Fields src, const Fields dst) {
+  const long long n = (long long)G.na * G.rows;
+  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
+    const int y = (int)(c / G.na), x = (int)(c - (long long)y * G.na);
+    const long long o = (long long)y * G.pitch + x;
+    double q[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) q[v] = src.f[v] ? src.f[v][c] : 0.0;
+    const double r = q[0];
+    const double ma = __dmul_rn(r, q[1]), mb = __dmul_rn(r, q[2]), mc = __dmul_rn(r, q[3]);
+    const double mx = ma, my = PLANE == PLANE_XY ? mb : mc, mz = PLANE == PLANE_XY ? mc : mb;
+    const double s = __dadd_rn(__dadd_rn(__dmul_rn(mx, mx), __dmul_rn(my, my)), __dmul_rn(mz, mz));
+    const double E = __dadd_rn(__ddiv_rn(__dmul_rn(0.5, s), r), __ddiv_rn(q[4], G.gm1));
+    const double u[5] = {r, ma, mb, mc, E};
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      const float hi = __double2float_rn(u[v]);
+      const float lo = __double2float_rn(u[v] - (double)hi);
+      reinterpret_cast<float2*>(dst.f[v])[o] = make_float2(hi, lo);
+    }
+  }
+}
+
+// consToPrim (States.h:34-45) of pairs, in FP64, into a caller's unpadded
+// arrays (a null one is skipped).
+template <int PLANE, bool WACT>
+__global__ void __launch_bounds__(256) pairs_to_prim_to(const Grid G, const Fields pairs, const Fields dst) {
+  const long long n = (long long)G.na * G.rows;
+  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
+    const int y = (int)(c / G.na), x = (int)(c - (long long)y * G.na);
+    const long long o = (long long)y * G.pitch + x;
+    double u[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      const float2 w = (WACT || v != 3) ? reinterpret_cast<const float2*>(pairs.f[v])[o] : make_float2(0.0f, 0.0f);
+      u[v] = (double)w.x + (double)w.y;
+    }
+    const double r = u[0];
+    const double va = __ddiv_rn(u[1], r), vb = __ddiv_rn(u[2], r), vc = WACT ? __ddiv_rn(u[3], r) : 0.0;
+    const double vx = va, vy = PLANE == PLANE_XY ? vb : vc, vz = PLANE == PLANE_XY ? vc : vb;
+    const double s = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
+    const double Ek = __dmul_rn(__dmul_rn(0.5, r), s);
+    const double q[5] = {r, va, vb, vc, __dmul_rn(__dsub_rn(u[4], Ek), G.gm1)};
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      if (dst.f[v]) dst.f[v][c] = q[v];
+  }
+}
+
 }  // namespace
 
 int batch_tile_shapes32(const TileShape** shapes) {
@@ -344,6 +396,25 @@ cudaError_t launch_reduce2d_mixed(const Grid& G, bool wact, Fields pairs, StepCt
 
 cudaError_t launch_pairs_from_double(const Grid& G, Fields src, Fields dst_pairs, cudaStream_t st) {
   pairs_from_double<<<grid_for((long long)G.na * G.rows, 256), 256, 0, st>>>(G, src, dst_pairs);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prim_to_pairs_from(const Grid& G, Fields src, Fields dst_pairs, cudaStream_t st) {
+  const int grid = grid_for((long long)G.na * G.rows, 128);
+  if (G.plane == PLANE_XY) prim_to_pairs_from<PLANE_XY><<<grid, 128, 0, st>>>(G, src, dst_pairs);
+  else prim_to_pairs_from<PLANE_XZ><<<grid, 128, 0, st>>>(G, src, dst_pairs);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pairs_to_prim_to(const Grid& G, bool wact, Fields src_pairs, Fields dst, cudaStream_t st) {
+  const int grid = grid_for((long long)G.na * G.rows, 128);
+  if (G.plane == PLANE_XY) {
+    if (wact) pairs_to_prim_to<PLANE_XY, true><<<grid, 128, 0, st>>>(G, src_pairs, dst);
+    else pairs_to_prim_to<PLANE_XY, false><<<grid, 128, 0, st>>>(G, src_pairs, dst);
+  } else {
+    if (wact) pairs_to_prim_to<PLANE_XZ, true><<<grid, 128, 0, st>>>(G, src_pairs, dst);
+    else pairs_to_prim_to<PLANE_XZ, false><<<grid, 128, 0, st>>>(G, src_pairs, dst);
+  }
   return cudaGetLastError();
 }
 

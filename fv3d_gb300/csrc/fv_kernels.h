@@ -131,6 +131,19 @@ cudaError_t launch_control(StepCtrl* ctrl, int n, int mode_override, double dt_g
 cudaError_t launch_prim_to_cons2d(const Grid& G, Fields u, cudaStream_t stream);
 cudaError_t launch_cons_to_prim2d(const Grid& G, Fields src, Fields dst, cudaStream_t stream);
 
+// consToPrim of src into unpadded arrays of na x rows values that the GPU can
+// address (storage order, a null field is skipped); wact as the stages'.
+cudaError_t launch_cons_to_prim_to(const Grid& G, bool wact, Fields src, Fields dst, cudaStream_t stream);
+// The same two for the FP32-mixed form's (hi, lo) pairs: primToCons of
+// unpadded primitive arrays into pairs, consToPrim of pairs into such arrays,
+// both in FP64 arithmetic.
+cudaError_t launch_prim_to_pairs_from(const Grid& G, Fields src, Fields dst_pairs, cudaStream_t stream);
+cudaError_t launch_pairs_to_prim_to(const Grid& G, bool wact, Fields src_pairs, Fields dst, cudaStream_t stream);
+// The device's view of the caller's arrays of n values when all of them are
+// pinned host memory from end to end (null entries stay null), so that a
+// kernel can read or write them in place; false otherwise.
+bool pinned_fields(const double* const host[5], long long n, Fields* view);
+
 // Compensated per-block partial sums of the five conserved fields:
 // partial[(blk*5 + v)*2 + {0,1}] = (sum, compensation).  Returns the block
 // count through nblocks.
