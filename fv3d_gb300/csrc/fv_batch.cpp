@@ -329,6 +329,12 @@ std::vector<BatchInst> Describe(const fv_batch* b, const Group& g, int shape, St
     const int chunks = g.ndim == 3 ? (I.G.nc + I.tz - 1) / I.tz : 1;
     I.tile0 = t0;
     I.rs = b->p[i].riemann_solver == FV_HLL ? 0 : 1;
+    const double inv_d[3] = {I.G.inv_dx, I.G.inv_dy, I.G.inv_dz};
+    for (int a = 0; a < 3; ++a) {
+      I.inv_d[a] = fv::float_pair(inv_d[a]);
+      I.mu_d[a] = fv::float_pair(I.G.mu * inv_d[a]);
+      I.kappa_d2[a] = fv::float_pair(I.G.kappa * inv_d[a] * inv_d[a]);
+    }
     t0 += I.tiles_x * I.tiles_y * chunks;
     out.push_back(I);
   }
@@ -481,6 +487,7 @@ int Autotune(fv_batch* b, Group& g) {
     std::memset(&hc[i], 0, sizeof(StepCtrl));
     hc[i].active = 1;
     hc[i].dt_cur = 1.0e-9;
+    hc[i].dt_pair = fv::float_pair(1.0e-9);
   }
   cudaMemcpyAsync(tune_ctrl, hc.data(), sizeof(StepCtrl) * b->n, cudaMemcpyHostToDevice, b->stream);
   cudaEvent_t e0, e1;

@@ -54,6 +54,7 @@ __device__ __forceinline__ void step_control(StepCtrl& c, int mode_override, dou
   c.parity = p;
   c.active = active;
   c.dt_cur = active ? dt : 0.0;
+  c.dt_pair = float_pair(c.dt_cur);
   if (active) {
     c.t = __dadd_rn(c.t, dt);
     c.step = c.step + 1;

@@ -33,7 +33,14 @@ struct StepCtrl {
   int mode;            // 0: dt = dt_given; 1: CFL dt, loop bound t + eps < tend
   int err;             // sticky: bit0 non-finite/negative state seen, bit1 a bounded wait (TMA staging) gave up
   int q_valid;         // the primitive copy of the state (2-D RK2 handles) matches it
+  float2 dt_pair;      // dt_cur as a (hi, lo) pair, for the marched FP32-mixed kernels
 };
+
+// x as hi + lo, hi = RN(x) in FP32.
+__host__ __device__ inline float2 float_pair(double x) {
+  const float hi = (float)x;
+  return make_float2(hi, (float)(x - (double)hi));
+}
 
 // Programmatic dependent launch (PTX griddepcontrol) for the kernels of the
 // step loop: each waits for the previous kernel of the stream to complete

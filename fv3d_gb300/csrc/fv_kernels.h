@@ -169,6 +169,8 @@ struct BatchInst {
   int tiles_y;  // tiles along b (3-D: column blocks along y)
   int tz;       // 3-D: z layers per work item (work item = column block x z chunk)
   int pad;
+  // Factors of the marched FP32-mixed kernels as (hi, lo) pairs, per axis x, y, z.
+  float2 inv_d[3], mu_d[3], kappa_d2[3];  // 1/d, mu/d, kappa/d^2
 };
 
 // Tile shapes the autotuner chooses from (cells along a x along b).

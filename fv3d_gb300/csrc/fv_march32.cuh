@@ -5,20 +5,23 @@
 // walks it row by row with the whole stencil in registers: the
 // b-direction differences, face states and fluxes are carried from row to
 // row, the a-direction neighbours come by warp shuffles.  Slopes are formed
-// once per cell and direction and every face is solved once; the conductive
-// and viscous fluxes are added to the face's hydrodynamic flux (scaled by
-// dt/d) before the flux difference is taken.  No shared memory, no barrier.
+// once per cell and direction and every face is solved once.  The conductive
+// and viscous fluxes are carried beside the hydrodynamic ones and differenced
+// on their own: added to a flux they would be rounded to the ulp of its
+// pressure, and so would a flux scaled by dt/d before the difference (RT with
+// conduction and viscosity 300x327, 64 steps: the error of w against FP64 was
+// 1.8 times as large).  No shared memory, no barrier.
 //
 // Bound by instruction issue, as the block form (fv_tile32.cuh) it replaces,
-// but with 21 (stage 1) and 25 (stage 2) warp instructions per cell with
+// but with 21 (stage 1) and 26 (stage 2) warp instructions per cell with
 // conduction and viscosity against 38 and 43: the block form forms each slope
 // and reads each primitive of a face twice, evaluates every viscous face from
 // both cells, and keeps the whole CTA at three barriers a block.  Four of 32
 // lanes only serve their neighbours (a strip as wide as the warp needs its
 // ghosts); two columns per lane (60 of 64 useful) took 255 registers and
-// measured the same.  A step, block form -> this: shear 4096^2 1,259 -> 775 us
-// (13.3 -> 21.6 G cell-updates/s), RT 512x1536 51.0 -> 40.8 us, 64 Sod / Sedov
-// problems of 64^2..256^2 130.6 -> 90.4 us, Sedov 256^2 13.2 -> 13.0 us.
+// measured the same.  A step, block form -> this: shear 4096^2 1,259 -> 795 us
+// (13.3 -> 21.1 G cell-updates/s), RT 512x1536 51.0 -> 41.1 us, 64 Sod / Sedov
+// problems of 64^2..256^2 130.6 -> 91 us, Sedov 256^2 13.2 -> 12.8 us.
 //
 // The arithmetic is that of the mixed form (fv_tile32.cuh): U^n as (hi, lo)
 // pairs, U* in FP32 with its internal energy, the pressure recovery in
@@ -48,6 +51,15 @@ __device__ __forceinline__ float sqrt_(float x) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+
+// a * b of (hi, lo) pairs, as a pair and rounded to FP32.
+__device__ __forceinline__ float2 mul_pair(float2 a, float2 b) {
+  const float p = mul(a.x, b.x);
+  return make_float2(p, add(fma_(a.x, b.x, -p), fma_(a.x, b.y, mul(a.y, b.x))));
+}
+__device__ __forceinline__ float mul_to(float2 a, float2 b) {
+  return fma_(a.x, b.x, fma_(a.x, b.y, mul(a.y, b.x)));
 }
 
 // minmod (Update.h:73-80) as the median of (a, b, 0): the argument of smaller
@@ -180,7 +192,7 @@ constexpr int kMarchWidth = 28;
 // buffer and writes the other's (flip: B -> A).  The CFL maximum and the
 // non-finite flag of the result are folded into red / bad.
 template <int PLANE, bool WACT, int KIND>
-__device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float dt, int x0, int ya, int yb,
+__device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float2 dtp, int x0, int ya, int yb,
                                              float& red, bool& bad) {
   using namespace m32;
   constexpr bool STAR = KIND == STAGE_RK_2;  // the stage input is U*
@@ -193,7 +205,12 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
   const bool tc = G.tc != 0, visc = WACT && G.visc != 0, grav = PLANE == PLANE_XZ && G.gravity != 0;
   const float gamma = G.gamma_f, gm1 = G.gm1_f, inv_gm1 = G.inv_gm1_f;
   const float odx = G.inv_dx_f, odb = PLANE == PLANE_XY ? G.inv_dy_f : G.inv_dz_f;
-  const float dtdx = mul(dt, odx), dtdb = mul(dt, odb);
+  // the factors every cell shares are products of pairs, rounded once: their
+  // errors, unlike a cell's, act the same way everywhere and in every step
+  // (pairs, because the FP64 pipe takes 19 cycles a warp for each operation:
+  // formed there they cost 8 us a step of 24^3)
+  constexpr int B = PLANE == PLANE_XY ? 1 : 2;
+  const float dt = dtp.x, dtdx = mul_to(dtp, I.inv_d[0]), dtdb = mul_to(dtp, I.inv_d[B]);
 
   const int x = x0 - 2 + lane;
   bool fa;
@@ -231,8 +248,8 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
   float T0, T1;        // their temperatures
   float d[5];          // q1 - q0
   float Ls[5];         // face state of row j towards row j+1
-  float Hb[5];         // scaled flux of face j-1/2 as cell j sees it
-  float duA[5];        // increment of row j from the a faces and the per-cell terms
+  float Fb[5];         // hydrodynamic flux of face j-1/2
+  float duA[5];        // increment of row j from the a faces, the diffusive flux of face j-1/2 and the per-cell terms
   float Fx[4];         // a-direction neighbour terms of row j (viscosity)
   bool fbn;
   float2 raw[5];
@@ -248,18 +265,28 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     if (WACT || v != 3) d[v] = sub(q1[v], q0[v]);
-    Ls[v] = Hb[v] = duA[v] = 0.0f;
+    Ls[v] = Fb[v] = duA[v] = 0.0f;
     if (v < 4) Fx[v] = 0.0f;
   }
 
   // viscous and conductive constants, dt, mu and kappa folded in
-  const float mdt = visc ? mul(G.mu_f, dt) : 0.0f;
-  const float vx1 = mul(mdt, odx), vx43 = mul(4.0f / 3.0f, vx1);
-  const float vb1 = mul(mdt, odb), vb43 = mul(4.0f / 3.0f, vb1);
-  const float cx = mul(0.25f, vx1), cx23 = mul(2.0f / 3.0f, cx);
-  const float cb = mul(0.25f, vb1), cb23 = mul(2.0f / 3.0f, cb);
-  const float ktx = tc ? mul(mul(G.kappa_f, dtdx), odx) : 0.0f;
-  const float ktb = tc ? mul(mul(G.kappa_f, dtdb), odb) : 0.0f;
+  float vx1 = 0.0f, vx43 = 0.0f, vb1 = 0.0f, vb43 = 0.0f, cx23 = 0.0f, cb23 = 0.0f, ktx = 0.0f, ktb = 0.0f;
+  if (visc) {
+    const float2 k43 = make_float2((float)(4.0 / 3.0), (float)(4.0 / 3.0 - (double)(float)(4.0 / 3.0)));
+    const float2 k16 = make_float2((float)(1.0 / 6.0), (float)(1.0 / 6.0 - (double)(float)(1.0 / 6.0)));
+    const float2 vx = mul_pair(dtp, I.mu_d[0]), vb = mul_pair(dtp, I.mu_d[B]);
+    vx1 = add(vx.x, vx.y);
+    vb1 = add(vb.x, vb.y);
+    vx43 = mul_to(vx, k43);
+    vb43 = mul_to(vb, k43);
+    cx23 = mul_to(vx, k16);
+    cb23 = mul_to(vb, k16);
+  }
+  const float cx = mul(0.25f, vx1), cb = mul(0.25f, vb1);
+  if (tc) {
+    ktx = mul_to(dtp, I.kappa_d2[0]);
+    ktb = mul_to(dtp, I.kappa_d2[B]);
+  }
 
   // one row: j - 2 .. ya - 1 only build up the carried state
 #pragma unroll 1
@@ -302,53 +329,54 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
         FxN[3] = sub(q1[2], dl[2]);
       }
     }
-    float duN[5], HbN[5], Hup[5];
+    float duN[5], FbN[5], VbN[5], Vup[5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) duN[v] = HbN[v] = Hup[v] = 0.0f;
+    for (int v = 0; v < 5; ++v) duN[v] = FbN[v] = VbN[v] = Vup[v] = 0.0f;
     if (j >= ya - 1) {
-      // ---- a faces of row j + 1: each lane the one right of its column
-      float Ha[5];
-      {
-        float L[5], R[5];
-        FV_EACH_V(v) {
-          const float s = plm ? minmod(dl[v], dR[v]) : 0.0f;
-          L[v] = fma_(0.5f, s, q1[v]);
-          R[v] = __shfl_down_sync(kAll, fma_(-0.5f, s, q1[v]), 1);
+      // ---- a faces of row j + 1 (row yb is another item's): each lane the one right of its column
+      if (j + 1 < yb) {
+        float Fa[5], Va[5];
+        {
+          float L[5], R[5];
+          FV_EACH_V(v) {
+            const float s = plm ? minmod(dl[v], dR[v]) : 0.0f;
+            L[v] = fma_(0.5f, s, q1[v]);
+            R[v] = __shfl_down_sync(kAll, fma_(-0.5f, s, q1[v]), 1);
+          }
+          riemann<PLANE, 0, WACT>(rs, L, R, gamma, inv_gm1, Fa);
         }
-        riemann<PLANE, 0, WACT>(rs, L, R, gamma, inv_gm1, Ha);
-        FV_EACH_V(v) Ha[v] = mul(Ha[v], dtdx);
-      }
-      if (tc) Ha[4] = fma_(-ktx, sub(__shfl_down_sync(kAll, T1, 1), T1), Ha[4]);
-      float z1 = 0.0f, z3 = 0.0f;
-      if (visc) {
-        // e: difference over rows j, j+2 of the velocities; IX fluxes take the
-        // in-plane pair (u, v) or (u, w) (slots 1, 2), the x-y IZ terms (u, w)
-        const float e0 = sub(qn[1], q0[1]), e1 = sub(qn[2], q0[2]);
-        const float s0 = add(e0, __shfl_down_sync(kAll, e0, 1));
-        const float s1 = add(e1, __shfl_down_sync(kAll, e1, 1));
-        const float ta = fma_(vx43, dR[1], -mul(cb23, s1));
-        const float tb = fma_(vx1, dR[2], mul(cb, s0));
-        const float tw = mul(vx1, dR[3]);
-        // the face's mean velocities: q + dR / 2
-        const float ma = fma_(0.5f, dR[1], q1[1]), mb = fma_(0.5f, dR[2], q1[2]), mw = fma_(0.5f, dR[3], q1[3]);
-        Ha[1] = sub(Ha[1], ta);
-        Ha[2] = sub(Ha[2], tb);
-        Ha[3] = sub(Ha[3], tw);
-        Ha[4] = sub(Ha[4], fma_(ta, ma, fma_(tb, mb, mul(tw, mw))));
-        if (PLANE == PLANE_XY) {
-          // the IZ branch (Viscosity.h:214-239) in an x-y run: its two sides
-          // differ only in the rows of the left column
-          z1 = -mul(cx, __shfl_up_sync(kAll, sub(qn[3], q0[3]), 1));
-          z3 = mul(cx23, __shfl_up_sync(kAll, e0, 1));
+        FV_EACH_V(v) duN[v] = mul(dtdx, sub(__shfl_up_sync(kAll, Fa[v], 1), Fa[v]));
+        Va[4] = tc ? mul(ktx, sub(__shfl_down_sync(kAll, T1, 1), T1)) : 0.0f;
+        float z1 = 0.0f, z3 = 0.0f;
+        if (visc) {
+          // e: difference over rows j, j+2 of the velocities; IX fluxes take the
+          // in-plane pair (u, v) or (u, w) (slots 1, 2), the x-y IZ terms (u, w)
+          const float e0 = sub(qn[1], q0[1]), e1 = sub(qn[2], q0[2]);
+          const float s0 = add(e0, __shfl_down_sync(kAll, e0, 1));
+          const float s1 = add(e1, __shfl_down_sync(kAll, e1, 1));
+          Va[1] = fma_(vx43, dR[1], -mul(cb23, s1));
+          Va[2] = fma_(vx1, dR[2], mul(cb, s0));
+          Va[3] = mul(vx1, dR[3]);
+          // the face's mean velocities: q + dR / 2
+          const float ma = fma_(0.5f, dR[1], q1[1]), mb = fma_(0.5f, dR[2], q1[2]), mw = fma_(0.5f, dR[3], q1[3]);
+          Va[4] = fma_(Va[1], ma, fma_(Va[2], mb, fma_(Va[3], mw, Va[4])));
+#pragma unroll
+          for (int v = 1; v < 4; ++v) duN[v] = add(duN[v], sub(Va[v], __shfl_up_sync(kAll, Va[v], 1)));
+          if (PLANE == PLANE_XY) {
+            // the IZ branch (Viscosity.h:214-239) in an x-y run: its two sides
+            // differ only in the rows of the left column
+            z1 = -mul(cx, __shfl_up_sync(kAll, sub(qn[3], q0[3]), 1));
+            z3 = mul(cx23, __shfl_up_sync(kAll, e0, 1));
+          }
         }
+        if (tc || visc) duN[4] = add(duN[4], sub(Va[4], __shfl_up_sync(kAll, Va[4], 1)));
+        if (PLANE == PLANE_XY && visc) {
+          duN[1] = add(duN[1], z1);
+          duN[3] = add(duN[3], z3);
+          duN[4] = add(duN[4], fma_(z1, q1[1], mul(z3, q1[3])));
+        }
+        if (grav) duN[2] = fma_(mul(dt, G.g_f), q1[0], duN[2]);
       }
-      FV_EACH_V(v) duN[v] = sub(__shfl_up_sync(kAll, Ha[v], 1), Ha[v]);
-      if (PLANE == PLANE_XY && visc) {
-        duN[1] = add(duN[1], z1);
-        duN[3] = add(duN[3], z3);
-        duN[4] = add(duN[4], fma_(z1, q1[1], mul(z3, q1[3])));
-      }
-      if (grav) duN[2] = fma_(mul(dt, G.g_f), q1[0], duN[2]);
       // ---- b face between rows j and j + 1
       {
         float R[5];
@@ -357,21 +385,17 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
           Ls[4] = fma_(mul(Ls[0], G.g_dz_f), 0.5f, Ls[4]);
           R[4] = fma_(mul(R[0], G.g_dz_f), -0.5f, R[4]);
         }
-        riemann<PLANE, 1, WACT>(rs, Ls, R, gamma, inv_gm1, HbN);
-        FV_EACH_V(v) HbN[v] = mul(HbN[v], dtdb);
+        riemann<PLANE, 1, WACT>(rs, Ls, R, gamma, inv_gm1, FbN);
       }
-      if (tc) HbN[4] = fma_(-ktb, sub(T1, T0), HbN[4]);
+      if (tc) VbN[4] = mul(ktb, sub(T1, T0));
       if (visc && PLANE == PLANE_XY) {  // IY (Viscosity.h:188-213)
         const float ma = fma_(0.5f, d[1], q0[1]), mb = fma_(0.5f, d[2], q0[2]), mw = fma_(0.5f, d[3], q0[3]);
-        const float ta = fma_(vb1, d[1], mul(cx, add(Fx[1], FxN[1])));
-        const float tb = fma_(vb43, d[2], -mul(cx23, add(Fx[0], FxN[0])));
-        const float tw = mul(vb1, d[3]);
-        HbN[1] = sub(HbN[1], ta);
-        HbN[2] = sub(HbN[2], tb);
-        HbN[3] = sub(HbN[3], tw);
-        HbN[4] = sub(HbN[4], fma_(ta, ma, fma_(tb, mb, mul(tw, mw))));
+        VbN[1] = fma_(vb1, d[1], mul(cx, add(Fx[1], FxN[1])));
+        VbN[2] = fma_(vb43, d[2], -mul(cx23, add(Fx[0], FxN[0])));
+        VbN[3] = mul(vb1, d[3]);
+        VbN[4] = fma_(VbN[1], ma, fma_(VbN[2], mb, fma_(VbN[3], mw, VbN[4])));
       }
-      FV_EACH_V(v) Hup[v] = HbN[v];
+      FV_EACH_V(v) Vup[v] = VbN[v];
       if (visc && PLANE == PLANE_XZ) {
         // IZ with the reference's mix-ups: both cells of the face read their own left column
         const float ma = fma_(0.5f, d[1], q0[1]), mb = fma_(0.5f, d[2], q0[2]), mw = fma_(0.5f, d[3], q0[3]);
@@ -381,22 +405,30 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
         const float tyz = fma_(vb1, d[3], -mul(cb, wv));
 #pragma unroll
         for (int k = 0; k < 2; ++k) {  // cell j (its upper face), cell j + 1 (its lower face)
-          float* H = k == 0 ? Hup : HbN;
+          float* V = k == 0 ? Vup : VbN;
           const float zz = fma_(add(cx23, cx23), k == 0 ? Fx[2] : FxN[2], tzz);
           const float xz = fma_(-add(cx, cx), k == 0 ? Fx[3] : FxN[3], txz);
-          H[1] = sub(H[1], xz);
-          H[2] = sub(H[2], zz);
-          H[3] = sub(H[3], tyz);
-          H[4] = sub(H[4], fma_(xz, ma, fma_(tyz, mw, mul(zz, mb))));
+          V[1] = xz;
+          V[2] = zz;
+          V[3] = tyz;
+          V[4] = fma_(xz, ma, fma_(tyz, mw, fma_(zz, mb, V[4])));
         }
       }
+      if (visc) {
+#pragma unroll
+        for (int v = 1; v < 4; ++v) duN[v] = sub(duN[v], VbN[v]);
+      }
+      if (tc || visc) duN[4] = sub(duN[4], VbN[4]);
     }
     // ---- row j: increments, accumulation on the pairs, CFL term
     if (own && j >= ya) {
       float du[5];
-      FV_EACH_V(v) du[v] = add(duA[v], sub(Hb[v], Hup[v]));
-      if (grav)  // half the mass fluxes of both faces (Update.h:150); Hb[0] = F dt / db
-        du[4] = fma_(mul(0.5f, G.g_dz_f), add(Hb[0], Hup[0]), du[4]);
+      FV_EACH_V(v) {
+        du[v] = fma_(dtdb, sub(Fb[v], FbN[v]), duA[v]);
+        if (v == 4 ? tc || visc : v > 0 && visc) du[v] = add(du[v], Vup[v]);
+      }
+      if (grav)  // half the mass fluxes of both faces (Update.h:150)
+        du[4] = fma_(mul(mul(0.5f, dt), G.g_f), add(Fb[0], FbN[0]), du[4]);
       // density floor on the hydro update (Update.h:160)
       const bool low = (STAR ? add(us[0], du[0]) : add(add(un[0].x, du[0]), un[0].y)) < 1.0e-6f;
       if (KIND == STAGE_RK_1) {
@@ -456,7 +488,7 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
     for (int v = 0; v < 5; ++v) {
       if (v == 3 && !WACT) continue;
       Ls[v] = fma_(0.5f, m[v], q1[v]);
-      Hb[v] = HbN[v];
+      Fb[v] = FbN[v];
       duA[v] = duN[v];
       q0[v] = q1[v];
       q1[v] = qn[v];
@@ -474,13 +506,10 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
 
 constexpr int kMarchWarps = 4;  // warps (work items in flight) per CTA
 constexpr int kMarchThreads = 32 * kMarchWarps;
-// Resident CTAs per SM asked of the register allocator: 4 (128 registers a
-// thread, 16 warps per SM) but 5 (96) where the descriptor sits in the
-// parameters and three momenta are carried: shear 4096^2 775 us a step
-// against 793 with 4; RT 512x1536 (two momenta) 43.5 against 40.8, its rows
-// then split into shorter items.
-template <bool WACT, bool ONE>
-constexpr int kMarchCtas = WACT && ONE ? 5 : 4;
+// Resident CTAs per SM asked of the register allocator: 128 registers a
+// thread, 16 warps per SM.  Five CTAs (96 registers) measured 824 us a step
+// against 810 on shear 4096^2 and the same on RT 512x1536.
+constexpr int kMarchCtas = 4;
 
 // Copies the descriptor of the problem holding work item t to the warp's slot
 // (binary search over the first items) unless it is there already.
@@ -506,7 +535,7 @@ __device__ __forceinline__ int march_fetch(const BatchInst* __restrict__ insts, 
 // stage by the calling warp.  active / dt_step: the problem's step in flight;
 // slot_next / err: its CFL maximum slot for the next step and its error flag.
 template <int PLANE, bool WACT, int KIND>
-__device__ __forceinline__ void march_stage_item(const BatchInst& I, int t, int flip, bool active, double dt_step,
+__device__ __forceinline__ void march_stage_item(const BatchInst& I, int t, int flip, bool active, float2 dt_step,
                                                  unsigned long long* slot_next, int* err) {
   constexpr int W = kMarchWidth;
   const int lane = threadIdx.x & 31;
@@ -533,7 +562,7 @@ __device__ __forceinline__ void march_stage_item(const BatchInst& I, int t, int 
   }
   float red = 0.0f;
   bool bad = false;
-  march_item32<PLANE, WACT, KIND>(I, flip, (float)dt_step, x0, ya, yb, red, bad);
+  march_item32<PLANE, WACT, KIND>(I, flip, dt_step, x0, ya, yb, red, bad);
   if (KIND != STAGE_RK_1) {
     // non-negative floats order like their bits
     const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(red));
@@ -550,7 +579,7 @@ __device__ __forceinline__ void march_stage_item(const BatchInst& I, int t, int 
 // ONE: a group of one problem, whose descriptor `one` is read from the
 // kernel's parameters (constant operands in place of registers and loads).
 template <int PLANE, bool WACT, int KIND, bool ONE>
-__global__ void __launch_bounds__(kMarchThreads, kMarchCtas<WACT, ONE>)
+__global__ void __launch_bounds__(kMarchThreads, kMarchCtas)
 march_stage32(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsigned* queue, int flip,
               const __grid_constant__ BatchInst one) {
   __shared__ BatchInst s_inst[ONE ? 1 : kMarchWarps];
@@ -568,7 +597,7 @@ march_stage32(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsign
     }
     if (!ONE) have = march_fetch(insts, ninst, t, have, &slot);
     StepCtrl* ctrl = I.ctrl;
-    march_stage_item<PLANE, WACT, KIND>(I, t, flip, ctrl->active != 0, ctrl->dt_cur,
+    march_stage_item<PLANE, WACT, KIND>(I, t, flip, ctrl->active != 0, ctrl->dt_pair,
                                            &ctrl->slot[ctrl->parity ^ 1], &ctrl->err);
   }
 }
@@ -590,11 +619,12 @@ constexpr int kMultiMaxProblems = 256;
 // barrier wait that runs out sets bit 1 of every problem's error flag and
 // the kernel returns.
 template <int PLANE, bool WACT, bool ONE>
-__global__ void __launch_bounds__(kMarchThreads, 4)
+__global__ void __launch_bounds__(kMarchThreads, kMarchCtas)
 march_multi32(const BatchInst* __restrict__ insts, int ninst, int ntiles, int nsteps, int mode_override,
               GridBarrier gb, const __grid_constant__ BatchInst one) {
   __shared__ BatchInst s_inst[ONE ? 1 : kMarchWarps];
   __shared__ double s_t[kMultiMaxProblems], s_dt[kMultiMaxProblems];
+  __shared__ float2 s_dtp[kMultiMaxProblems];  // the same as pairs
   __shared__ long long s_step[kMultiMaxProblems];
   __shared__ int s_act[kMultiMaxProblems], s_par[kMultiMaxProblems], s_err[kMultiMaxProblems];
   __shared__ int s_any;
@@ -632,6 +662,7 @@ march_multi32(const BatchInst* __restrict__ insts, int ninst, int ntiles, int ns
       const int p = (int)(s_step[m] & 1);
       if (bad) s_err[m] = 1;
       s_dt[m] = active ? dt : 0.0;
+      s_dtp[m] = float_pair(s_dt[m]);
       s_act[m] = active;
       s_par[m] = p;
       if (blockIdx.x == 0) c->slot[p ^ 1] = 0ull;  // read by no CTA in this step
@@ -646,7 +677,7 @@ march_multi32(const BatchInst* __restrict__ insts, int ninst, int ntiles, int ns
     if (!s_any) break;  // every CTA decides alike: no problem steps any more
     for (int t = warp0; t < ntiles; t += nwarps) {
       const int m = have = ONE ? 0 : march_fetch(insts, ninst, t, have, &slot);
-      march_stage_item<PLANE, WACT, STAGE_RK_1>(I, t, 0, s_act[m] != 0, s_dt[m], nullptr, nullptr);
+      march_stage_item<PLANE, WACT, STAGE_RK_1>(I, t, 0, s_act[m] != 0, s_dtp[m], nullptr, nullptr);
     }
     if (!grid_sync(gb, bar++)) {
       timed_out();
@@ -655,7 +686,7 @@ march_multi32(const BatchInst* __restrict__ insts, int ninst, int ntiles, int ns
     for (int t = warp0; t < ntiles; t += nwarps) {
       const int m = have = ONE ? 0 : march_fetch(insts, ninst, t, have, &slot);
       StepCtrl* ctrl = I.ctrl;
-      march_stage_item<PLANE, WACT, STAGE_RK_2>(I, t, 0, s_act[m] != 0, s_dt[m], &ctrl->slot[s_par[m] ^ 1],
+      march_stage_item<PLANE, WACT, STAGE_RK_2>(I, t, 0, s_act[m] != 0, s_dtp[m], &ctrl->slot[s_par[m] ^ 1],
                                                    &ctrl->err);
     }
     if (!grid_sync(gb, bar++)) {
@@ -670,6 +701,7 @@ march_multi32(const BatchInst* __restrict__ insts, int ninst, int ntiles, int ns
         c->parity = s_par[m];
         c->active = s_act[m];
         c->dt_cur = s_dt[m];
+        c->dt_pair = s_dtp[m];
       }
       c->t = s_t[m];
       c->step = s_step[m];
