@@ -53,6 +53,7 @@ constexpr int kMultiChunk = 256;  // steps per multi-step launch of a loop with 
 
 struct Group {
   int ndim = 2;     // 3: 3-D problems (one kernel shape, grouped by solver)
+  bool march = false;  // FP32-mixed 3-D: the z-marched form (every member is one it runs)
   int rs = -1;      // 3-D groups: the shared Riemann solver (bit 0) and corrected physics (bit 1)
   int plane = 0;
   bool wact = false;
@@ -227,7 +228,7 @@ std::string GroupKey(const fv_batch* b, const Group& g) {
   }
   std::ostringstream k;
   // k2: the generation of the stage kernels; a choice tuned on others is not taken over
-  k << "p" << b->precision << "k2_d" << g.ndim << "_co" << (g.rs >= 2) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
+  k << "p" << b->precision << "k2" << (g.march ? "m" : "") << "_d" << g.ndim << "_co" << (g.rs >= 2) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
     << rs_mask << "_ts" << b->ts << "_n" << g.members.size() << "_c" << cells << "_h" << std::hex << h;
   return k.str();
 }
@@ -254,10 +255,42 @@ Schedule ShapeSchedule(const fv_batch* b, int shape) {
   return sc;
 }
 
-// The schedule of a 3-D group: 16 x 16 column blocks, z layers per work item;
-// the FP64 kernel shares the x / y faces' viscous fluxes.
-Schedule Schedule3d(const fv_batch* b, int layers) {
+// The sides of a 3-D group's column blocks (the most, for the z-marched form).
+void Block3d(const Group& g, int* cols, int* rows) {
+  if (g.march) fv::march3d_block(cols, rows);
+  else *cols = *rows = fv::batch3d_columns();
+}
+
+bool Viscous(const fv_batch* b, const Group& g) {
+  for (int i : g.members)
+    if (b->G[i].visc) return true;
+  return false;
+}
+
+// Whether the z-marched FP32-mixed form runs problem i: not the z-boundary
+// physics (C91, well-balanced fluxes, fixed conduction boundaries) and not the
+// corrected physics, which only the block form has; and not plain Euler steps
+// without slopes, whose layers are too cheap to hide its barrier (blast 256^3
+// 782 us a step against 712 with the block form; with slopes, two stages,
+// conduction or viscosity it is the faster one: 192^3 PLM Euler 377 against
+// 409, PCM RK2 561 / 616, PLM RK2 596 / 749, with both terms 765 / 1,000).
+bool Marched3d(const fv_batch* b, int i) {
+  const Grid& G = b->G[i];
+  if (b->ts != FV_TS_RK2 && G.recon != fv::R_PLM && !G.tc && !G.visc) return false;
+  return b->precision != FV_PREC_FP64 && G.ndim == 3 && G.bc_c != fv::DBC_C91 && !G.wb_flux_z && !G.corrected &&
+         !(G.tc && (G.bctc_zmin != FV_BCTC_NONE || G.bctc_zmax != FV_BCTC_NONE));
+}
+
+// The schedule of a 3-D group: blocks of 16 x 16 columns (30 x 15 in the
+// z-marched form), z layers per work item; the FP64 kernel shares the x / y
+// faces' viscous fluxes.
+Schedule Schedule3d(const fv_batch* b, const Group& g, int layers) {
   Schedule sc;
+  if (g.march) {
+    fv::march3d_block(&sc.tx, &sc.block_rows);
+    sc.rows = layers > 0 ? layers : 16;
+    return sc;
+  }
   sc.tx = fv::batch3d_columns();
   sc.rows = layers > 0 ? layers : 16;
   sc.block_rows = 0;
@@ -275,6 +308,9 @@ int ItemsPerCta(const fv_batch* b, const Group& g, int shape) {
 int GridFor(const fv_batch* b, const Group& g, int shape, int occupancy, int ntiles);
 
 int Occupancy(const fv_batch* b, const Group& g, int shape) {
+  if (g.march)
+    return fv::march3d_occupancy(b->ts == FV_TS_RK2 ? fv::STAGE_RK_2 : fv::STAGE_EULER, Viscous(b, g),
+                                 g.members.size() == 1);
   if (g.ndim == 3)
     return b->precision == FV_PREC_FP64 ? fv::batch_stage3d_occupancy64(g.rs, g.tc)
                                         : fv::batch_stage3d_occupancy32(g.rs, g.tc);
@@ -288,6 +324,9 @@ int Occupancy(const fv_batch* b, const Group& g, int shape) {
 // one: the host copy of insts[0] (used when the group has one problem).
 cudaError_t LaunchStage(const fv_batch* b, const Group& g, const BatchInst* insts, const BatchInst* one, int ntiles,
                         int grid, unsigned* queue, int kind, int flip) {
+  if (g.march)
+    return fv::launch_march3d32(insts, (int)g.members.size(), ntiles, queue, kind, flip, Viscous(b, g), grid, b->stream,
+                                g.members.size() == 1 ? one : nullptr);
   if (g.ndim == 3)
     return b->precision == FV_PREC_FP64
                ? fv::launch_batch_stage3d64(insts, (int)g.members.size(), ntiles, queue, kind, flip, g.rs, grid, g.tc,
@@ -309,8 +348,8 @@ std::vector<BatchInst> Describe(const fv_batch* b, const Group& g, int shape, St
                                 int rows = 0) {
   const fv::TileShape* shapes;
   NumShapes(b->precision, &shapes);
-  const int tx = g.ndim == 3 ? fv::batch3d_columns() : shapes[shape].tx;
-  const int ty = g.ndim == 3 ? fv::batch3d_columns() : (rows > 0 ? rows : shapes[shape].ty);
+  int tx = shapes[shape].tx, ty = rows > 0 ? rows : shapes[shape].ty;
+  if (g.ndim == 3) Block3d(g, &tx, &ty);
   std::vector<BatchInst> out;
   int t0 = 0;
   for (int i : g.members) {
@@ -387,7 +426,11 @@ int Autotune(fv_batch* b, Group& g) {
   // the first shape of a kernel (it serves every row count): strip width,
   // block rows and viscous form
   auto shape_of = [&](const Schedule& sc) {
-    if (d3) return sc.tx == fv::batch3d_columns() ? 0 : -1;
+    if (d3) {
+      int cols, rows;
+      Block3d(g, &cols, &rows);
+      return sc.tx == cols ? 0 : -1;
+    }
     for (int s = 0; s < ns; ++s) {
       const Schedule k = ShapeSchedule(b, s);
       if (k.tx == sc.tx && k.block_rows == sc.block_rows && k.vface == sc.vface && Occupancy(b, g, s) > 0) return s;
@@ -409,8 +452,9 @@ int Autotune(fv_batch* b, Group& g) {
       char* r = rest;
       if (*r == '/') sc.block_rows = (int)std::strtol(r + 1, &r, 10);
       sc.vface = *r == 'v' ? 1 : 0;
-      if (d3) {
-        sc = Schedule3d(b, sc.rows);
+      if (d3) {  // 16 forces the block form, 30 the z-marched one
+        if (sc.tx == fv::batch3d_columns()) g.march = false;
+        sc = Schedule3d(b, g, sc.rows);
       } else if (b->precision == FV_PREC_FP64) {  // one kernel per strip width
         const int rows = sc.rows;
         for (int s = 0; s < ns; ++s)
@@ -439,11 +483,12 @@ int Autotune(fv_batch* b, Group& g) {
     // and the chunk lengths that make the work items fill 1-4 rounds of the
     // resident CTAs (the fewest layers with at most r rounds of items)
     const long long slots = (long long)Occupancy(b, g, 0) * SmCount();
-    const int side = fv::batch3d_columns();
+    int cols, rows;
+    Block3d(g, &cols, &rows);
     auto items = [&](int z) {
       long long n = 0;
       for (int i : g.members)
-        n += (long long)((b->G[i].na + side - 1) / side) * ((b->G[i].nb + side - 1) / side) *
+        n += (long long)((b->G[i].na + cols - 1) / cols) * ((b->G[i].nb + rows - 1) / rows) *
              ((b->G[i].nc + z - 1) / z);
       return n;
     };
@@ -563,7 +608,7 @@ int Autotune(fv_batch* b, Group& g) {
   const bool log = std::getenv("FV3D_TILE_LOG") != nullptr;
   for (size_t c = 0; c < cand.size(); ++c) {
     if (log) {
-      const Schedule k = d3 ? Schedule3d(b, cand[c].second) : ShapeSchedule(b, cand[c].first);
+      const Schedule k = d3 ? Schedule3d(b, g, cand[c].second) : ShapeSchedule(b, cand[c].first);
       std::fprintf(stderr, "fv3d tile candidate %dx%d/%d%s: %.4f ms (%d items, %d CTAs)\n", k.tx, cand[c].second,
                    k.block_rows, k.vface ? "v" : "", grid[c] ? best_ms[c] : -1.0f, ntiles[c], grid[c]);
     }
@@ -588,7 +633,7 @@ int Autotune(fv_batch* b, Group& g) {
   cudaEventDestroy(e1);
   if (best_c < 0) return Fail(b, FV_ERR_CUDA, "no tile shape could be launched for a batch group");
   std::lock_guard<std::mutex> lock(g_cache_mutex);
-  Schedule chosen = d3 ? Schedule3d(b, g.rows) : ShapeSchedule(b, g.shape);
+  Schedule chosen = d3 ? Schedule3d(b, g, g.rows) : ShapeSchedule(b, g.shape);
   chosen.rows = g.rows;
   g_cache[key] = chosen;
   SaveCacheEntry(key, chosen);
@@ -627,6 +672,7 @@ int Prepare(fv_batch* b) {
       g->plane = b->G[i].plane;
       g->wact = b->wact[i];
     }
+    g->march = ndim == 3 && Marched3d(b, i) && (g->members.empty() || g->march);
     g->members.push_back(i);
     g->tc = g->tc || b->G[i].tc;
   }
@@ -1106,8 +1152,8 @@ int fvgpu_batch_schedule(fv_batch* b, int* ngroups, int* tx, int* rows, int* blo
   for (int gi = 0; gi < *ngroups && gi < max_groups; ++gi) {
     const Group& g = b->groups[gi];
     Schedule sc;
-    if (g.ndim == 3) {  // column blocks of 16 x 16 marched over chunks of `rows` z layers
-      sc = Schedule3d(b, g.rows);
+    if (g.ndim == 3) {  // column blocks marched over chunks of `rows` z layers
+      sc = Schedule3d(b, g, g.rows);
     } else {
       sc = ShapeSchedule(b, g.shape);
       if (g.rows > 0) sc.rows = g.rows;
@@ -1130,10 +1176,11 @@ int fvgpu_batch_tiling(fv_batch* b, int* ngroups, int* tx, int* ty, int max_grou
   NumShapes(b->precision, &shapes);
   *ngroups = (int)b->groups.size();
   for (int g = 0; g < *ngroups && g < max_groups; ++g) {
-    const bool d3 = b->groups[g].ndim == 3;
-    if (tx) tx[g] = d3 ? fv::batch3d_columns() : shapes[b->groups[g].shape].tx;
-    if (ty) ty[g] = d3 ? fv::batch3d_columns()
-                       : (b->groups[g].rows > 0 ? b->groups[g].rows : shapes[b->groups[g].shape].ty);
+    const Group& gr = b->groups[g];
+    int cols = shapes[gr.shape].tx, rows = gr.rows > 0 ? gr.rows : shapes[gr.shape].ty;
+    if (gr.ndim == 3) Block3d(gr, &cols, &rows);
+    if (tx) tx[g] = cols;
+    if (ty) ty[g] = rows;
   }
   return FV_OK;
 }

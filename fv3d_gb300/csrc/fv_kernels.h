@@ -218,6 +218,15 @@ cudaError_t launch_batch_stage3d32(const BatchInst* insts, int ninst, int ntiles
 int batch_stage3d_occupancy64(int rs, bool tc);
 int batch_stage3d_occupancy32(int rs, bool tc);
 
+// The z-marched form of the FP32-mixed 3-D stage (fv_march3d32.cu): work items
+// are blocks of at most *cols x *rows columns (of equal size per problem,
+// numbered x fastest) and chunks of BatchInst::tz layers.  It runs everything
+// but the z-boundary physics and the corrected physics.
+int march3d_block(int* cols, int* rows);
+int march3d_occupancy(int kind, bool visc, bool one);
+cudaError_t launch_march3d32(const BatchInst* insts, int ninst, int ntiles, unsigned* queue, int kind, int flip, bool visc,
+                             int grid, cudaStream_t stream, const BatchInst* one);
+
 // Several RK2 steps of a group of FP32-mixed 2-D problems in one cooperative
 // launch (fv_march32.cuh, march_multi32; marched shapes only): for small
 // grids, whose steps are bound by launch latency.  At most

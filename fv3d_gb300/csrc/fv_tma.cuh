@@ -50,6 +50,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* m, uns
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(m)), "r"(bytes) : "memory");
 }
 
+// Arrives (release) for the calling thread and what it is ordered after.
+__device__ __forceinline__ void mbar_arrive(unsigned long long* m) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(m)) : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1,
                                             unsigned long long* m) {
   asm volatile(
