@@ -178,8 +178,19 @@ def read_ini(path):
     return p
 
 
+_double_at = C.c_double.from_address
+
+
 def _ptr(a):
-    return None if a is None else a.ctypes.data_as(_dp)
+    """double* of an array's data, which it keeps alive (ndarray.ctypes.data_as
+    takes about 2 us a call; an array of no elements keeps it)."""
+    if a is None:
+        return None
+    if not a.size:
+        return a.ctypes.data_as(_dp)
+    p = _dp(_double_at(a.__array_interface__["data"][0]))
+    p._arr = a
+    return p
 
 
 def _checked(a, shape):
@@ -194,6 +205,8 @@ def _checked(a, shape):
 def _as_field(a, shape):
     if a is None:
         return None
+    if type(a) is np.ndarray and a.dtype == np.float64 and a.shape == shape and a.flags.c_contiguous:
+        return a
     return np.ascontiguousarray(np.broadcast_to(np.asarray(a, dtype=np.float64), shape))
 
 
