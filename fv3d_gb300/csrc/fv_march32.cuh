@@ -506,10 +506,21 @@ __device__ __forceinline__ void march_item32(const BatchInst& I, int flip, float
 
 constexpr int kMarchWarps = 4;  // warps (work items in flight) per CTA
 constexpr int kMarchThreads = 32 * kMarchWarps;
-// Resident CTAs per SM asked of the register allocator: 128 registers a
-// thread, 16 warps per SM.  Five CTAs (96 registers) measured 824 us a step
-// against 810 on shear 4096^2 and the same on RT 512x1536.
-constexpr int kMarchCtas = 4;
+// Resident CTAs per SM asked of the register allocator: 4 (128 registers a
+// thread, 16 warps per SM; five CTAs and 96 registers measured 824 us a step
+// against 810 on shear 4096^2 and the same on RT 512x1536), but 3 where the x-z
+// plane's viscous fluxes and a descriptor in shared memory come together: 4
+// spill the row on its way, whose loads are then waited for at once (two RT
+// 1024x3072 with conduction and viscosity 464 us a step against 374; x-y, two
+// shear layers 2048^2, 456 against 471 with 3).
+template <int PLANE, bool WACT, bool ONE>
+constexpr int kMarchCtas = PLANE == PLANE_XZ && WACT && !ONE ? 3 : 4;
+
+// The multi-step kernel holds both stages and spilled 20-100 bytes at 4: 3 gives
+// four RT 128x384 with conduction and viscosity 23.7 us a step against 32.0, one
+// 12.7 / 14.4, three shear layers 256^2 22.7 / 27.0, one 512^2 25.2 / 24.9; the
+// hydro-only forms need no more than 128 registers and stay at 4 CTAs.
+constexpr int kMultiCtas = 3;
 
 // Copies the descriptor of the problem holding work item t to the warp's slot
 // (binary search over the first items) unless it is there already.
@@ -579,7 +590,7 @@ __device__ __forceinline__ void march_stage_item(const BatchInst& I, int t, int 
 // ONE: a group of one problem, whose descriptor `one` is read from the
 // kernel's parameters (constant operands in place of registers and loads).
 template <int PLANE, bool WACT, int KIND, bool ONE>
-__global__ void __launch_bounds__(kMarchThreads, kMarchCtas)
+__global__ void __launch_bounds__(kMarchThreads, (kMarchCtas<PLANE, WACT, ONE>))
 march_stage32(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsigned* queue, int flip,
               const __grid_constant__ BatchInst one) {
   __shared__ BatchInst s_inst[ONE ? 1 : kMarchWarps];
@@ -619,7 +630,7 @@ constexpr int kMultiMaxProblems = 256;
 // barrier wait that runs out sets bit 1 of every problem's error flag and
 // the kernel returns.
 template <int PLANE, bool WACT, bool ONE>
-__global__ void __launch_bounds__(kMarchThreads, kMarchCtas)
+__global__ void __launch_bounds__(kMarchThreads, kMultiCtas)
 march_multi32(const BatchInst* __restrict__ insts, int ninst, int ntiles, int nsteps, int mode_override,
               GridBarrier gb, const __grid_constant__ BatchInst one) {
   __shared__ BatchInst s_inst[ONE ? 1 : kMarchWarps];
