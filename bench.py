@@ -50,10 +50,10 @@ ALGO_BYTES_PER_CELL_UPDATE = 160  # 5 passes x 4 fields x 8 B (F = 4, inviscid 2
 NCU_TRAFFIC_BYTES_PER_STEP = 106.86e6
 # FP64 arithmetic lane operations (DFMA thread instructions; sums and products
 # are issued as DFMAs) per cell-update of this workload from an ncu capture
-# (stage 1: 262.6, stage 2: 301.7).  The FP64 kernel is bound by the FP64
+# (stage 1: 252.5, stage 2: 289.6).  The FP64 kernel is bound by the FP64
 # pipe: its roofline against the FP64 FMA rate measured live by
 # fvgpu_probe_fp64_rate.
-FP64_OPS_PER_CELL_UPDATE = 564
+FP64_OPS_PER_CELL_UPDATE = 542
 
 
 def peaks():

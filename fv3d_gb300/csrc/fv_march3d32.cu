@@ -21,10 +21,11 @@
 // as the block form (fv_stage3d32.cu) it replaces where it is the faster one:
 // that one forms each slope twice, reads every primitive of a face four times
 // and evaluates every viscous face from both cells (52 and 56 warp instructions
-// per cell against some 43 and 46 here).  192^3, RK2, a step: PLM with
+// per cell against some 44 and 46 here).  192^3, RK2, a step: PLM with
 // conduction and viscosity 1,000 -> 765 us, with conduction 829 -> 603, hydro
 // alone 749 -> 596, PCM with both 865 -> 736; 100x80x90, PLM with both 124 ->
 // 95; 24^3 55 -> 40.  Two CTAs of 8 warps (30 x 7 columns) measured 8 % slower,
+// one of 12 or 14 warps (168 or 144 registers, no spills) 19-21 % on 192^3,
 // prefetching the cells' own values of the update into L1 2 %, a barrier
 // without the split arrival 11 %.
 //

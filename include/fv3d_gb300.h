@@ -299,21 +299,25 @@ int fvgpu_batch_launch_count(const fv_batch* b, long* count);
 /* Problems sharing plane and layout form a group advanced by one persistent
  * launch per stage; reports the groups and the work-item shape the autotuner
  * chose for each: cells along x by rows along the second axis (a strip
- * segment; 3-D groups: 16 x 16 columns), tuning first if needed; every
- * problem must have a state.  The autotuner times one whole step of each
+ * segment; 3-D groups: blocks of at most 16 x 16 columns, 30 x 15 in the
+ * z-marched FP32-mixed form), tuning first if needed; every problem must have
+ * a state.  The autotuner times one whole step of each
  * candidate shape (the state is saved and restored around it); FV3D_TILE=WxH
  * forces a shape, FV3D_TILE_LOG=1 prints each candidate's time to stderr. */
 int fvgpu_batch_tiling(fv_batch* b, int* ngroups, int* tx, int* ty, int max_groups);
 /* The full schedule the autotuner chose per group (arrays of max_groups,
  * any may be NULL): strip width tx and rows per work item (as
  * fvgpu_batch_tiling), the rows of one marched block (cells per thread in
- * the update: tx x block_rows / 256; 3-D groups: 0) and whether the viscous
- * fluxes of the face-only branches are computed once per face in a separate
- * pass (1) or fused into each cell's update (0).  The FP32-mixed kernels
- * offer 8- and 16-row blocks and both viscous forms, tuned per (grid sizes,
- * precision, group) and remembered in the tile cache; FV3D_TILE=WxH/Bv
- * forces width W, rows H, block rows B and (suffix v) the per-face form.
- * No reference counterpart. */
+ * the update: tx x block_rows / 256; 0 where the rows are not marched in
+ * blocks; 3-D groups: 0, the z-marched form its 15 rows of columns) and whether
+ * the viscous fluxes of the face-only branches are computed once per face in a
+ * separate pass (1) or fused into each cell's update (0).  FP32-mixed 2-D
+ * groups are marched by warps (tx 28, block_rows 0), their rows per item tuned
+ * per (grid sizes, precision, group) and remembered in the tile cache;
+ * FV3D_TILE=28xH forces the rows, FV3D_TILE=WxH/Bv with W 32 or 64 the
+ * block form: width W, rows H, block rows B (8 or 16) and (suffix v) the
+ * per-face viscous fluxes.  3-D groups: FV3D_TILE=30xH forces H layers per
+ * item, 16xH in the block form.  No reference counterpart. */
 int fvgpu_batch_schedule(fv_batch* b, int* ngroups, int* tx, int* rows, int* block_rows, int* split_viscous,
                          int max_groups);
 
