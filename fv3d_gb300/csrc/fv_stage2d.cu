@@ -80,6 +80,12 @@ struct Strips {
 // faces, conversions and cell updates of a CTA and divides the SM's sum by the
 // share of the pipe its CTAs keep busy between their barriers: 60 % for one,
 // 95 % for two against three (1024^2: 1,330, 850 and 813 us a step).
+// On grids of less than a block of rows per CTA the latency of one segment is
+// the step: a CTA whose rows end one strip and begin the next takes twice as
+// long, so a whole number of CTAs per strip is tried first, and kept unless all
+// there is room for are estimated faster (96x64 49.7 -> 31.2 us a step, 100^2
+// 51.3 -> 32.5, 160^2 58.9 -> 40.6, 90x700 113 -> 102, x-z 64x192 with viscosity
+// 86.7 -> 52.9; 200^2, 256^2 and larger choose as they did).
 Strips split_strips(const Grid& G, int rs, bool wact, int resident) {
   const int sms = sm_count();
   const bool visc = wact && G.visc;
@@ -95,15 +101,24 @@ Strips split_strips(const Grid& G, int rs, bool wact, int resident) {
     int w = (G.na + n_strips - 1) / n_strips;
     if (w0 == kTileX && G.na >= 8 * kTileX) w = kTileX;
     const long long units = (long long)n_strips * G.nb;
-    for (int per_sm = 1; per_sm <= resident; ++per_sm) {
-      const long long ctas = std::min(units, (long long)per_sm * sms);
+    auto warps = [](double lanes) { return std::ceil(lanes / 32.0); };
+    auto segment = [&](double rows) {  // FP64 warp operations of `rows` rows of a strip
+      return face * (warps((w + 1.0) * rows) + warps(w * (rows + 1.0))) + cell * warps(w * rows) +
+             conv * warps((w + 4.0) * (rows + 4.0));
+    };
+    for (int k = 0; k < 2 * resident; ++k) {
+      // a whole number of CTAs per strip, then all there is room for
+      const long long room = std::min(units, (long long)(k / 2 + 1) * sms), aligned = room / n_strips * n_strips;
+      const bool cross = room != aligned;  // some CTA's rows end one strip and begin the next
+      const long long ctas = k & 1 ? room : aligned;
+      if (ctas == 0 || (k & 1 && !cross)) continue;
       const long long rows = (units + ctas - 1) / ctas;  // of the busiest CTA
       const double blocks = std::ceil((double)rows / kTileY);
-      auto warps = [](double lanes) { return std::ceil(lanes / 32.0); };
-      const double work = face * (warps((w + 1.0) * rows) + warps(w * (rows + 1.0))) + cell * warps((double)w * rows) +
-                          conv * warps((w + 4.0) * (rows + 4.0));
       const long long on_sm = (ctas + sms - 1) / sms;
-      const double t = std::max(work * on_sm / busy[std::min(on_sm, 3LL) - 1], phase * blocks);
+      double t = std::max(segment((double)rows) * on_sm / busy[std::min(on_sm, 3LL) - 1], phase * blocks);
+      // two segments one after the other; beyond one block the rest of the SM's work hides it
+      if (k & 1 && blocks == 1.0)
+        t = std::max(t, std::max(2.0 * segment(0.5 * rows) / busy[0], phase * 2.0));
       if (best.ctas == 0 || t < best_t * 0.995) {
         best = Strips{w, units, ctas};
         best_t = t;
