@@ -93,12 +93,16 @@ __device__ __forceinline__ X64 four_thirds_of<X64>() { return s_op64.four_thirds
 // Ziv, "Fast evaluation of elementary mathematical functions with correctly
 // rounded last bit", ACM TOMS 17(3), 1991): r y in units in the last place of
 // Q, computed in FP32 (error below 2^-13), must lie at least 2^-12 away from
-// every half.  Where it does not (one result in 2,048), and for operands so
+// every half, and is taken only up to 2^10 (beyond, neither bound holds; Q is
+// within 2^9 of the result unless the pair crossed a power of two).  Where it
+// does not (one result in 2,048), and for operands so
 // small or large that a step could leave the normal range (divisors outside
 // 2^-150 .. 2^150, numerators outside 2^-750 .. 2^800, roots outside 2^-700 ..
-// 2^700), the IEEE operation itself is called.  A result
-// beside a power of two, where the spacing changes, is taken only if r is
-// zero (an exact quotient).
+// 2^700), the IEEE operation itself is called.  The last place of a quotient is
+// that of Q's own binade, which the seed need not share: a seed up to two FP32
+// units below a power of two can belong to a quotient above it.  A Q within
+// 2^10 of its last places of a power of two, where the spacing changes between
+// it and the result, is taken only if r is zero (an exact quotient).
 static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
 static __device__ __noinline__ double sqrt_ieee(double x) { return sqrt(x); }
 
@@ -115,6 +119,12 @@ __device__ __forceinline__ bool clear_of_half(float t) {
   const float n = __fadd_rn(t, 12582912.0f) - 12582912.0f;  // nearest integer (t < 2^12)
   return fabsf(t - n) < 0.5f - 0x1p-12f;
 }
+
+// The largest correction taken, in units in the last place, and the high word
+// (as a float's exponent) of the residual it belongs to: a quotient's
+// correction is at most twice the residual, a root's at most half.
+constexpr unsigned long long kCorrection = 1ull << 10;
+constexpr int kMaxQuotRes = (127 + 9) << 20, kMaxRootRes = (127 + 11) << 20;
 
 // A divisor prepared for several quotients.
 struct Div64 {
@@ -165,15 +175,15 @@ __device__ __forceinline__ double quot_core(double a, const Div64& D, bool& good
   const double Q = __longlong_as_double(q ^ ((long long)sign << 32));
   const double res = fma(-D.b, Q, a);
   const double out = fma(res, D.y, Q);
-  // the rounding test
+  // the rounding test, in units in the last place of Q's binade: [1, 2) times a power of two, or [1/2, 1)
+  const bool upper = (int)(q >> 32) >= (int)(ea - eb + (1023u << 20));
   const unsigned rhi = (unsigned)__double2hiint(res) & 0x7fffffffu, rlo = (unsigned)__double2loint(res);
   const int x = (int)(rhi - ea + ((127u + 52u) << 20));
   float t = __fmul_rn(x > 0 ? __uint_as_float(__funnelshift_l(rlo, (unsigned)x, 3)) : 0.0f, D.r);
-  t = big ? t : t + t;
-  const bool edge = ((qb + 1u) & 0x007fffffu) <= 1u && (rhi | rlo) != 0u;
+  t = upper ? t : t + t;
+  const bool edge = (((unsigned long long)q + kCorrection) << 12) < (kCorrection << 13) && (rhi | rlo) != 0u;
   const bool zero = ((ahi << 1) | alo) == 0u;  // 0 / b
-  good = D.ok && (zero || (ea - (273u << 20) < (1550u << 20) && x < (int)((127u + 12u) << 20) && clear_of_half(t) &&
-                           !edge));
+  good = D.ok && (zero || (ea - (273u << 20) < (1550u << 20) && x < kMaxQuotRes && clear_of_half(t) && !edge));
   return zero ? __hiloint2double((int)sign, 0) : out;
 }
 
@@ -259,7 +269,7 @@ __device__ __forceinline__ double sqrt_core(double x, bool& good) {
   const int s = (int)(rhi - ((unsigned)(2 * half_e + 1023) << 20) + ((127u + 52u) << 20));
   const float t = __fmul_rn(s > 0 ? __uint_as_float(__funnelshift_l(rlo, (unsigned)s, 3)) : 0.0f, h);
   const bool inside = gb - 0x3f800001u < 0x007ffffeu;  // 1 < g0 < 2, not beside either
-  good = hi - (323u << 20) < (1400u << 20) && s < (int)((127u + 12u) << 20) && clear_of_half(t) &&
+  good = hi - (323u << 20) < (1400u << 20) && s < kMaxRootRes && clear_of_half(t) &&
                     (inside || (rhi | rlo) == 0u);
   return out;
 }
