@@ -70,13 +70,15 @@ __device__ __forceinline__ float minmod(float a, float b) {
 
 // HLLC of RiemannSolvers.h:39-112 (kinetic energy of the normal and first
 // transverse velocity, as the reference) on states in storage order; UN, T1,
-// T2: the slots of the normal and transverse velocities.  cmax^2 =
-// gamma max(pL/rL, pR/rR) takes one reciprocal of rL rR.
+// T2: the slots of the normal and transverse velocities.  Each side has its own
+// reciprocal of the density: products of two densities or of a density and a
+// pressure leave the range of FP32 (rho above 9e18, p rho below 1.2e-38) where
+// the quotients do not.
 template <int UN, int T1, int T2, bool WACT>
 __device__ __forceinline__ void hllc(const float L[5], const float R[5], float gamma, float inv_gm1, float f[5]) {
   constexpr bool H1 = WACT || T1 != 3, H2 = WACT || T2 != 3;
   const float rL = L[0], uL = L[UN], pL = L[4], rR = R[0], uR = R[UN], pR = R[4];
-  const float cmax = sqrt_(mul(mul(gamma, fmaxf(mul(pL, rR), mul(pR, rL))), rcp(mul(rL, rR))));
+  const float cmax = sqrt_(mul(gamma, fmaxf(mul(pL, rcp(rL)), mul(pR, rcp(rR)))));
   const float SL = sub(fminf(uL, uR), cmax);
   const float SR = add(fmaxf(uL, uR), cmax);
   const float dL = sub(uL, SL), dR = sub(SR, uR);
