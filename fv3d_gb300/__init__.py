@@ -179,6 +179,7 @@ def read_ini(path):
 
 
 _double_at = C.c_double.from_address
+_MAX_GROUPS = 10  # the most groups a batch can have
 
 
 def _ptr(a):
@@ -420,15 +421,15 @@ class Batch:
     def schedule(self):
         """[{tx, rows, block_rows, split_viscous}] the autotuner chose per group."""
         ng = C.c_int()
-        arrs = [(C.c_int * 8)() for _ in range(4)]
-        self._check(self.lib.fvgpu_batch_schedule(self._h, C.byref(ng), *arrs, 8), "batch_schedule")
+        arrs = [(C.c_int * _MAX_GROUPS)() for _ in range(4)]
+        self._check(self.lib.fvgpu_batch_schedule(self._h, C.byref(ng), *arrs, _MAX_GROUPS), "batch_schedule")
         keys = ("tx", "rows", "block_rows", "split_viscous")
         return [{k: a[g] for k, a in zip(keys, arrs)} for g in range(ng.value)]
 
     def tiling(self):
         """[(tx, ty)] tile shape chosen per group."""
         ng = C.c_int()
-        tx = (C.c_int * 8)()
-        ty = (C.c_int * 8)()
-        self._check(self.lib.fvgpu_batch_tiling(self._h, C.byref(ng), tx, ty, 8), "batch_tiling")
+        tx = (C.c_int * _MAX_GROUPS)()
+        ty = (C.c_int * _MAX_GROUPS)()
+        self._check(self.lib.fvgpu_batch_tiling(self._h, C.byref(ng), tx, ty, _MAX_GROUPS), "batch_tiling")
         return [(tx[g], ty[g]) for g in range(ng.value)]

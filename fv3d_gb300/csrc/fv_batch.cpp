@@ -44,7 +44,9 @@ using fv::StepCtrl;
 namespace {
 
 constexpr int kGraphSteps = 8;
-constexpr int kMaxGroups = 8;  // two work-queue counters each
+// Two work-queue counters each; there can be 10: 2-D planes and layouts 4, 3-D
+// solvers with the corrected physics 2 and without 4 (marched, block form).
+constexpr int kMaxGroups = 10;
 // Problems of at most this many cells in all run several steps per launch
 // (FP32-mixed RK2, one group of 2-D problems): their steps are bound by
 // launch latency, not by the GPU's throughput.
@@ -53,7 +55,7 @@ constexpr int kMultiChunk = 256;  // steps per multi-step launch of a loop with 
 
 struct Group {
   int ndim = 2;     // 3: 3-D problems (one kernel shape, grouped by solver)
-  bool march = false;  // FP32-mixed 3-D: the z-marched form (every member is one it runs)
+  bool march = false;  // FP32-mixed 3-D: the z-marched form (all members are problems it runs)
   int rs = -1;      // 3-D groups: the shared Riemann solver (bit 0) and corrected physics (bit 1)
   int plane = 0;
   bool wact = false;
@@ -653,26 +655,30 @@ void ReleaseGroups(fv_batch* b) {
   b->prepared = false;
 }
 
-// Groups problems by (plane, third-momentum layout), picks tile shapes and
-// uploads the descriptors.
+// Groups problems by (plane, third-momentum layout; 3-D: solver, physics and
+// kernel form), picks tile shapes and uploads the descriptors.
 int Prepare(fv_batch* b) {
   if (b->prepared) return FV_OK;
   ReleaseGroups(b);
   for (int i = 0; i < b->n; ++i) {
     const int ndim = b->G[i].ndim;
     const int rs = ndim == 3 ? (b->p[i].riemann_solver == FV_HLL ? 0 : 1) + (b->G[i].corrected ? 2 : 0) : -1;
+    // apart from the problems of the block form, so that a problem's form, and
+    // with it its rounding, does not depend on its neighbours in the batch
+    const bool march = Marched3d(b, i);
     Group* g = nullptr;
     for (auto& h : b->groups)
-      if (h.ndim == ndim && h.rs == rs && h.plane == b->G[i].plane && h.wact == (bool)b->wact[i]) g = &h;
+      if (h.ndim == ndim && h.rs == rs && h.march == march && h.plane == b->G[i].plane && h.wact == (bool)b->wact[i])
+        g = &h;
     if (!g) {
       b->groups.push_back(Group());
       g = &b->groups.back();
       g->ndim = ndim;
       g->rs = rs;
+      g->march = march;
       g->plane = b->G[i].plane;
       g->wact = b->wact[i];
     }
-    g->march = ndim == 3 && Marched3d(b, i) && (g->members.empty() || g->march);
     g->members.push_back(i);
     g->tc = g->tc || b->G[i].tc;
   }
