@@ -86,6 +86,7 @@ int Fail(fv_sim* s, int code, const char* fmt, ...) {
   std::vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
   if (s) s->err = buf;
+  cudaGetLastError();  // reported here; the launches of the next call ask for their own
   return code;
 }
 

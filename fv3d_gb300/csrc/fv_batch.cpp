@@ -109,6 +109,7 @@ int Fail(fv_batch* b, int code, const char* fmt, ...) {
   std::vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
   if (b) b->err = buf;
+  cudaGetLastError();  // reported here; the launches of the next call ask for their own
   return code;
 }
 
