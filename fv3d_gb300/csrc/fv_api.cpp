@@ -7,9 +7,9 @@
 // the step is active (t + epsilon < tend), and the stage kernels follow;
 // fvgpu_advance replays a captured CUDA graph of several such steps and only
 // reads the control block back between replays.
+#include <cudaTypedefs.h>  // PFN_cuPointerGetAttributes
 #include <cmath>
 #include <cstdarg>
-#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -542,20 +542,32 @@ int SetState(fv_sim* s, const double* const ref_fields[5], bool prim) {
 namespace fv {
 
 bool pinned_fields(const double* const host[5], long long n, Fields* view) {
+  static const PFN_cuPointerGetAttributes_v7000 query = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool ok = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 7000, cudaEnableDefault, &q) ==
+                        cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return reinterpret_cast<PFN_cuPointerGetAttributes_v7000>(ok ? fn : nullptr);
+  }();
   for (int v = 0; v < 5; ++v) {
     view->f[v] = nullptr;
     if (!host[v]) continue;
-    cudaPointerAttributes a{}, z{};
-    if (cudaPointerGetAttributes(&a, host[v]) != cudaSuccess ||
-        cudaPointerGetAttributes(&z, host[v] + (n - 1)) != cudaSuccess) {
-      cudaGetLastError();
+    // both ends pinned would not do: they can belong to two registrations with
+    // pageable memory between them, so the array must lie in one of them
+    unsigned type = 0, managed = 0;
+    CUdeviceptr first = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* values[] = {&type, &managed, &first, &start, &size};
+    if (!query || query(5, what, values, reinterpret_cast<CUdeviceptr>(host[v])) != CUDA_SUCCESS) return false;
+    const size_t bytes = (size_t)n * sizeof(double);
+    if (type != CU_MEMORYTYPE_HOST || managed || !first || first % sizeof(double) || first < start || bytes > size ||
+        first - start > size - bytes)
       return false;
-    }
-    double* first = static_cast<double*>(a.devicePointer);
-    if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !first ||
-        reinterpret_cast<uintptr_t>(first) % sizeof(double) || z.devicePointer != first + (n - 1))
-      return false;
-    view->f[v] = first;
+    view->f[v] = reinterpret_cast<double*>(first);
   }
   return true;
 }

@@ -139,9 +139,9 @@ cudaError_t launch_cons_to_prim_to(const Grid& G, bool wact, Fields src, Fields 
 // both in FP64 arithmetic.
 cudaError_t launch_prim_to_pairs_from(const Grid& G, Fields src, Fields dst_pairs, cudaStream_t stream);
 cudaError_t launch_pairs_to_prim_to(const Grid& G, bool wact, Fields src_pairs, Fields dst, cudaStream_t stream);
-// The device's view of the caller's arrays of n values when all of them are
-// pinned host memory from end to end (null entries stay null), so that a
-// kernel can read or write them in place; false otherwise.
+// The device's view of the caller's arrays of n values when each of them lies
+// in one pinned host allocation or registration (null entries stay null), so
+// that a kernel can read or write them in place; false otherwise.
 bool pinned_fields(const double* const host[5], long long n, Fields* view);
 
 // Compensated per-block partial sums of the five conserved fields:
