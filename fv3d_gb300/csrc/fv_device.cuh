@@ -36,6 +36,12 @@ struct StepCtrl {
   float2 dt_pair;      // dt_cur as a (hi, lo) pair, for the marched FP32-mixed kernels
 };
 
+// Sets bit 1 of an error flag when a bounded wait ran out for any lane of the
+// calling warp: every lane polls for itself, so any of them can be the one.
+__device__ __forceinline__ void report_late(bool late, int* err) {
+  if (__any_sync(0xffffffffu, late) && (threadIdx.x & 31) == 0) atomicOr(err, 2);
+}
+
 // x as hi + lo, hi = RN(x) in FP32.
 __host__ __device__ inline float2 float_pair(double x) {
   const float hi = (float)x;

@@ -512,7 +512,7 @@ march_stage3d32(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsi
     float red = 0.0f;
     bool bad = false;
     march_block32<KIND, VISC>(I, flip, ctrl->dt_pair, x0, y0, nx, ny, k0, k1, smem_f, &s_mbar, phase, late, red, bad);
-    if (late && (threadIdx.x & 31) == 0) atomicOr(&ctrl->err, 2);
+    report_late(late, &ctrl->err);
     if (KIND != STAGE_RK_1) {
       const unsigned mx = __reduce_max_sync(0xffffffffu, __float_as_uint(red));  // non-negative floats order like their bits
       const bool any_bad = __any_sync(0xffffffffu, bad);
