@@ -448,11 +448,13 @@ int Autotune(fv_batch* b, Group& g) {
     return true;
   };
   if (const char* force = std::getenv("FV3D_TILE")) {  // WxH, WxH/B, WxHv, WxH/Bv
-    Schedule sc;
+    Schedule sc;  // blocks of 16 rows, but where the width is that of the marched form, which has none
     char rest[16] = "";
     const int got = std::sscanf(force, "%dx%d%15s", &sc.tx, &sc.rows, rest);
     if (got >= 2 && sc.rows > 0) {
       char* r = rest;
+      for (int s = 0; s < ns && !d3; ++s)
+        if (b->precision != FV_PREC_FP64 && fv::batch_shape_marched32(s) && shapes[s].tx == sc.tx) sc.block_rows = 0;
       if (*r == '/') sc.block_rows = (int)std::strtol(r + 1, &r, 10);
       sc.vface = *r == 'v' ? 1 : 0;
       if (d3) {  // 16 forces the block form, 30 the z-marched one
