@@ -515,14 +515,23 @@ int Autotune(fv_batch* b, Group& g) {
     if (slots <= 0) continue;
     long long units = 0;
     for (int i : g.members) units += (long long)((b->G[i].na + shapes[s].tx - 1) / shapes[s].tx) * b->G[i].nb;
-    // the rows that fill the resident slots once (marched: at most once to four times)
-    for (int k = 1; k <= (marched ? 4 : 1); ++k) {
-      const int rows = marched ? RowsForSlots(b, g, shapes[s].tx, k * slots)
-                               : (int)std::max(4LL, (units + slots - 1) / slots);
+    auto add = [&](int rows) {
       bool dup = false;
       for (auto& c : cand) dup = dup || (shape_of(ShapeSchedule(b, c.first)) == s && c.second == rows);
       if (!dup) cand.push_back({s, rows});
+    };
+    if (!marched) {
+      add((int)std::max(4LL, (units + slots - 1) / slots));  // fill the resident slots once
+      continue;
     }
+    // the rows that fill the resident slots at most once to four times, and a
+    // third and a half of them: an item's first two rows only fill registers,
+    // so that on small grids fewer, longer items are the faster ones (Euler
+    // 256^2: 1 row 10.0 us a step, 2 8.2, 3 7.7, 4 8.2; 700x500: 3 rows 17.2,
+    // 5 14.1, 8 13.1, 16 16.0)
+    for (int k = 1; k <= 4; ++k) add(RowsForSlots(b, g, shapes[s].tx, k * slots));
+    for (int k = 2; k <= 3; ++k) add(RowsForSlots(b, g, shapes[s].tx, slots / k));
+    for (int rows : {8, 16}) add(rows);
   }
   StepCtrl* tune_ctrl = nullptr;
   BatchInst* tune_inst = nullptr;
