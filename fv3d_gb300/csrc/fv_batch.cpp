@@ -45,7 +45,7 @@ namespace {
 
 constexpr int kGraphSteps = 8;
 // Two work-queue counters each; there can be 10: 2-D planes and layouts 4, 3-D
-// solvers with the corrected physics 2 and without 4 (marched, block form).
+// solvers with the corrected physics 2 and without 4 (z-boundary physics or none).
 constexpr int kMaxGroups = 10;
 // Problems of at most this many cells in all run several steps per launch
 // (FP32-mixed RK2, one group of 2-D problems): their steps are bound by
@@ -55,8 +55,8 @@ constexpr int kMultiChunk = 256;  // steps per multi-step launch of a loop with 
 
 struct Group {
   int ndim = 2;     // 3: 3-D problems (one kernel shape, grouped by solver)
-  bool march = false;  // FP32-mixed 3-D: the z-marched form (all members are problems it runs)
-  int rs = -1;      // 3-D groups: the shared Riemann solver (bit 0) and corrected physics (bit 1)
+  int rs = -1;      // 3-D groups: the shared Riemann solver (bit 0), corrected physics (bit 1), PlainMixed3d (bit 2)
+  bool march = false;  // PlainMixed3d groups: the z-marched form, else the block form
   int plane = 0;
   bool wact = false;
   bool tc = false;
@@ -230,8 +230,8 @@ std::string GroupKey(const fv_batch* b, const Group& g) {
     cells += (long long)s.first * s.second;
   }
   std::ostringstream k;
-  // k2: the generation of the stage kernels; a choice tuned on others is not taken over
-  k << "p" << b->precision << "k2" << (g.march ? "m" : "") << "_d" << g.ndim << "_co" << (g.rs >= 2) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
+  // the generation of the stage kernels and of what is tried; a choice tuned on others is not taken over
+  k << "p" << b->precision << (b->precision == FV_PREC_FP64 ? "k2" : "k3") << (g.march ? "m" : "") << "_d" << g.ndim << "_co" << (g.rs >= 0 && (g.rs & 2)) << "_pl" << g.plane << "_w" << g.wact << "_tc" << g.tc << "_v" << visc << "_rs"
     << rs_mask << "_ts" << b->ts << "_n" << g.members.size() << "_c" << cells << "_h" << std::hex << h;
   return k.str();
 }
@@ -270,16 +270,12 @@ bool Viscous(const fv_batch* b, const Group& g) {
   return false;
 }
 
-// Whether the z-marched FP32-mixed form runs problem i: not the z-boundary
-// physics (C91, well-balanced fluxes, fixed conduction boundaries) and not the
-// corrected physics, which only the block form has; and not plain Euler steps
-// without slopes, whose layers are too cheap to hide its barrier (blast 256^3
-// 782 us a step against 712 with the block form; with slopes, two stages,
-// conduction or viscosity it is the faster one: 192^3 PLM Euler 377 against
-// 409, PCM RK2 561 / 616, PLM RK2 596 / 749, with both terms 765 / 1,000).
-bool Marched3d(const fv_batch* b, int i) {
+// Whether problem i is one of the FP32-mixed 3-D problems that both the
+// z-marched and the block form run, with the same bits: no z-boundary physics
+// (C91, well-balanced fluxes, fixed conduction boundaries) and no corrected
+// physics, which have a body of the block form to themselves.
+bool PlainMixed3d(const fv_batch* b, int i) {
   const Grid& G = b->G[i];
-  if (b->ts != FV_TS_RK2 && G.recon != fv::R_PLM && !G.tc && !G.visc) return false;
   return b->precision != FV_PREC_FP64 && G.ndim == 3 && G.bc_c != fv::DBC_C91 && !G.wb_flux_z && !G.corrected &&
          !(G.tc && (G.bctc_zmin != FV_BCTC_NONE || G.bctc_zmax != FV_BCTC_NONE));
 }
@@ -316,7 +312,9 @@ int Occupancy(const fv_batch* b, const Group& g, int shape) {
                                  g.members.size() == 1);
   if (g.ndim == 3)
     return b->precision == FV_PREC_FP64 ? fv::batch_stage3d_occupancy64(g.rs, g.tc)
-                                        : fv::batch_stage3d_occupancy32(g.rs, g.tc);
+                                        : fv::batch_stage3d_occupancy32(
+                                              g.rs, g.tc, Viscous(b, g),
+                                              b->ts == FV_TS_RK2 ? fv::STAGE_RK_2 : fv::STAGE_EULER);
   return b->precision == FV_PREC_FP64 ? fv::batch_stage_occupancy64(g.plane, g.wact, shape, g.tc)
                                       : fv::batch_stage_occupancy32(
                                             g.plane, g.wact, shape, g.tc,
@@ -335,7 +333,7 @@ cudaError_t LaunchStage(const fv_batch* b, const Group& g, const BatchInst* inst
                ? fv::launch_batch_stage3d64(insts, (int)g.members.size(), ntiles, queue, kind, flip, g.rs, grid, g.tc,
                                             b->stream)
                : fv::launch_batch_stage3d32(insts, (int)g.members.size(), ntiles, queue, kind, flip, g.rs, grid, g.tc,
-                                            b->stream);
+                                            Viscous(b, g), b->stream);
   return b->precision == FV_PREC_FP64
              ? fv::launch_batch_stage64(g.plane, g.wact, g.shape, insts, (int)g.members.size(), ntiles, queue, kind,
                                         flip, grid, g.tc, b->stream)
@@ -394,6 +392,82 @@ int SmCount() {
 int GridFor(const fv_batch* b, const Group& g, int shape, int occupancy, int ntiles) {
   const int per = ItemsPerCta(b, g, shape);
   return std::max(1, std::min(occupancy * SmCount(), (ntiles + per - 1) / per));
+}
+
+// Work items of a 3-D group: blocks of cols x rows columns times chunks of z layers.
+long long Items3d(const fv_batch* b, const Group& g, int cols, int rows, int z) {
+  long long n = 0;
+  for (int i : g.members)
+    n += (long long)((b->G[i].na + cols - 1) / cols) * ((b->G[i].nb + rows - 1) / rows) * ((b->G[i].nc + z - 1) / z);
+  return n;
+}
+
+// The z layers per work item worth trying for a 3-D group (each item converts
+// the layers around its chunk first): powers of two, and the chunk lengths
+// that make the work items fill 1-4 rounds of the resident CTAs (the fewest
+// layers with at most r rounds of items).
+std::vector<int> LayersToTry(const fv_batch* b, const Group& g, int cols, int rows, long long slots) {
+  int max_nc = 1;
+  for (int i : g.members) max_nc = std::max(max_nc, b->G[i].nc);
+  std::vector<int> layers;
+  for (int z : {8, 16, 32, 64})
+    if (z == 8 || z <= max_nc) layers.push_back(z);
+  for (int r = 1; r <= 4 && slots > 0; ++r) {
+    int z = 4;
+    while (z < max_nc && Items3d(b, g, cols, rows, z) > r * slots) ++z;
+    if (std::find(layers.begin(), layers.end(), z) == layers.end() && Items3d(b, g, cols, rows, z) <= r * slots)
+      layers.push_back(z);
+  }
+  return layers;
+}
+
+// Whether a group of PlainMixed3d problems runs z-marched or in 16 x 16 blocks
+// (the same bits either way).  One marched CTA of 30 x 15 columns fills an SM;
+// it hides the latency of few layers best, but leaves lanes idle where its
+// blocks do not divide the plane (32 x 32 columns take six).  Four 16 x 16
+// CTAs share an SM (three with viscosity).  Groups that give every SM at most
+// one marched item of four layers march (24^3 PLM RK2 32 us a step against
+// 36, 33x47x21 34 / 40, 48^3 33 / 38), but for Euler steps without slopes or
+// diffusion (24^3 18.3 / 17.8).  The others take the form with the smaller
+// estimate below, fitted to both forms on 196 groups of one to 200 problems
+// (9 % at worst above the faster form, 0.5 % on average): PLM RK2 with
+// conduction and viscosity, 64 of 32^3 638 marched, 300 in blocks; 300x75x100
+// 237 / 311; PCM RK2 160^3 388 / 280, 100 of 24^3 211 / 189; PLM RK2
+// 101x83x61 69 / 80.
+bool MarchedIsFaster(const fv_batch* b, Group& g) {
+  bool plm = false, tc = false, visc = false;
+  for (int i : g.members) {
+    plm = plm || b->G[i].recon == fv::R_PLM;
+    tc = tc || b->G[i].tc;
+    visc = visc || b->G[i].visc;
+  }
+  if (b->ts != FV_TS_RK2 && !plm && !tc && !visc) return false;
+  const long long sms = SmCount();
+  double time[2] = {0.0, 0.0};  // blocks, marched: microseconds a stage, about
+  for (int form = 0; form < 2; ++form) {
+    g.march = form == 1;
+    const int resident = Occupancy(b, g, 0);
+    if (resident <= 0) return form == 0;
+    int cols, rows;
+    Block3d(g, &cols, &rows);
+    if (form == 1 && Items3d(b, g, cols, rows, 4) <= sms) return true;
+    int max_nc = 1;
+    for (int i : g.members) max_nc = std::max(max_nc, b->G[i].nc);
+    for (int z : LayersToTry(b, g, cols, rows, resident * sms)) {
+      const double items = (double)Items3d(b, g, cols, rows, z);
+      const double per_sm = std::ceil(items / sms), layers = std::min(z, max_nc);
+      double t;
+      if (form == 1) {
+        t = std::ceil(per_sm / resident) * (layers + 1.3) * (2.3 + 0.2 * plm + 0.1 * tc + 0.85 * visc);
+      } else {  // a layer of a CTA takes longer the more of them share the SM
+        const double layer = 1.1 + 0.4 * plm + 0.25 * tc + 0.45 * visc;
+        t = std::max(1.0, items / (double)(resident * sms)) * (layers + 1.4) * layer *
+            (0.75 + 0.85 * std::min(per_sm, (double)resident));
+      }
+      if (time[form] == 0.0 || t < time[form]) time[form] = t;
+    }
+  }
+  return time[1] < time[0];
 }
 
 // The fewest rows per work item with which the group's strips of tx columns
@@ -459,6 +533,7 @@ int Autotune(fv_batch* b, Group& g) {
       sc.vface = *r == 'v' ? 1 : 0;
       if (d3) {  // 16 forces the block form, 30 the z-marched one
         if (sc.tx == fv::batch3d_columns()) g.march = false;
+        else if (g.rs & 4) g.march = true;
         sc = Schedule3d(b, g, sc.rows);
       } else if (b->precision == FV_PREC_FP64) {  // one kernel per strip width
         const int rows = sc.rows;
@@ -480,30 +555,10 @@ int Autotune(fv_batch* b, Group& g) {
   // that give each resident CTA one work item's worth of strip rows (the
   // balanced split for a few large problems).
   std::vector<std::pair<int, int>> cand;
-  int max_nc = 1;
-  for (int i : g.members) max_nc = std::max(max_nc, b->G[i].nc);
-  if (d3) {  // z layers per work item; a 4-layer prologue is converted per item
-    for (int z : {8, 16, 32, 64})
-      if (z == 8 || z <= max_nc) cand.push_back({0, z});
-    // and the chunk lengths that make the work items fill 1-4 rounds of the
-    // resident CTAs (the fewest layers with at most r rounds of items)
-    const long long slots = (long long)Occupancy(b, g, 0) * SmCount();
+  if (d3) {
     int cols, rows;
     Block3d(g, &cols, &rows);
-    auto items = [&](int z) {
-      long long n = 0;
-      for (int i : g.members)
-        n += (long long)((b->G[i].na + cols - 1) / cols) * ((b->G[i].nb + rows - 1) / rows) *
-             ((b->G[i].nc + z - 1) / z);
-      return n;
-    };
-    for (int r = 1; r <= 4 && slots > 0; ++r) {
-      int z = 4;
-      while (z < max_nc && items(z) > r * slots) ++z;
-      bool dup = false;
-      for (auto& c : cand) dup = dup || c.second == z;
-      if (!dup && items(z) <= r * slots) cand.push_back({0, z});
-    }
+    for (int z : LayersToTry(b, g, cols, rows, (long long)Occupancy(b, g, 0) * SmCount())) cand.push_back({0, z});
   }
   const bool marched = !d3 && b->precision != FV_PREC_FP64;  // mixed 2-D: the warp-marched shapes
   for (int s = 0; s < ns && !d3; ++s)
@@ -667,27 +722,25 @@ void ReleaseGroups(fv_batch* b) {
   b->prepared = false;
 }
 
-// Groups problems by (plane, third-momentum layout; 3-D: solver, physics and
-// kernel form), picks tile shapes and uploads the descriptors.
+// Groups problems by (plane, third-momentum layout; 3-D: solver and physics),
+// picks tile shapes and uploads the descriptors.
 int Prepare(fv_batch* b) {
   if (b->prepared) return FV_OK;
   ReleaseGroups(b);
   for (int i = 0; i < b->n; ++i) {
     const int ndim = b->G[i].ndim;
-    const int rs = ndim == 3 ? (b->p[i].riemann_solver == FV_HLL ? 0 : 1) + (b->G[i].corrected ? 2 : 0) : -1;
-    // apart from the problems of the block form, so that a problem's form, and
-    // with it its rounding, does not depend on its neighbours in the batch
-    const bool march = Marched3d(b, i);
+    // 3-D: the body a problem takes, and with it its rounding, depends on the problem alone
+    const int rs = ndim == 3 ? (b->p[i].riemann_solver == FV_HLL ? 0 : 1) + (b->G[i].corrected ? 2 : 0) +
+                                   (PlainMixed3d(b, i) ? 4 : 0)
+                             : -1;
     Group* g = nullptr;
     for (auto& h : b->groups)
-      if (h.ndim == ndim && h.rs == rs && h.march == march && h.plane == b->G[i].plane && h.wact == (bool)b->wact[i])
-        g = &h;
+      if (h.ndim == ndim && h.rs == rs && h.plane == b->G[i].plane && h.wact == (bool)b->wact[i]) g = &h;
     if (!g) {
       b->groups.push_back(Group());
       g = &b->groups.back();
       g->ndim = ndim;
       g->rs = rs;
-      g->march = march;
       g->plane = b->G[i].plane;
       g->wact = b->wact[i];
     }
@@ -696,6 +749,7 @@ int Prepare(fv_batch* b) {
   }
   if ((int)b->groups.size() > kMaxGroups) return Fail(b, FV_ERR_UNSUPPORTED, "more than %d batch groups", kMaxGroups);
   for (auto& g : b->groups) {
+    g.march = g.ndim == 3 && (g.rs & 4) && MarchedIsFaster(b, g);
     int rc = Autotune(b, g);
     if (rc) return rc;
     std::vector<BatchInst> d = Describe(b, g, g.shape, b->d_ctrl, &g.ntiles, g.rows);

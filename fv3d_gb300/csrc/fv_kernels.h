@@ -213,10 +213,12 @@ int batch3d_columns();  // column-block side (16)
 cudaError_t launch_batch_stage3d64(const BatchInst* insts, int ninst, int ntiles, unsigned* queue, int kind, int flip,
                                    int rs, int grid, bool tc, cudaStream_t stream);
 cudaError_t launch_batch_stage3d32(const BatchInst* insts, int ninst, int ntiles, unsigned* queue, int kind, int flip,
-                                   int rs, int grid, bool tc, cudaStream_t stream);
-// rs: Riemann solver (bit 0), corrected physics (bit 1).
+                                   int rs, int grid, bool tc, bool visc, cudaStream_t stream);
+// rs: Riemann solver (bit 0), corrected physics (bit 1); FP32-mixed: neither
+// z-boundary nor corrected physics (bit 2), the body whose bits are those of
+// the z-marched form.
 int batch_stage3d_occupancy64(int rs, bool tc);
-int batch_stage3d_occupancy32(int rs, bool tc);
+int batch_stage3d_occupancy32(int rs, bool tc, bool visc, int kind);
 
 // The z-marched form of the FP32-mixed 3-D stage (fv_march3d32.cu): work items
 // are blocks of at most *cols x *rows columns (of equal size per problem,
