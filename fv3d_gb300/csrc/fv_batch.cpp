@@ -48,8 +48,8 @@ constexpr int kGraphSteps = 8;
 // solvers with the corrected physics 2 and without 4 (z-boundary physics or none).
 constexpr int kMaxGroups = 10;
 // Problems of at most this many cells in all run several steps per launch
-// (FP32-mixed RK2, one group of 2-D problems): their steps are bound by
-// launch latency, not by the GPU's throughput.
+// (FP32-mixed RK2, one group of 2-D problems): their steps are bound by the
+// latency of launches and stages, not by the GPU's throughput.
 constexpr long long kMultiMaxCells = 1LL << 21;
 constexpr int kMultiChunk = 256;  // steps per multi-step launch of a loop with a time bound
 
@@ -767,7 +767,7 @@ int Prepare(fv_batch* b) {
 // that gave up, bit 0 a non-finite state or dt.
 int ErrStatus(int err) { return (err & 2) ? FV_ERR_TIMEOUT : FV_ERR_NONFINITE; }
 
-// Whether run / advance take several steps per launch (batch_multi32): the
+// Whether run / advance take several steps per launch (march_multi32): the
 // FP32-mixed RK2 form, one group of 2-D problems, few cells in all.
 // FV3D_MULTISTEP=0 keeps the per-stage launches, =1 takes the multi-step
 // launch whatever the size.

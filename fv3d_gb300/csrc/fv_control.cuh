@@ -1,7 +1,7 @@
 // fv_control.cuh -- the per-step control arithmetic of one problem (dt from
 // the fused CFL reduction, the loop bound, the active flag), shared by the
 // control kernels (fv_aux.cu) and the persistent multi-step kernel
-// (fv_batch32.cu) so that both take bit-identical steps.  IEEE double
+// (fv_march32.cuh) so that both take bit-identical steps.  IEEE double
 // operations are written as intrinsics: the including files differ in their
 // contraction and fast-math settings.
 #pragma once

@@ -1,7 +1,8 @@
 // fv_exact64.cuh -- FP64 building blocks that round exactly like the plain
 // IEEE operations they replace, with fewer FP64-pipe instructions.
 //
-// On GB300 the FP64 pipe executes about 1/64 of the FP32 rate, so the plain
+// On GB300 the FP64 pipe executes 1/59 of the FP32 rate at most (measured:
+// 628 G FMA/s with three register operands against 36,750), so the plain
 // FP64 path is bound by its count of FP64 instructions.  Every helper here
 // returns bit-for-bit the value of the reference expression it stands for
 // (for finite operands away from the subnormal range), so the FP64 stage

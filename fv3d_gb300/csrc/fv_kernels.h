@@ -231,7 +231,7 @@ cudaError_t launch_march3d32(const BatchInst* insts, int ninst, int ntiles, unsi
 
 // Several RK2 steps of a group of FP32-mixed 2-D problems in one cooperative
 // launch (fv_march32.cuh, march_multi32; marched shapes only): for small
-// grids, whose steps are bound by launch latency.  At most
+// grids, whose steps are bound by the latency of launches and stages.  At most
 // batch_multi_problems32() problems; grid at most batch_multi_occupancy32() x
 // SMs CTAs (all resident); the barrier counter and abort flag of gb zeroed
 // before the launch; a grid-barrier wait that runs out sets bit 1 of every

@@ -488,11 +488,10 @@ march_stage3d32(const BatchInst* __restrict__ insts, int ninst, int ntiles, unsi
     const int per_layer = I.tiles_x * I.tiles_y;
     const int bz = lt / per_layer, rem = lt - bz * per_layer;
     const int by = rem / I.tiles_x, bx = rem - by * I.tiles_x;
-    // blocks of equal size
+    // blocks of equal size; none is empty: bw <= kBX and na > (tiles_x - 1) kBX, likewise the rows
     const int bw = (I.G.na + I.tiles_x - 1) / I.tiles_x, bh = (I.G.nb + I.tiles_y - 1) / I.tiles_y;
     const int x0 = bx * bw, y0 = by * bh, k0 = bz * I.tz, k1 = min(k0 + I.tz, I.G.nc);
     const int nx = min(bw, I.G.na - x0), ny = min(bh, I.G.nb - y0);
-    if (nx <= 0 || ny <= 0) continue;  // rounding left this block empty
     if (!ctrl->active) {
       if (KIND == STAGE_EULER) {  // an inactive Euler step hands its state on
         for (int i = threadIdx.x; i < nx * ny * (k1 - k0); i += kThreads3) {

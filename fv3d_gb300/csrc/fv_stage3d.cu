@@ -327,10 +327,8 @@ __device__ __forceinline__ void viscous_iz3d(const PA& P, X64 odx, X64 odz, X64 
 
 // One stage for the w x h columns from (x0, y0) on and z layers [k0, k1); rs 0 HLL /
 // 1 HLLC, kind a StageKind (constants in the one-problem kernel, per work
-// item in the batch kernel); P2: every cell size is a power of two (callers
-// branch on it once, uniformly).  Every thread of the CTA must call it; the
-// CFL maximum is folded into red (the caller reduces it once per CTA or work
-// item).
+// item in the batch kernel).  Every thread of the CTA must call it; the CFL
+// maximum is folded into red (the caller reduces it once per CTA or work item).
 template <bool CORR>
 __device__ __forceinline__ void stage3d_segment(const Grid& G, const Fields& uin, const Fields& u0,
                                                 const Fields& uout, StepCtrl* __restrict__ ctrl, int rs, int kind,

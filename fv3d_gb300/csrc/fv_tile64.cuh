@@ -50,10 +50,6 @@ template <int TX_, int TY_>
 struct Tile {
   static constexpr int TX = TX_, TY = TY_;
   static constexpr int HX = TX + 4, HY = TY + 4;         // tile + 2-cell halo
-  static constexpr int NFA = (TX + 1) * TY;              // a-faces
-  static constexpr int NFA_PAD = (NFA + 31) / 32 * 32;   // keeps each warp on one face kind
-  static constexpr int NFB = TX * (TY + 1);              // b-faces
-  static constexpr int CELLS = TX * TY;
 };
 
 // Division of small indices by a strip's width, known only at run time: exact
