@@ -95,7 +95,7 @@ struct fv_batch {
   cudaGraphExec_t graph_loop = nullptr;  // steps in each control block's own mode
   BatchInst* d_inst_multi = nullptr;     // descriptors of the multi-step launch
   BatchInst one_multi{};
-  int ntiles_multi = 0, grid_multi = 0, rows_multi = 0;
+  int ntiles_multi = 0, grid_multi = 0;
   long launches = 0;
   std::string err;
 };
@@ -786,7 +786,12 @@ bool MultiEligible(const fv_batch* b) {
 // Descriptors of the multi-step launch: the fewest rows per work item that
 // give each resident warp at most one item (the items are assigned
 // statically, so a second round of them would wait for the first;
-// FV3D_MULTI_ROWS forces the rows).
+// FV3D_MULTI_ROWS forces the rows).  Three CTAs on an SM are enough where that
+// takes no more than 5 rows: a fourth on some SMs lengthens the short items of
+// all (us a step of 30x1000 with 1 row, 500 CTAs 12.6, with 2 rows, 250 CTAs
+// 11.4; 100 of 32^2 3 rows 21.3, 4 rows 20.4; 420x400 17.2 / 16.9); of longer
+// items it leaves fewer (512^2 20.8 with 4 rows and 4 CTAs, 21.0 with 6; 1024^2
+// 48.7 with 16, 55.6 with 24).
 int PrepareMulti(fv_batch* b) {
   if (b->d_inst_multi) return FV_OK;
   Group& g = b->groups[0];
@@ -795,7 +800,9 @@ int PrepareMulti(fv_batch* b) {
   const fv::TileShape* shapes;
   NumShapes(b->precision, &shapes);
   const int tx = shapes[g.shape].tx;
-  int rows = RowsForSlots(b, g, tx, (long long)occ * SmCount() * ItemsPerCta(b, g, g.shape));
+  const long long warps = (long long)SmCount() * ItemsPerCta(b, g, g.shape);  // of one CTA per SM
+  int rows = RowsForSlots(b, g, tx, std::min(occ, 3) * warps);
+  if (rows > 5) rows = RowsForSlots(b, g, tx, occ * warps);
   if (const char* f = std::getenv("FV3D_MULTI_ROWS")) rows = std::max(1, std::atoi(f));
   std::vector<BatchInst> d = Describe(b, g, g.shape, b->d_ctrl, &b->ntiles_multi, rows);
   b->one_multi = d[0];
@@ -803,8 +810,9 @@ int PrepareMulti(fv_batch* b) {
   BCUDA(b, cudaMemcpyAsync(b->d_inst_multi, d.data(), sizeof(BatchInst) * d.size(), cudaMemcpyHostToDevice,
                            b->stream));
   BCUDA(b, cudaStreamSynchronize(b->stream));
-  b->rows_multi = rows;
   b->grid_multi = GridFor(b, g, g.shape, occ, b->ntiles_multi);
+  if (std::getenv("FV3D_TILE_LOG"))
+    std::fprintf(stderr, "fv3d multi-step: %d rows (%d items, %d CTAs)\n", rows, b->ntiles_multi, b->grid_multi);
   return FV_OK;
 }
 
