@@ -86,6 +86,12 @@ struct Strips {
 // there is room for are estimated faster (96x64 49.7 -> 31.2 us a step, 100^2
 // 51.3 -> 32.5, 160^2 58.9 -> 40.6, 90x700 113 -> 102, x-z 64x192 with viscosity
 // 86.7 -> 52.9; 200^2, 256^2 and larger choose as they did).
+// On planes of less than half a block of rows a CTA's rows can span many strips,
+// one started after the other, which a share of the rows alone does not show:
+// they are counted, and one CTA per strip is tried too, more than there is room
+// for at once (PLM RK2 9001x2 113 -> 40 us a step, 15000x5 181 -> 102, 4000x3 74
+// -> 35, 60000x4 334 -> 306; from 8 rows on it gains and loses: 30000x8 265 ->
+// 242, with conduction and viscosity 514 -> 534, 40000x12 441 -> 478).
 Strips split_strips(const Grid& G, int rs, bool wact, int resident) {
   const int sms = sm_count();
   const bool visc = wact && G.visc;
@@ -93,6 +99,7 @@ Strips split_strips(const Grid& G, int rs, bool wact, int resident) {
   const double cell = 55 + (G.tc ? 20 : 0) + (visc ? 40 : 0), conv = 8;
   const double phase = 7000.0 / 16.0;  // latency of a block's phases, in FP64 warp operations
   const double busy[3] = {0.60, 0.95, 1.0};
+  const bool low = G.nb < kTileY / 2;
   Strips best{};
   double best_t = 0.0;
   for (int w0 : {kTileX, 24, 16, 12, 8}) {
@@ -106,19 +113,28 @@ Strips split_strips(const Grid& G, int rs, bool wact, int resident) {
       return face * (warps((w + 1.0) * rows) + warps(w * (rows + 1.0))) + cell * warps(w * rows) +
              conv * warps((w + 4.0) * (rows + 4.0));
     };
-    for (int k = 0; k < 2 * resident; ++k) {
-      // a whole number of CTAs per strip, then all there is room for
+    const int forms = 2 * resident + (low && n_strips > resident * sms);
+    for (int k = 0; k < forms; ++k) {
+      // a whole number of CTAs per strip, then all there is room for; at last, on low planes, one per strip
+      const bool each = k == 2 * resident;
       const long long room = std::min(units, (long long)(k / 2 + 1) * sms), aligned = room / n_strips * n_strips;
-      const bool cross = room != aligned;  // some CTA's rows end one strip and begin the next
-      const long long ctas = k & 1 ? room : aligned;
-      if (ctas == 0 || (k & 1 && !cross)) continue;
+      const bool cross = !each && k & 1;  // some CTA's rows end one strip and begin the next
+      const long long ctas = each ? n_strips : (cross ? room : aligned);
+      if (ctas == 0 || (cross && room == aligned)) continue;
       const long long rows = (units + ctas - 1) / ctas;  // of the busiest CTA
       const double blocks = std::ceil((double)rows / kTileY);
       const long long on_sm = (ctas + sms - 1) / sms;
       double t = std::max(segment((double)rows) * on_sm / busy[std::min(on_sm, 3LL) - 1], phase * blocks);
       // two segments one after the other; beyond one block the rest of the SM's work hides it
-      if (k & 1 && blocks == 1.0)
+      if (cross && blocks == 1.0)
         t = std::max(t, std::max(2.0 * segment(0.5 * rows) / busy[0], phase * 2.0));
+      // low planes: each start of a segment takes some three phases
+      if (low && cross && rows > G.nb + 1) {
+        const long long pieces = 2 + (rows - 2) / G.nb;
+        t = std::max(t, std::max(pieces * segment((double)rows / pieces) * on_sm / busy[std::min(on_sm, 3LL) - 1],
+                                 3.0 * phase * pieces));
+      }
+      if (each) t = std::max(t, 3.0 * phase * ((on_sm + resident - 1) / resident));
       if (best.ctas == 0 || t < best_t * 0.995) {
         best = Strips{w, units, ctas};
         best_t = t;
