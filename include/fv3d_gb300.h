@@ -296,7 +296,8 @@ int fvgpu_batch_times(fv_batch* b, double* t);
 int fvgpu_batch_set_stream(fv_batch* b, void* cuda_stream);
 int fvgpu_batch_synchronize(fv_batch* b);
 int fvgpu_batch_launch_count(const fv_batch* b, long* count);
-/* Problems sharing plane and layout form a group advanced by one persistent
+/* Problems sharing plane and layout (3-D: Riemann solver, and the kernel body
+ * their physics takes) form a group, ten at most, advanced by one persistent
  * launch per stage; reports the groups and the work-item shape the autotuner
  * chose for each: cells along x by rows along the second axis (a strip
  * segment; 3-D groups: blocks of at most 16 x 16 columns, 30 x 15 in the
@@ -316,8 +317,10 @@ int fvgpu_batch_tiling(fv_batch* b, int* ngroups, int* tx, int* ty, int max_grou
  * per (grid sizes, precision, group) and remembered in the tile cache;
  * FV3D_TILE=28xH forces the rows, FV3D_TILE=WxH/Bv with W 32 or 64 the
  * block form: width W, rows H, block rows B (8 or 16) and (suffix v) the
- * per-face viscous fluxes.  3-D groups: FV3D_TILE=30xH forces H layers per
- * item, 16xH in the block form.  No reference counterpart. */
+ * per-face viscous fluxes.  3-D groups: FV3D_TILE=16xH forces H layers per
+ * item in 16 x 16 blocks, 30xH z-marched (FP32-mixed without z-boundary and
+ * corrected physics, where both give the same bits and the sizes choose).
+ * No reference counterpart. */
 int fvgpu_batch_schedule(fv_batch* b, int* ngroups, int* tx, int* rows, int* block_rows, int* split_viscous,
                          int max_groups);
 
